@@ -4,6 +4,7 @@
 // flowAdvance (solver.jl:19-189), the RK3 stage loop (solver.jl:416-444), exchange_ghost
 // (mpi.jl:2-103) and fillGhost (boundary.jl:151-156). Every entry point validates its
 // arguments, launches asynchronously on the caller's stream and returns a status code.
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -26,6 +27,30 @@ static int fixed_branch_of(const f3d_params& p) {
     if (p.phi1 <= 0.0 && p.phi2 <= 0.0 && p.phi3 > top) return 2;
     if (p.phi1 <= 0.0 && p.phi2 <= 0.0 && p.phi3 <= 0.0) return 3;
     return -1;
+}
+
+// The linear coefficients as integers over a common denominator D (f3d_fixed.cuh): 420 m with
+// the smallest m <= 500 that makes 420 m (up7 phi + cd6 (1 - phi)) whole for the given blend
+// (m = 1 for phi = 0 and 1, 2 for 0.5, 10 for 0.9, ...), with the signs of a blend in [0, 1] and
+// 32-bit accumulations' room (sum |c| < 2^20).
+static void integer_coefficients(double phi, DevParams& d) {
+    const double up7[7] = {-3, 25, -101, 319, 214, -38, 4}, cd6[7] = {0, 7, -56, 259, 259, -56, 7};
+    d.lin_int = 0;
+    if (!(phi >= 0.0 && phi <= 1.0)) return;
+    for (int m = 1; m <= 500; m++) {
+        int c[7];
+        bool whole = true;
+        for (int k = 0; k < 7; k++) {
+            const double v = m * (up7[k] * phi + cd6[k] * (1.0 - phi)), r = std::nearbyint(v);
+            c[k] = (int)r;
+            whole = whole && std::fabs(v - r) <= 1e-12 * m;
+        }
+        if (!whole) continue;
+        for (int k = 0; k < 7; k++) d.lin_c[k] = c[k];
+        d.lin_s = 1.0 / (420.0 * m);
+        d.lin_int = 1;
+        return;
+    }
 }
 
 int validate_params(const f3d_params& p, std::string& why) {
@@ -103,6 +128,7 @@ DevParams make_dev_params(const f3d_params& p) {
     const double up7[7] = {-3.0 / 420, 25.0 / 420, -101.0 / 420, 319.0 / 420, 214.0 / 420, -38.0 / 420, 4.0 / 420};
     const double cd6[7] = {0.0, 1.0 / 60, -2.0 / 15, 37.0 / 60, 37.0 / 60, -2.0 / 15, 1.0 / 60};
     for (int m = 0; m < 7; m++) d.lin[m] = up7[m] * p.linear_phi + cd6[m] * (1.0 - p.linear_phi);
+    integer_coefficients(p.linear_phi, d);
     d.split = p.split_method; d.character = p.character; d.viscous = p.viscous;
     d.precision = p.precision;
     d.lts = p.lts;

@@ -68,6 +68,10 @@ struct DevParams {
     double eps_clamp;    // utils.jl:12,18
     double phi1, phi2, phi3;
     double lin[7];       // run.jl:75-77
+    // the same as integers over a common denominator: lin[k] = lin_c[k] lin_s, lin_s = 1/D; 0 in
+    // lin_int where no small denominator exists (the FP64 sums are then used)
+    int lin_int, lin_c[7];
+    double lin_s;
     int split, character, viscous;
     int precision;       // F3D_PREC_*
     int ref32;           // F3D_PREC_REF32: Float32 arrays and the reference's Float32 arithmetic

@@ -1,0 +1,134 @@
+// f3d_fixed.cuh — the linear reconstruction (UP7 / CD6 blend, schemes.jl:119-142) of FP64 split
+// fluxes as exact integer sums.
+//
+// What bounds it: an FP64 instruction holds an SM sub-core's FP64 pipe for 64 cycles (FMA of
+// three registers) or 76 (add, multiply, or an FMA with a constant operand; measured with
+// dependent chains), an integer multiply-add of 32 x 32 + 64 bits for 2. The linear face flux is
+// 14 products with fixed coefficients per component, 70 FP64 instructions a face and 40% of the
+// FP64 work of a sweep. Its coefficients are rationals with a small common denominator D
+// (420 for UP7: -3, 25, -101, 319, 214, -38, 4), so D times the flux is an integer combination of
+// the fluxes' mantissas. A strip of five faces of one line and one component aligns the eleven Fp
+// and eleven Fm it reads to the largest of them as 62-bit integers, sums the 5 x 14 products in
+// integers without rounding, and rounds each sum to FP64 once before the product with 1/D: one
+// FP64 instruction a face and component instead of 14. On the 256x64x64 shock tube the three
+// sweeps' FP64 thread instructions go from 181-189 / 160-167 / 166-184 million a launch to
+// 112 / 90 / 107, the sweeps from 517 / 434 / 453 to 366 / 324 / 373 us and the RK3 step from 4.68
+// to 3.67 ms; the viscous ramp's step at 512x256x128 from 75.4 to 61.0 ms. Five faces a strip:
+// their windows share four positions, which bounds the spread, and 22 conversions serve five
+// faces; 13 strips cover a tile's 65 faces exactly.
+//
+// Accuracy: a value whose exponent lies within 9 of the largest is exact; smaller ones lose bits
+// below 2^-62 of the largest. A strip is taken only when a flux that all of its five faces read is
+// within 2^5 of the largest, so every face's error stays below an FP64 evaluation's rounding of
+// its own terms; other strips (and infinities, NaN and magnitudes near the ends of the FP64
+// range) are summed in FP64 as before.
+#pragma once
+#include "f3d_kernels.cuh"
+
+namespace f3d {
+
+constexpr int LIN_STRIP = 5;    // faces a strip: the five windows share positions 4..7
+constexpr int LIN_SPREAD = 5;   // largest exponent minus that of the shared positions
+
+// x 2^(1084 - E) as an integer (E: the strip's largest biased exponent), truncated towards zero
+__device__ __forceinline__ long long fixed_of(double x, int E) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const int e = (int)((hi >> 20) & 0x7ffu);
+    // mantissa with its leading one at bit 63, then right to bit 61 and by the exponent's distance
+    // (zeros and subnormals: E >= 200 makes the distance more than 63, which gives 0)
+    const unsigned long long m =
+        ((unsigned long long)(__funnelshift_l(lo, hi, 11) | 0x80000000u) << 32) | (unsigned long long)(lo << 11);
+    unsigned long long v;
+    asm("shr.u64 %0, %1, %2;" : "=l"(v) : "l"(m), "r"(E - e + 2));  // shifts past 63 give 0
+    const long long s = (long long)((int)hi >> 31);
+    return ((long long)v ^ s) - s;
+}
+
+// The FP64 number nearest to (T 2^32 + r) 2^(E - 1084)
+__device__ __forceinline__ double fixed_to_f64(long long T, unsigned r, int E) {
+    const bool neg = T < 0;
+    if (neg) {
+        r = 0u - r;
+        T = ~T + (r == 0u ? 1 : 0);
+    }
+    unsigned w2 = (unsigned)((unsigned long long)T >> 32), w1 = (unsigned)T, w0 = r;
+    int lead = 95;
+    if (w2 == 0u) {
+        w2 = w1; w1 = w0; w0 = 0u; lead -= 32;
+        if (w2 == 0u) { w2 = w1; w1 = 0u; lead -= 32; }
+    }
+    const int lz = __clz((int)w2);
+    lead -= lz;
+    const unsigned h = __funnelshift_l(w1, w2, lz), l = __funnelshift_l(w0, w1, lz);
+    const unsigned long long m = ((unsigned long long)h << 32) | l;
+    unsigned long long b = (m >> 11) + ((m >> 10) & 1ull);       // 53 bits, rounded
+    b += (unsigned long long)(unsigned)(E + lead - 62) << 52;    // the leading bit adds 1 to the exponent
+    if (w2 == 0u) b = 0ull;
+    return __longlong_as_double((long long)(b | (neg ? 0x8000000000000000ull : 0ull)));
+}
+
+// The five faces t0 .. t0+4 of one line and component: out[f] = sum_k lin[k] (Fp(t+k) + Fm(t+7-k)),
+// t = t0 + f. FP / FM(p) read the split fluxes at position p; positions past `last` were not
+// filled and count as zero (no face that is kept reads them).
+template <class FPA, class FMA>
+__device__ __forceinline__ void linear_strip(const DevParams& P, int t0, int last, FPA FP, FMA FM,
+                                             double out[LIN_STRIP]) {
+    constexpr int NV = LIN_STRIP + 6;
+    // FP64 bit patterns without their sign order like the magnitudes
+    unsigned top = 0u, mid = 0u;
+#pragma unroll
+    for (int p = 0; p < NV; p++) {
+        const unsigned a = t0 + p <= last ? (unsigned)__double2hiint(FP(t0 + p)) & 0x7fffffffu : 0u;
+        const unsigned b = t0 + p + 1 <= last ? (unsigned)__double2hiint(FM(t0 + p + 1)) & 0x7fffffffu : 0u;
+        top = max(top, max(a, b));
+        if (p >= LIN_STRIP - 1 && p <= 6) mid = max(mid, max(a, b));
+    }
+    const int E = (int)(top >> 20), Em = (int)(mid >> 20);
+    if (top == 0u) {  // all zero (or below 2^-1042)
+#pragma unroll
+        for (int f = 0; f < LIN_STRIP; f++) out[f] = 0.0;
+        return;
+    }
+    if (E < 200 || E > 1900 || E - Em > LIN_SPREAD) {
+#pragma unroll
+        for (int f = 0; f < LIN_STRIP; f++) {
+            const int t = t0 + f;
+            out[f] = 0.0;
+            if (t + 7 <= last)
+                out[f] = P.cd.lin[0] * (FP(t) + FM(t + 7)) + P.cd.lin[1] * (FP(t + 1) + FM(t + 6)) +
+                         P.cd.lin[2] * (FP(t + 2) + FM(t + 5)) + P.cd.lin[3] * (FP(t + 3) + FM(t + 4)) +
+                         P.cd.lin[4] * (FP(t + 4) + FM(t + 3)) + P.cd.lin[5] * (FP(t + 5) + FM(t + 2)) +
+                         P.cd.lin[6] * (FP(t + 6) + FM(t + 1));
+        }
+        return;
+    }
+    // sums of the upper words (signed), and of the lower words under the positive and the
+    // negative coefficients (0, 2 and 5)
+    long long hs[LIN_STRIP];
+    unsigned long long lp[LIN_STRIP], ln[LIN_STRIP];
+#pragma unroll
+    for (int f = 0; f < LIN_STRIP; f++) { hs[f] = 0; lp[f] = ln[f] = 0ull; }
+    auto add = [&](int f, int k, int vh, unsigned vl) {
+        hs[f] += (long long)vh * P.lin_c[k];
+        if (k == 0 || k == 2 || k == 5) ln[f] += (unsigned long long)vl * (unsigned)(-P.lin_c[k]);
+        else lp[f] += (unsigned long long)vl * (unsigned)P.lin_c[k];
+    };
+#pragma unroll
+    for (int p = 0; p < NV; p++) {
+        const long long v = t0 + p <= last ? fixed_of(FP(t0 + p), E) : 0ll;
+        const long long w = t0 + p + 1 <= last ? fixed_of(FM(t0 + p + 1), E) : 0ll;
+#pragma unroll
+        for (int f = 0; f < LIN_STRIP; f++) {
+            const int kp = p - f, km = 6 + f - p;  // Fp(t + kp), Fm(t + 7 - km)
+            if (kp >= 0 && kp < 7) add(f, kp, (int)(v >> 32), (unsigned)v);
+            if (km >= 0 && km < 7) add(f, km, (int)(w >> 32), (unsigned)w);
+        }
+    }
+#pragma unroll
+    for (int f = 0; f < LIN_STRIP; f++) {
+        const long long l = (long long)(lp[f] - ln[f]);
+        out[f] = fixed_to_f64(hs[f] + (l >> 32), (unsigned)l, E) * P.lin_s;
+    }
+}
+
+}  // namespace f3d

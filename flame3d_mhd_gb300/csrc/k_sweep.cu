@@ -15,6 +15,7 @@
 // [var][pos][line] for d = y, z (threads run across x-adjacent lines), so global loads
 // coalesce along i and shared loads are conflict-free in both cases.
 #include "f3d_face.cuh"
+#include "f3d_fixed.cuh"
 #include "f3d_sweep_epilogue.cuh"
 
 namespace f3d {
@@ -57,7 +58,8 @@ template <> struct Tile<2, double> { static constexpr int TL = SW_D_TL12, TC = S
 template <int DIR, class R> constexpr size_t sweep_smem_bytes(bool hybrid) {
     using T = Tile<DIR, R>;
     return sizeof(R) * ((size_t)T::TL * (T::TC + 8) * (10 + (hybrid ? 1 : 0)) + (size_t)T::TL * (T::TC + 1) * 5) +
-           sizeof(int) * (2 * (size_t)T::TL * (T::TC + 1) + 4);
+           sizeof(int) * (2 * (size_t)T::TL * (T::TC + 1) + 4) +
+           (sizeof(R) == 8 ? (((size_t)T::TL * (T::TC + 1) + 7) & ~(size_t)7) : 0);  // faces of the linear strips
 }
 
 template <int DIR, bool CHAR, class R>
@@ -97,7 +99,7 @@ __global__ void __launch_bounds__(Tile<DIR, R>::NT, Tile<DIR, R>::MINB) k_sweep(
     auto fidx = [&](int l, int t) { return DIR == 0 ? l * NF + t : t * TL + l; };
     const long long pl = P.plane;
 
-    if (threadIdx.x < 2) reinterpret_cast<int*>(sPhi + TL * NP)[2 * TL * NF + threadIdx.x] = 0;
+    if (threadIdx.x < 3) reinterpret_cast<int*>(sPhi + TL * NP)[2 * TL * NF + threadIdx.x] = 0;
     // ---- Phase A: split every cell the tile's stencils reach (positions 0..nc+7, full
     // index c0 + p along d).
     for (int it = threadIdx.x; it < TL * NP; it += SWEEP_THREADS) {
@@ -122,10 +124,11 @@ __global__ void __launch_bounds__(Tile<DIR, R>::NT, Tile<DIR, R>::MINB) k_sweep(
     __syncthreads();
 
     // ---- Phase B: faces t = 0..nc (face t lies between positions t+3 and t+4).
-    // With the hybrid switch, UP7 and NND2 faces are done at once and the WENO7 / WENO5
-    // faces are queued and then processed by consecutive threads: near a shock only a few
-    // faces of a warp take the long WENO paths, and done in place they would run with the
-    // other lanes idle (and a warp holding both kinds would run both paths).
+    // With the hybrid switch, NND2 faces are done at once and the WENO7 / WENO5 faces are queued
+    // and then processed by consecutive threads: near a shock only a few faces of a warp take
+    // the long WENO paths, and done in place they would run with the other lanes idle (and a
+    // warp holding both kinds would run both paths). FP64 linear faces are done as integer strips
+    // (f3d_fixed.cuh) where their coefficients allow it, others at once.
     auto do_face = [&](int l, int t, int br) {
         const long long cl = cell(l, c0 + t + 3), cr = cl + stride;
         R out[5];
@@ -137,23 +140,19 @@ __global__ void __launch_bounds__(Tile<DIR, R>::NT, Tile<DIR, R>::MINB) k_sweep(
         const int f = fidx(l, t);
 #pragma unroll
         for (int n = 0; n < 5; n++) sF[n * TL * NF + f] = out[n];
-        if (a.faces) {  // face-flux output in the reference's Fx/Fy/Fz shape
-            const long long fx = P.nx + (DIR == 0), fy = P.ny + (DIR == 1), fz = P.nz + (DIR == 2);
-            long long fi, fj, fk;
-            if (DIR == 0) { fi = c0 + t; fj = l0 + l; fk = other; }
-            else if (DIR == 1) { fi = l0 + l; fj = c0 + t; fk = other; }
-            else { fi = l0 + l; fj = other; fk = c0 + t; }
-            const long long fo = fi + fx * (fj + fy * fk), nf = fx * fy * fz;
-#pragma unroll
-            for (int n = 0; n < 5; n++) a.faces[fo + n * nf] = (double)out[n];
-        }
+    };
+    auto face_lt = [&](int it, int& l, int& t) {
+        if (DIR == 0) { l = it / NF; t = it - l * NF; } else { t = it / TL; l = it - t * TL; }
     };
     int* list7 = reinterpret_cast<int*>(sPhi + TL * NP);
     int* list5 = list7 + TL * NF;
-    int* counts = list5 + TL * NF;
+    int* counts = list5 + TL * NF;  // WENO7 and WENO5 faces, next chunk
+    unsigned char* sLin = reinterpret_cast<unsigned char*>(counts + 4);  // faces left to the strips
+    const bool strips = sizeof(R) == 8 && P.lin_int;
     for (int it = threadIdx.x; it < TL * NF; it += SWEEP_THREADS) {
         int l, t;
-        if (DIR == 0) { l = it / NF; t = it - l * NF; } else { t = it / TL; l = it - t * TL; }
+        face_lt(it, l, t);
+        if (strips) sLin[it] = 0;
         if (l >= nl || t > nc) continue;
         int br = P.fixed_branch;
         if (hybrid) {
@@ -167,16 +166,79 @@ __global__ void __launch_bounds__(Tile<DIR, R>::NT, Tile<DIR, R>::MINB) k_sweep(
                 continue;
             }
         }
+        if (strips && br == 0) {
+            sLin[it] = 1;
+            continue;
+        }
         do_face(l, t, br);
     }
-    if (hybrid) {
+    if (hybrid || strips) {
         __syncthreads();
         const int n7 = counts[0], n5 = counts[1];
-        for (int k = threadIdx.x; k < n7 + n5; k += SWEEP_THREADS) {
-            const int it = k < n7 ? list7[k] : list5[k - n7];
+        if constexpr (sizeof(R) == 4) {
+            for (int k = threadIdx.x; k < n7 + n5; k += SWEEP_THREADS) {
+                int l, t;
+                face_lt(k < n7 ? list7[k] : list5[k - n7], l, t);
+                do_face(l, t, k < n7 ? 1 : 2);
+            }
+        } else {
+            // chunks of 32 items taken by warps as they come free: the WENO faces first (~1300
+            // FP64 instructions each), then the strips, so that no warp waits at the barrier
+            // while another works through the block's WENO faces
+            const int ns = (nc + LIN_STRIP) / LIN_STRIP, per = ns * (DIR == 0 ? nl : TL), items = 5 * per;
+            const int ch7 = (n7 + 31) / 32, ch5 = (n5 + 31) / 32, chs = strips ? (items + 31) / 32 : 0;
+            const int lane = threadIdx.x & 31;
+            for (;;) {
+                int ch = 0;
+                if (lane == 0) ch = atomicAdd(&counts[2], 1);
+                ch = __shfl_sync(0xffffffffu, ch, 0);
+                if (ch >= ch7 + ch5 + chs) break;
+                if (ch < ch7 + ch5) {
+                    const bool w7 = ch < ch7;
+                    const int k = (w7 ? ch : ch - ch7) * 32 + lane;
+                    if (k < (w7 ? n7 : n5)) {
+                        int l, t;
+                        face_lt(w7 ? list7[k] : list5[k], l, t);
+                        do_face(l, t, w7 ? 1 : 2);
+                    }
+                    continue;
+                }
+                const int k = (ch - ch7 - ch5) * 32 + lane;
+                if (k >= items) continue;
+                const int n = k / per, r = k - n * per;
+                int l, st;
+                if (DIR == 0) { l = r / ns; st = r - l * ns; } else { st = r / TL; l = r - st * TL; }
+                const int t0 = st * LIN_STRIP;
+                unsigned want = 0u;
+#pragma unroll
+                for (int f = 0; f < LIN_STRIP; f++)
+                    if (t0 + f < NF && sLin[fidx(l, t0 + f)]) want |= 1u << f;
+                if (!want) continue;
+                const R* fp = sFp + n * TL * NP;
+                const R* fm = sFm + n * TL * NP;
+                double out[LIN_STRIP];
+                linear_strip(P, t0, nc + 7, [&](int p) { return (double)fp[sidx(l, p)]; },
+                             [&](int p) { return (double)fm[sidx(l, p)]; }, out);
+#pragma unroll
+                for (int f = 0; f < LIN_STRIP; f++)
+                    if (want >> f & 1u) sF[n * TL * NF + fidx(l, t0 + f)] = out[f];
+            }
+        }
+    }
+    if (sizeof(R) == 8 && a.faces) {  // face-flux output in the reference's Fx/Fy/Fz shape
+        __syncthreads();
+        const long long fx = P.nx + (DIR == 0), fy = P.ny + (DIR == 1), fz = P.nz + (DIR == 2), nf = fx * fy * fz;
+        for (int it = threadIdx.x; it < TL * NF; it += SWEEP_THREADS) {
             int l, t;
-            if (DIR == 0) { l = it / NF; t = it - l * NF; } else { t = it / TL; l = it - t * TL; }
-            do_face(l, t, k < n7 ? 1 : 2);
+            face_lt(it, l, t);
+            if (l >= nl || t > nc) continue;
+            long long fi, fj, fk;
+            if (DIR == 0) { fi = c0 + t; fj = l0 + l; fk = other; }
+            else if (DIR == 1) { fi = l0 + l; fj = c0 + t; fk = other; }
+            else { fi = l0 + l; fj = other; fk = c0 + t; }
+            const long long fo = fi + fx * (fj + fy * fk);
+#pragma unroll
+            for (int n = 0; n < 5; n++) a.faces[fo + n * nf] = (double)sF[n * TL * NF + it];
         }
     }
     if (a.out_mode == OUT_FACES) return;
