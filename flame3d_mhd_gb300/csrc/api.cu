@@ -227,6 +227,10 @@ struct f3d_ctx {
     double* dscalar = nullptr;  // 8 bytes for reductions
     unsigned* kstat = nullptr;  // kernel status word (bit 0: a TMA tile wait gave up)
     unsigned* tile_ctr = nullptr;  // next-tile counters of the TMA sweeps
+    // listed WENO faces of the state being swept (hybrid finite-difference scheme in FP64;
+    // null elsewhere)
+    WenoList weno = {};
+    int sms = 0;
     // mixed form: the TMA-staged sweeps and their tensor maps (three directions)
     bool use_tma = false;
     void* tma_maps = nullptr;
@@ -253,9 +257,9 @@ struct f3d_ctx {
 namespace {
 
 enum KernelKind { K_SOUND = 0, K_SENSOR, K_VISCOUS, K_SWEEP_X, K_SWEEP_Y, K_SWEEP_Z, K_PRIM_FILL, K_STAGE_UPDATE,
-                  K_NKIND };
+                  K_WENO, K_NKIND };
 const char* kKernelNames[K_NKIND] = {"sound_speed", "shock_sensor", "viscous_flux", "sweep_xi",
-                                     "sweep_eta", "sweep_zeta", "prim_ghost_fill", "stage_update"};
+                                     "sweep_eta", "sweep_zeta", "prim_ghost_fill", "stage_update", "weno_faces"};
 
 void mark(f3d_ctx* ctx, int kind, cudaStream_t st, int launches = 1) {
     Prof* p = ctx->prof;
@@ -351,6 +355,24 @@ SweepArgs sweep_args(f3d_ctx* ctx, int dir, const double* Q, bool hybrid, const 
     return a;
 }
 
+// List the WENO faces of a state and compute their fluxes (k_weno.cu); the sweeps then read them.
+int list_weno(f3d_ctx* ctx, const double* Q, const double* csnd, const double* phi, cudaStream_t st) {
+    if (!ctx->weno.list) return F3D_OK;
+    WenoArgs a;
+    a.P = ctx->dp;
+    a.w = ctx->weno;
+    a.Q = Q;
+    a.csnd = csnd;
+    for (int n = 0; n < 9; n++) {
+        a.A[n] = ctx->m[n];
+        a.H[n] = ctx->Ah[n];
+    }
+    for (int d = 0; d < 3; d++) a.S[d] = ctx->S[d];
+    F3D_CUDA(ctx, launch_weno(a, phi, ctx->sms, st));
+    mark(ctx, K_WENO, st, 2);
+    return F3D_OK;
+}
+
 // Sensor, viscous fluxes and the three sweeps. last.out_mode is OUT_RHS or OUT_STAGE.
 // fill_current: the previous stage's primitive fill already wrote what the sweeps read besides
 // Q (mixed precision: the FP32 copy of Q; FP64: the sound speed), so it is not made again.
@@ -427,8 +449,10 @@ int run_rhs(f3d_ctx* ctx, const double* Q, double* acc, SweepArgs last, cudaStre
         }
     }
     if (ctx->use_tma) F3D_CUDA(ctx, cudaMemsetAsync(ctx->tile_ctr, 0, 3 * sizeof(unsigned), st));
+    if (int rc = list_weno(ctx, Q, ctx->csnd, ctx->phi, st)) return rc;
     for (int d = 0; d < 3; d++) {
         SweepArgs a = sweep_args(ctx, d, Q, hybrid);
+        if (ctx->weno.list) a.wflux = ctx->weno.flux + 5 * d * P.plane;
         a.acc = mx ? (void*)ctx->acc32 : (void*)acc;
         if (d == 0) a.out_mode = OUT_SET;
         else if (d == 1) {
@@ -570,8 +594,10 @@ int rhs_prepared(f3d_ctx* ctx, const double* Q, const double* csnd, const double
     const DevParams& P = ctx->dp;
     const bool hybrid = P.fixed_branch < 0;
     if (ctx->params.viscous) F3D_CUDA(ctx, launch_viscous(P, Q, ctx->m, ctx->J, ctx->Fv[0], ctx->Fv[1], ctx->Fv[2], st));
+    if (int rc = list_weno(ctx, Q, csnd, phi, st)) return rc;
     for (int d = 0; d < 3; d++) {
         SweepArgs a = sweep_args(ctx, d, Q, hybrid, phi);
+        if (ctx->weno.list) a.wflux = ctx->weno.flux + 5 * d * P.plane;
         a.csnd = csnd;
         a.acc = out;
         a.out = out;
@@ -749,8 +775,29 @@ int f3d_create(const f3d_params* p, f3d_ctx** out) {
     } else {    // [Q32(6) + A32(9) + J32 + acc32b(5), mixed only] + H32(9) + S32(3) + phi32 + acc32(5) [+ viscous 12]
         total += up(nc * 4) * ((r32 ? 0 : 21) + 9 + 3 + 1 + 5) + (p->viscous ? 3 * up(nv * 4 * 4) : 0);
     }
-    cudaError_t e = cudaMalloc(&ctx->slab, total);
+    // the listed WENO faces (k_weno.cu) of the hybrid finite-difference scheme in FP64: 132 bytes
+    // a cell, taken up to 25 GiB (a tenth of the device's memory) and where there is
+    // room; without them the tiles keep their WENO faces. So do the FP32 forms, whose faces are
+    // cheap and whose results would change in the last FP32 bits with the place they are computed in
+    const size_t bl = up(3 * nc * 4), lists = 256 + bl + 15 * nc * 8;
+    bool listed = !fvm && !mx && ctx->dp.fixed_branch < 0 && lists <= ((size_t)25 << 30);
+    cudaError_t e = cudaMalloc(&ctx->slab, up(total) + (listed ? lists : 0));
+    if (e != cudaSuccess && listed) {
+        cudaGetLastError();
+        listed = false;
+        e = cudaMalloc(&ctx->slab, total);
+    }
+    if (e == cudaSuccess && listed) {
+        char* w = (char*)ctx->slab + up(total);
+        ctx->weno.count = (unsigned*)w;
+        ctx->weno.list = (int*)(w + 256);
+        ctx->weno.flux = (double*)(w + 256 + bl);
+        if ((e = cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->device)) == cudaSuccess)
+            e = cudaMemset(w, 0, 256);
+        total = up(total) + lists;
+    }
     if (e != cudaSuccess) {
+        if (ctx->slab) cudaFree(ctx->slab);
         if (ctx->extra) cudaFree(ctx->extra);
         delete ctx;
         std::fprintf(stderr, "f3d_create: cudaMalloc(%zu) failed: %s\n", total, cudaGetErrorString(e));

@@ -3,7 +3,7 @@
 // speed, shared by the direct-load sweeps (k_sweep.cu) and the TMA-staged ones
 // (k_sweep_tma.cu).
 #pragma once
-#include "f3d_kernels.cuh"
+#include "f3d_sweep_epilogue.cuh"
 
 namespace f3d {
 
@@ -21,14 +21,10 @@ template <class R> struct CharBasis {
 };
 
 template <class R>
-__device__ __forceinline__ void char_basis(const DevParams& P, const SweepArgs& a, R s0, long long cl, long long cr,
-                                           CharBasis<R>& b) {
+__device__ __forceinline__ void char_basis(const DevParams& P, const R* Qr, const R* A0, const R* A1p, const R* A2p, R s0,
+                                           long long cl, long long cr, CharBasis<R>& b) {
     const Cst<R>& K = cst<R>(P);
     const long long pl = P.plane;
-    const R* Qr = static_cast<const R*>(a.Q);
-    const R* A0 = static_cast<const R*>(a.A[0]);
-    const R* A1p = static_cast<const R*>(a.A[1]);
-    const R* A2p = static_cast<const R*>(a.A[2]);
     const R u = R(0.5) * (Qr[cr + pl] + Qr[cl + pl]);
     const R v = R(0.5) * (Qr[cr + 2 * pl] + Qr[cl + 2 * pl]);
     const R w = R(0.5) * (Qr[cr + 3 * pl] + Qr[cl + 3 * pl]);
@@ -140,6 +136,36 @@ __device__ __forceinline__ R char_right_row(const CharBasis<R>& b, int k, const 
     return f[0] * (ak - b.c * nk) + f[1] * ap + f[2] * (ak + b.c * nk) + f[3] * lk + f[4] * mk;
 }
 
+// Component n of a component-wise WENO7 (schemes.jl:143-230) / WENO5 (:231-276) face
+template <class R, class FPA, class FMA>
+__device__ __forceinline__ R comp_field_flux(const DevParams& P, int n, int br, int p0, R s0, FPA FP, FMA FM) {
+    const R tmp1 = R(1) / R(12), tmp2 = R(1) / R(6);
+    if constexpr (sizeof(R) == 4) {
+        if (P.ref32) {  // the reference's Float32 reconstruction
+            if (br == 1) {
+                const double fp = weno7_ref32(FP(n, p0), FP(n, p0 + 1), FP(n, p0 + 2), FP(n, p0 + 3), FP(n, p0 + 4),
+                                              FP(n, p0 + 5), FP(n, p0 + 6), s0);
+                const double fm = weno7_ref32(FM(n, p0 + 7), FM(n, p0 + 6), FM(n, p0 + 5), FM(n, p0 + 4),
+                                              FM(n, p0 + 3), FM(n, p0 + 2), FM(n, p0 + 1), s0);
+                return (float)((fp + fm) * (double)tmp1);
+            }
+            return (weno5_ref32(FP(n, p0 + 1), FP(n, p0 + 2), FP(n, p0 + 3), FP(n, p0 + 4), FP(n, p0 + 5), s0) +
+                    weno5_ref32(FM(n, p0 + 6), FM(n, p0 + 5), FM(n, p0 + 4), FM(n, p0 + 3), FM(n, p0 + 2), s0)) *
+                   tmp2;
+        }
+    }
+    if (br == 1) {
+        R fp = weno7(FP(n, p0), FP(n, p0 + 1), FP(n, p0 + 2), FP(n, p0 + 3), FP(n, p0 + 4), FP(n, p0 + 5),
+                     FP(n, p0 + 6), s0);
+        R fm = weno7(FM(n, p0 + 7), FM(n, p0 + 6), FM(n, p0 + 5), FM(n, p0 + 4), FM(n, p0 + 3), FM(n, p0 + 2),
+                     FM(n, p0 + 1), s0);
+        return (fp + fm) * tmp1;
+    }
+    R fp = weno5(FP(n, p0 + 1), FP(n, p0 + 2), FP(n, p0 + 3), FP(n, p0 + 4), FP(n, p0 + 5), s0);
+    R fm = weno5(FM(n, p0 + 6), FM(n, p0 + 5), FM(n, p0 + 4), FM(n, p0 + 3), FM(n, p0 + 2), s0);
+    return (fp + fm) * tmp2;
+}
+
 // Face flux of one face from the split fluxes of the 8 cells around it, positions
 // p0..p0+7 of the line (face between positions p0+3 and p0+4). FP/FM(n, pos) read shared
 // memory. For characteristic mode the face state comes from global memory at the two
@@ -178,45 +204,15 @@ __device__ __forceinline__ void face_flux(const DevParams& P, const SweepArgs& a
         }
         return;
     }
-    const R tmp1 = R(1) / R(12), tmp2 = R(1) / R(6);
-    if (!CHAR) {  // component-wise WENO7 (schemes.jl:143-230) / WENO5 (:231-276)
+    if (!CHAR) {
 #pragma unroll 1
-        for (int n = 0; n < 5; n++) {
-            if constexpr (sizeof(R) == 4) {
-                if (P.ref32) {  // the reference's Float32 reconstruction
-                    if (br == 1) {
-                        const double fp = weno7_ref32(FP(n, p0), FP(n, p0 + 1), FP(n, p0 + 2), FP(n, p0 + 3),
-                                                      FP(n, p0 + 4), FP(n, p0 + 5), FP(n, p0 + 6), s0);
-                        const double fm = weno7_ref32(FM(n, p0 + 7), FM(n, p0 + 6), FM(n, p0 + 5), FM(n, p0 + 4),
-                                                      FM(n, p0 + 3), FM(n, p0 + 2), FM(n, p0 + 1), s0);
-                        out[n] = (float)((fp + fm) * (double)tmp1);
-                    } else {
-                        out[n] = (weno5_ref32(FP(n, p0 + 1), FP(n, p0 + 2), FP(n, p0 + 3), FP(n, p0 + 4),
-                                              FP(n, p0 + 5), s0) +
-                                  weno5_ref32(FM(n, p0 + 6), FM(n, p0 + 5), FM(n, p0 + 4), FM(n, p0 + 3),
-                                              FM(n, p0 + 2), s0)) *
-                                 tmp2;
-                    }
-                    continue;
-                }
-            }
-            if (br == 1) {
-                R fp = weno7(FP(n, p0), FP(n, p0 + 1), FP(n, p0 + 2), FP(n, p0 + 3), FP(n, p0 + 4), FP(n, p0 + 5),
-                             FP(n, p0 + 6), s0);
-                R fm = weno7(FM(n, p0 + 7), FM(n, p0 + 6), FM(n, p0 + 5), FM(n, p0 + 4), FM(n, p0 + 3),
-                             FM(n, p0 + 2), FM(n, p0 + 1), s0);
-                out[n] = (fp + fm) * tmp1;
-            } else {
-                R fp = weno5(FP(n, p0 + 1), FP(n, p0 + 2), FP(n, p0 + 3), FP(n, p0 + 4), FP(n, p0 + 5), s0);
-                R fm = weno5(FM(n, p0 + 6), FM(n, p0 + 5), FM(n, p0 + 4), FM(n, p0 + 3), FM(n, p0 + 2), s0);
-                out[n] = (fp + fm) * tmp2;
-            }
-        }
+        for (int n = 0; n < 5; n++) out[n] = comp_field_flux<R>(P, n, br, p0, s0, FP, FM);
         return;
     }
     // characteristic-wise, schemes.jl:756-999
     CharBasis<R> cb;
-    char_basis<R>(P, a, s0, cl, cr, cb);
+    char_basis<R>(P, static_cast<const R*>(a.Q), static_cast<const R*>(a.A[0]), static_cast<const R*>(a.A[1]),
+                  static_cast<const R*>(a.A[2]), s0, cl, cr, cb);
     R flux[5];
 #pragma unroll 1
     for (int n = 0; n < 5; n++) flux[n] = char_field_flux<R>(P, cb, n, br, p0, s0, FP, FM);
@@ -231,9 +227,12 @@ template <> __device__ __forceinline__ double split_sound<double>(const DevParam
                                                                   const double*) {
     return static_cast<const double*>(a.csnd)[c];
 }
+__device__ __forceinline__ float split_sound32(const DevParams& P, const float* q) {
+    return P.split == F3D_SPLIT_SW ? sqrtf(P.cf.grg * q[5]) : sqrtf(P.cf.gamma * q[4] / q[0]);
+}
 template <> __device__ __forceinline__ float split_sound<float>(const DevParams& P, const SweepArgs&, long long,
                                                                 const float* q) {
-    return P.split == F3D_SPLIT_SW ? sqrtf(P.cf.grg * q[5]) : sqrtf(P.cf.gamma * q[4] / q[0]);
+    return split_sound32(P, q);
 }
 
 }  // namespace f3d

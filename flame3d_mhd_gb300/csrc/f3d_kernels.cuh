@@ -9,6 +9,25 @@ namespace f3d {
 
 enum OutMode { OUT_SET = 0, OUT_ADD = 1, OUT_RHS = 2, OUT_STAGE = 3, OUT_FACES = 4 };
 
+// The listed WENO faces of a state (k_weno.cu): one list of `plane` left-cell indices a direction,
+// WENO7 faces from its front and WENO5 faces from its back, their six counts (and the finished
+// blocks of k_weno_faces), and the fluxes, five planes a direction.
+struct WenoList {
+    int* list;
+    unsigned* count;
+    double* flux;
+};
+struct WenoArgs {
+    DevParams P;
+    WenoList w;
+    const double* Q;
+    const double* csnd;
+    const double* A[9];
+    const double* H[9];
+    const double* S[3];
+};
+cudaError_t launch_weno(const WenoArgs& a, const double* phi, int sms, cudaStream_t st);
+
 // Arguments of one sweep. The field pointers are typed by the sweep's arithmetic: double
 // arrays for the FP64 form, float arrays (FP32 copies) for the mixed form (fp32 = 1).
 // J, U, Un, out and faces are double in both forms.
@@ -20,6 +39,7 @@ struct SweepArgs {
     const void* Ah[3];    // A * (1/|A|)
     const void* S;        // |A|
     const void* phi;      // shock sensor (only read when P.fixed_branch < 0)
+    const double* wflux;  // FP64 form: fluxes of this direction's WENO faces at their left cells, or null
     const void* Fv;       // viscous flux of this direction ((Nt-4)^3 x 4) or null
     const double* J;      // Jacobian
     void* acc;            // RHS accumulator (U layout)

@@ -1,0 +1,54 @@
+"""GPU: the FP64 right-hand side, whose WENO faces are listed and computed apart from the tiles
+(k_weno.cu), against the differences of the face fluxes that f3d_debug_face_flux computes within
+the tiles. Sizes around the 32-face chunks and the tiles; thresholds that give every branch, only
+WENO7 faces (the list filled from its front to its end), only WENO5 faces (from its back), or none."""
+import numpy as np
+import pytest
+
+from flame3d_mhd_gb300 import abi
+
+pytestmark = pytest.mark.gpu
+EPS = 2.0 ** -53
+TINY, FAR = 1e-300, 5.0
+THRESHOLDS = {"all": (0.05, 0.3, 0.6), "weno7": (TINY, 4.5, FAR), "weno5": (TINY, 2 * TINY, FAR), "none": (FAR - 1, FAR, FAR)}
+
+
+@pytest.mark.parametrize("n", [(4, 4, 4), (33, 5, 9), (64, 65, 6), (70, 9, 31)])
+@pytest.mark.parametrize("which", sorted(THRESHOLDS))
+@pytest.mark.parametrize("character,split", [(1, "SW"), (0, "AUSM")])
+def test_rhs_equals_differences_of_tile_faces(gpu_lib, n, which, character, split):
+    import torch
+
+    from flame3d_mhd_gb300.solver import Flame3D
+    nx, ny, nz = n
+    per = dict(kind=abi.BC_PERIODIC)
+    p1, p2, p3 = THRESHOLDS[which]
+    s = Flame3D(abi.make_params(nx, ny, nz, phi1=p1, phi2=p2, phi3=p3, viscous=0, character=character, split=split,
+                                bc=[per] * 6))
+    shape = (nz + 8, ny + 8, nx + 8)
+    r = np.random.default_rng(11)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    eye = [1.0, 0.0, 0.0, 0.0, 1.0, 0.0, 0.0, 0.0, 1.0]
+    s.set_metrics([dev(e + 0.1 * r.uniform(-1, 1, shape)) for e in eye], dev(np.ones(shape)))
+    q = np.empty((6, *shape))
+    q[0] = r.uniform(0.7, 1.3, shape)
+    q[1:4] = r.uniform(-0.6, 0.6, (3, *shape))
+    q[4] = r.uniform(0.3, 1.5, shape) ** 2
+    q[5] = q[4] / (q[0] * 287.0)
+    Q, phi = dev(q), s.field(1)
+    s.shockSensor(phi, Q)
+    want, scale = 0.0, 0.0
+    for d in range(3):
+        F = s.face_field(d)
+        s.advect(d, F, phi, Q)
+        f = np.moveaxis(F.cpu().numpy(), 3 - d, -1)
+        want = want + np.moveaxis(f[..., :-1] - f[..., 1:], -1, 3 - d)
+        scale = scale + np.moveaxis(np.abs(f[..., :-1]) + np.abs(f[..., 1:]), -1, 3 - d)
+    I = (slice(None), *(slice(4, -4),) * 3)
+    for _ in range(2):  # the second pass starts from the counts the first one cleared
+        got = s.rhs(Q).cpu().numpy()[I]
+        # the two paths form the same face fluxes in another order of rounding: an FP64 WENO flux of
+        # this state is within ~1e3 eps of its exact value relative to the largest component
+        tol = 2048 * EPS * scale.max(0)
+        assert (np.abs(got - want).max(0) <= tol).all(), float((np.abs(got - want).max(0) / tol).max())
+    s.close()
