@@ -21,21 +21,20 @@
 namespace f3d {
 
 // Tile (lines TL x cells TC), threads and resident blocks per SM of a sweep, by type.
-// FP64: 8 x 64 in every direction on 288 threads, two blocks per SM (~76 KB of shared memory
-// each): the tile's 8 x 72 split positions take exactly two rounds of 288 threads. Against
-// 256 threads on 8 x 64 (xi) and 16 x 32 (eta, zeta) tiles, whose 576 / 640 positions took
-// 2.25 / 2.5 rounds: +0.7% per RK3 step on the 256x64x64 shock tube (same box, three rounds
-// of alternating builds); two blocks of nine warps leave 96 registers a thread (five warps on
-// one of the SM's four register-file quarters), which the characteristic-wise instantiations
-// use without spilling (72-92 component-wise). FP32:
-// half-height tiles on 128 threads, six blocks per SM (~20 KB each): the same step time as
+// FP64: 4 x 64 in every direction on 160 threads, four blocks per SM (~38 KB of shared memory
+// each, 96 registers a thread): 20 warps an SM hide each other's loads, barriers and FP64
+// latencies better than two blocks of nine warps on 8 x 64 tiles, at the same halo. Measured on
+// one box (RK3 step): shock tube 256x64x64 3.03 -> 2.91 ms, ramp 512x256x128 61.1 -> 58.7 ms,
+// plate 125x61x37 1.67 -> 1.55 ms. 32-cell tiles split a quarter of their cells twice (tube 3.2
+// ms, ramp 63.6 ms); 128 threads x 5 blocks and 192 x 3 on this tile: 3.04 / 3.22 ms.
+// FP32: half-height tiles on 128 threads, six blocks per SM (~20 KB each): the same step time as
 // three 256-thread blocks on that tube, 6% less per RHS on the component-wise tube and on
 // the viscous vortex.
 #ifndef SW_D_THREADS
-#define SW_D_THREADS 288
-#define SW_D_BLOCKS 2
-#define SW_D_TL0 8
-#define SW_D_TL12 8
+#define SW_D_THREADS 160
+#define SW_D_BLOCKS 4
+#define SW_D_TL0 4
+#define SW_D_TL12 4
 #endif
 #ifndef SW_D_TC0
 #define SW_D_TC0 64
