@@ -435,12 +435,12 @@ int run_rhs(f3d_ctx* ctx, const double* Q, double* acc, SweepArgs last, cudaStre
             mark(ctx, K_VISCOUS, st);
         }
     } else {
-        if (!fill_current) {
+        if (!fill_current && !hybrid) {  // with the sensor when there is one
             F3D_CUDA(ctx, launch_sound(P, Q, ctx->csnd, st));
             mark(ctx, K_SOUND, st);
         }
         if (hybrid) {
-            F3D_CUDA(ctx, launch_sensor(P, Q, ctx->phi, st));
+            F3D_CUDA(ctx, launch_sensor(P, Q, ctx->phi, st, false, fill_current ? nullptr : ctx->csnd));
             mark(ctx, K_SENSOR, st);
         }
         if (ctx->params.viscous) {

@@ -137,11 +137,25 @@ __device__ __forceinline__ void c2prim_cell(const DevParams& P, const double U[5
 // the mixed form needs for its FP64 state arithmetic. These work on the IEEE 754 binary64 /
 // binary32 bit layouts with integer operations in the binary32 normal range and use the
 // conversion instruction elsewhere (zeros, subnormal results, overflow, infinities, NaN).
+// The instruction is volatile so that it stays behind its branch: the compiler otherwise runs it
+// for every value beside the integer form and selects (64 cycles of the FP64 pipe a conversion;
+// the sensor issued 7.6 a warp and the mixed form's primitive pass and stage update one a value).
+__device__ __forceinline__ float cvt_f32_rn(double x) {
+    float r;
+    asm volatile("cvt.rn.f32.f64 %0, %1;" : "=f"(r) : "d"(x));
+    return r;
+}
+__device__ __forceinline__ double cvt_f64(float x) {
+    double r;
+    asm volatile("cvt.f64.f32 %0, %1;" : "=d"(r) : "f"(x));
+    return r;
+}
 __device__ __forceinline__ float f64_to_f32_rn(double x) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(x);
     const unsigned int hi = (unsigned int)(b >> 32);
     const int e = (int)((hi >> 20) & 0x7ffu);  // biased binary64 exponent
-    if (e < 897 || e > 1150) return __double2float_rn(x);  // outside binary32 exponents 1..254
+    if (e < 897 || e > 1150)  // outside binary32 exponents 1..254; +-0 as they are
+        return b << 1 ? cvt_f32_rn(x) : __uint_as_float(hi);
     const unsigned int m23 = (unsigned int)((b >> 29) & 0x7fffffull);
     const unsigned int rest = (unsigned int)(b & 0x1fffffffull);  // the 29 dropped bits
     unsigned int f = (hi & 0x80000000u) | ((unsigned int)(e - 896) << 23) | m23;
@@ -153,7 +167,7 @@ __device__ __forceinline__ float f64_to_f32_rn(double x) {
 __device__ __forceinline__ double f32_to_f64(float x) {  // exact
     const unsigned int b = __float_as_uint(x);
     const unsigned int e = (b >> 23) & 0xffu;
-    if (e == 0u || e == 0xffu) return (double)x;
+    if (e == 0u || e == 0xffu) return b << 1 ? cvt_f64(x) : __longlong_as_double((long long)b << 32);  // +-0 as they are
     const unsigned long long r = ((unsigned long long)(b & 0x80000000u) << 32) |
                                  ((unsigned long long)(e + 896u) << 52) | ((unsigned long long)(b & 0x7fffffu) << 29);
     return __longlong_as_double((long long)r);

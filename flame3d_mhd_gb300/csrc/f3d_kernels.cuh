@@ -7,6 +7,35 @@
 
 namespace f3d {
 
+// Programmatic dependent launch of the light kernels between the sweeps on small grids. Such a
+// kernel may be scheduled while its predecessor in the stream drains; it begins with
+// after_previous(), which waits until everything before it has completed and its writes are visible,
+// so the order of all memory accesses is that of plain launches. On 16^3 cells, where launches
+// and block start-up are a third of a right-hand side, it takes 53 to 49 us. Larger grids take
+// plain launches (the ramp's mixed step at 512x256x128 ran 2% slower with it: an SM that never
+// empties keeps the sweeps' shared-memory split, and the stencil kernels miss their L1), and so do
+// the kernels whose blocks must spread evenly over the SMs (the sweeps and the WENO faces: the
+// 32x16x16 tube's step ran 10% slower when they filled whatever room the last kernel left).
+constexpr long long OVERLAP_CELLS = 1 << 16;
+__device__ __forceinline__ void after_previous() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... Params, class... Args>
+inline cudaError_t launch_after(const DevParams& P, void (*kernel)(Params...), unsigned grid, unsigned block, cudaStream_t st,
+                                Args&&... args) {
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = P.plane <= OVERLAP_CELLS ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 enum OutMode { OUT_SET = 0, OUT_ADD = 1, OUT_RHS = 2, OUT_STAGE = 3, OUT_FACES = 4 };
 
 // The listed WENO faces of a state (k_weno.cu): one list of `plane` left-cell indices a direction,
@@ -169,8 +198,9 @@ cudaError_t launch_prim2c(const DevParams& P, const double* Q, double* U, cudaSt
 cudaError_t launch_lincomb(const DevParams& P, double* U, const double* Un, double a, double b, cudaStream_t st);
 cudaError_t launch_sound(const DevParams& P, const double* Q, double* csnd, cudaStream_t st);
 // exact: phi bit for bit as the oracle's; otherwise values that give the same branch map
-// (FP32 away from the thresholds, FP64 near them)
-cudaError_t launch_sensor(const DevParams& P, const double* Q, double* phi, cudaStream_t st, bool exact = false);
+// (FP32 away from the thresholds, FP64 near them); csnd: also the split's sound speed (not exact)
+cudaError_t launch_sensor(const DevParams& P, const double* Q, double* phi, cudaStream_t st, bool exact = false,
+                          double* csnd = nullptr);
 cudaError_t launch_metric_prep(const DevParams& P, const double* const m[9], double* S[3], double* Ah[9],
                                cudaStream_t st);
 cudaError_t launch_split_debug(const DevParams& P, const double* Q, const double* csnd, const double* const A[3],

@@ -33,6 +33,7 @@ __device__ __forceinline__ double sound_speed(const DevParams& P, const double q
 // sound speed and the FP32 copy when they are asked for.
 __global__ void k_prim_interior(const DevParams P, const double* U, double* Q, double* csnd, float* Q32,
                                 int from_q) {
+    after_previous();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long long)P.nx * P.ny * P.nz) return;
     int i, j, k;
@@ -88,6 +89,7 @@ __device__ __forceinline__ void ghost_ijk(const DevParams& P, long long g, int& 
 }
 
 __global__ void k_prim_ghost(const DevParams P, const double* U, double* Q, double* Ug, double* csnd, float* Q32) {
+    after_previous();
     const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= P.plane - (long long)P.nx * P.ny * P.nz) return;
     const long long pl = P.plane;
@@ -125,8 +127,8 @@ __global__ void k_prim_ghost(const DevParams P, const double* U, double* Q, doub
 cudaError_t launch_prim_fill(const DevParams& P, const double* U, double* Q, double* Ug, double* csnd, int from_q,
                              cudaStream_t st, float* Q32) {
     const long long ni = (long long)P.nx * P.ny * P.nz;
-    if (!from_q || csnd || Q32) k_prim_interior<<<pw_blocks(ni), PW_THREADS, 0, st>>>(P, U, Q, csnd, Q32, from_q);
-    k_prim_ghost<<<pw_blocks(P.plane - ni), PW_THREADS, 0, st>>>(P, U, Q, Ug, csnd, Q32);
+    if (!from_q || csnd || Q32) launch_after(P, k_prim_interior, pw_blocks(ni), PW_THREADS, st, P, U, Q, csnd, Q32, from_q);
+    launch_after(P, k_prim_ghost, pw_blocks(P.plane - ni), PW_THREADS, st, P, U, Q, Ug, csnd, Q32);
     return cudaGetLastError();
 }
 
@@ -243,6 +245,7 @@ cudaError_t launch_lincomb(const DevParams& P, double* U, const double* Un, doub
 }
 
 __global__ void k_sound(const DevParams P, const double* Q, double* csnd) {
+    after_previous();
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= P.plane) return;
     double q[6];
@@ -251,7 +254,7 @@ __global__ void k_sound(const DevParams P, const double* Q, double* csnd) {
     csnd[c] = sound_speed(P, q);
 }
 cudaError_t launch_sound(const DevParams& P, const double* Q, double* csnd, cudaStream_t st) {
-    k_sound<<<pw_blocks(P.plane), PW_THREADS, 0, st>>>(P, Q, csnd);
+    launch_after(P, k_sound, pw_blocks(P.plane), PW_THREADS, st, P, Q, csnd);
     return cudaGetLastError();
 }
 
@@ -271,9 +274,18 @@ __device__ __forceinline__ double sensor_term(double a, double b, double c) {
 // FP32 evaluation is within 1e-6 of the exact value (pressure rounding 2^-24 relative, five
 // FP32 roundings), so a kept value is on the same side of every threshold as the FP64 value:
 // the branch map is the FP64 sensor's, with three FP64 divisions saved at almost every cell.
-template <bool EXACT> __global__ void k_sensor(const DevParams P, const double* Q, double* phi) {
+// csnd (optional): the split's sound speed of every cell is formed here too, for a right-hand side
+// whose state no primitive fill has prepared (one launch and one pass over p and T less).
+template <bool EXACT> __global__ void k_sensor(const DevParams P, const double* Q, double* phi, double* csnd) {
+    after_previous();
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= P.plane) return;
+    if (!EXACT && csnd) {
+        double q[6];
+#pragma unroll
+        for (int n = 0; n < 6; n++) q[n] = Q[c + n * P.plane];
+        csnd[c] = sound_speed(P, q);
+    }
     int i, j, k;
     cell_ijk(P, c, i, j, k);
     if (i < 1 || i > P.nxt - 2 || j < 1 || j > P.nyt - 2 || k < 1 || k > P.nzt - 2) return;
@@ -299,9 +311,9 @@ template <bool EXACT> __global__ void k_sensor(const DevParams P, const double* 
     double fz = sensor_term(pzm, pc, pzp);
     phi[c] = __dadd_rn(__dadd_rn(fx, fy), fz);
 }
-cudaError_t launch_sensor(const DevParams& P, const double* Q, double* phi, cudaStream_t st, bool exact) {
-    if (exact) k_sensor<true><<<pw_blocks(P.plane), PW_THREADS, 0, st>>>(P, Q, phi);
-    else k_sensor<false><<<pw_blocks(P.plane), PW_THREADS, 0, st>>>(P, Q, phi);
+cudaError_t launch_sensor(const DevParams& P, const double* Q, double* phi, cudaStream_t st, bool exact, double* csnd) {
+    if (exact) k_sensor<true><<<pw_blocks(P.plane), PW_THREADS, 0, st>>>(P, Q, phi, nullptr);
+    else launch_after(P, k_sensor<false>, pw_blocks(P.plane), PW_THREADS, st, P, Q, phi, csnd);
     return cudaGetLastError();
 }
 

@@ -31,6 +31,7 @@ __device__ __forceinline__ int face_branch(const DevParams& P, const double* phi
 }
 
 __global__ void __launch_bounds__(256) k_weno_list(const DevParams P, const double* __restrict__ phi, const WenoList w) {
+    after_previous();
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     int g[3] = {0, 0, 0};
     const bool in_grid = c < P.plane;
@@ -157,7 +158,7 @@ __global__ void __launch_bounds__(WF_WARPS * 32, 4) k_weno_faces(const WenoArgs 
 cudaError_t launch_weno(const WenoArgs& a, const double* phi, int sms, cudaStream_t st) {
     const long long most = (long long)a.P.nx * a.P.ny * a.P.nz / WF_FACES + 1;
     const int blocks = most < 4 * sms ? (int)most : 4 * sms;
-    k_weno_list<<<cdiv(a.P.plane, 256), 256, 0, st>>>(a.P, phi, a.w);
+    launch_after(a.P, k_weno_list, cdiv(a.P.plane, 256), 256, st, a.P, phi, a.w);
     if (a.P.character) k_weno_faces<true><<<blocks, WF_WARPS * 32, 0, st>>>(a);
     else k_weno_faces<false><<<blocks, WF_WARPS * 32, 0, st>>>(a);
     return cudaGetLastError();
