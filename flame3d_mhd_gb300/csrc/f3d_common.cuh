@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/flame3d_gpu.h"
+#include "f3d_f64.cuh"
 
 namespace f3d {
 
@@ -93,9 +94,10 @@ struct DevParams {
     double* profb[6];       // their cotangents, accumulated by the adjoint when set
 };
 
-template <class R> __host__ __device__ inline const Cst<R>& cst(const DevParams& P);
-template <> __host__ __device__ inline const Cst<double>& cst<double>(const DevParams& P) { return P.cd; }
-template <> __host__ __device__ inline const Cst<float>& cst<float>(const DevParams& P) { return P.cf; }
+template <class R> __host__ __device__ inline const auto& cst(const DevParams& P) {
+    if constexpr (sizeof(R) == 8) return P.cd;
+    else return P.cf;
+}
 
 __host__ __device__ inline long long lin3(const DevParams& P, int i, int j, int k) {
     return (long long)i + (long long)P.nxt * ((long long)j + (long long)P.nyt * k);
@@ -104,7 +106,10 @@ __host__ __device__ inline long long lin3(const DevParams& P, int i, int j, int 
 // ------------------------------------------------------------------------------------
 // Per-cell physics in FP64 with the reference's operation order. __dmul_rn/__dadd_rn
 // keep nvcc from contracting into FMA so that c2Prim and the ghost rules are bitwise
-// equal to the CPU restatement; the flux arithmetic is free to contract.
+// equal to the CPU restatement; the flux arithmetic is free to contract. mul64 and add64 are the
+// same rounded operations as three-register FMAs (f3d_f64.cuh), for the kernels of every stage.
+__device__ __forceinline__ double mul64(double a, double b) { return F64(f64(a) * f64(b)).v; }
+__device__ __forceinline__ double add64(double a, double b) { return (f64(a) + f64(b)).v; }
 
 // Julia's max(x, e) (a NaN x passes through) for a floor e > 0, on the bit patterns with
 // integer instructions instead of FP64-pipe compares: for x >= 0 the order of doubles is the
@@ -112,7 +117,7 @@ __host__ __device__ inline long long lin3(const DevParams& P, int i, int j, int 
 // NaN has all exponent bits set and a nonzero mantissa. The same value as fmax for every x.
 __device__ __forceinline__ double max_floor(double x, double e) {
     const long long bx = __double_as_longlong(x), be = __double_as_longlong(e);
-    if (be <= 0) return x != x ? x : fmax(x, e);  // a floor of 0 or below
+    if (be <= 0) return x != x ? x : ::fmax(x, e);  // a floor of 0 or below
     return (bx > be || (bx & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL) ? x : e;
 }
 
@@ -120,12 +125,12 @@ __device__ __forceinline__ double max_floor(double x, double e) {
 __device__ __forceinline__ void c2prim_cell(const DevParams& P, const double U[5], double q[6]) {
     const double rho = max_floor(U[0], P.eps_clamp);
     double rinv = 1.0 / rho;
-    double u = __dmul_rn(U[1], rinv), v = __dmul_rn(U[2], rinv), w = __dmul_rn(U[3], rinv);
-    double ke = __dadd_rn(__dadd_rn(__dmul_rn(u, u), __dmul_rn(v, v)), __dmul_rn(w, w));
-    double eraw = __dadd_rn(U[4], -__dmul_rn(__dmul_rn(0.5, rho), ke));
+    double u = mul64(U[1], rinv), v = mul64(U[2], rinv), w = mul64(U[3], rinv);
+    double ke = add64(add64(mul64(u, u), mul64(v, v)), mul64(w, w));
+    double eraw = add64(U[4], -mul64(mul64(constant_here(0.5), rho), ke));
     const double ei = max_floor(eraw, P.eps_clamp);
-    double p = __dmul_rn(P.gm1, ei);
-    double T = p / __dmul_rn(rho, P.rg);
+    double p = mul64(constant_here(P.gm1), ei);
+    double T = p / mul64(rho, constant_here(P.rg));
     q[0] = rho; q[1] = u; q[2] = v; q[3] = w; q[4] = p; q[5] = T;
 }
 
@@ -182,20 +187,21 @@ __device__ __forceinline__ double recip_nr(double x) {
     // the range test on the biased exponent (integer instructions): 2^-119 <= |x| < 2^120
     const unsigned ex = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
     if (ex - 904u > 238u) return 1.0 / x;
-    double r = f32_to_f64(__frcp_rn(f64_to_f32_rn(x)));
-    r = fma(r, fma(-x, r, 1.0), r);
-    return fma(r, fma(-x, r, 1.0), r);
+    F64 r = f64(f32_to_f64(__frcp_rn(f64_to_f32_rn(x))));
+    const F64 one = f64(in_register(1.0));
+    r = r * (one - f64(x) * r) + r;
+    return (r * (one - f64(x) * r) + r).v;
 }
 
 __device__ __forceinline__ void c2prim_cell_fast(const DevParams& P, const double U[5], double q[6]) {
     const double rho = max_floor(U[0], P.eps_clamp);
-    const double rinv = recip_nr(rho);
-    const double u = U[1] * rinv, v = U[2] * rinv, w = U[3] * rinv;
+    const F64 rinv = f64(recip_nr(rho));
+    const F64 m1 = f64(U[1]), m2 = f64(U[2]), m3 = f64(U[3]);
+    const F64 u = m1 * rinv, v = m2 * rinv, w = m3 * rinv;
     // rho |u|^2 / 2 as (momentum . velocity) / 2, folded into the subtraction from E
-    const double eraw = fma(-0.5, U[1] * u + U[2] * v + U[3] * w, U[4]);
-    const double ei = max_floor(eraw, P.eps_clamp);
-    const double p = P.gm1 * ei;
-    q[0] = rho; q[1] = u; q[2] = v; q[3] = w; q[4] = p; q[5] = p * (rinv * P.inv_rg);
+    const F64 eraw = F64(-0.5) * (m1 * u + m2 * v + m3 * w) + f64(U[4]);
+    const F64 p = F64(P.gm1) * f64(max_floor(eraw.v, P.eps_clamp));
+    q[0] = rho; q[1] = u.v; q[2] = v.v; q[3] = w.v; q[4] = p.v; q[5] = F64(p * (rinv * F64(P.inv_rg))).v;
 }
 
 // utils.jl:33-54 prim2c of one cell (also the U of Dirichlet and wall ghosts,

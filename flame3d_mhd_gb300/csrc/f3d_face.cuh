@@ -23,7 +23,8 @@ template <class R> struct CharBasis {
 template <class R>
 __device__ __forceinline__ void char_basis(const DevParams& P, const R* Qr, const R* A0, const R* A1p, const R* A2p, R s0,
                                            long long cl, long long cr, CharBasis<R>& b) {
-    const Cst<R>& K = cst<R>(P);
+    // (F64 has the layout of double)
+    const auto& K = cst<R>(P);
     const long long pl = P.plane;
     const R u = R(0.5) * (Qr[cr + pl] + Qr[cl + pl]);
     const R v = R(0.5) * (Qr[cr + 2 * pl] + Qr[cl + 2 * pl]);
@@ -87,7 +88,6 @@ __device__ __forceinline__ void char_left_row(const CharBasis<R>& b, int n, R l[
 template <class R, class FPA, class FMA>
 __device__ __forceinline__ R char_field_flux(const DevParams& P, const CharBasis<R>& b, int n, int br, int p0, R s0,
                                              FPA FP, FMA FM) {
-    const R tmp1 = R(1) / R(12), tmp2 = R(1) / R(6);
     R l[5];
     char_left_row<R>(b, n, l);
     auto projP = [&](int pos) {
@@ -96,7 +96,10 @@ __device__ __forceinline__ R char_field_flux(const DevParams& P, const CharBasis
     auto projM = [&](int pos) {
         return FM(0, pos) * l[0] + FM(1, pos) * l[1] + FM(2, pos) * l[2] + FM(3, pos) * l[3] + FM(4, pos) * l[4];
     };
-    if constexpr (sizeof(R) == 4) {
+    if constexpr (sizeof(R) == 8) {
+        return weno_pair(br, s0, [&](int k) { return projP(p0 + k); }, [&](int k) { return projM(p0 + 7 - k); });
+    } else {
+        const R tmp1 = R(1) / R(12), tmp2 = R(1) / R(6);
         if (P.ref32) {  // the reference's Float32 reconstruction of the characteristic fields
             if (br == 1) {
                 const double fp = weno7_ref32(projP(p0), projP(p0 + 1), projP(p0 + 2), projP(p0 + 3), projP(p0 + 4),
@@ -109,17 +112,17 @@ __device__ __forceinline__ R char_field_flux(const DevParams& P, const CharBasis
                     weno5_ref32(projM(p0 + 6), projM(p0 + 5), projM(p0 + 4), projM(p0 + 3), projM(p0 + 2), s0)) *
                    tmp2;
         }
+        if (br == 1) {
+            R fp = weno7(projP(p0), projP(p0 + 1), projP(p0 + 2), projP(p0 + 3), projP(p0 + 4), projP(p0 + 5),
+                         projP(p0 + 6), s0);
+            R fm = weno7(projM(p0 + 7), projM(p0 + 6), projM(p0 + 5), projM(p0 + 4), projM(p0 + 3), projM(p0 + 2),
+                         projM(p0 + 1), s0);
+            return (fp + fm) * tmp1;
+        }
+        R fp = weno5(projP(p0 + 1), projP(p0 + 2), projP(p0 + 3), projP(p0 + 4), projP(p0 + 5), s0);
+        R fm = weno5(projM(p0 + 6), projM(p0 + 5), projM(p0 + 4), projM(p0 + 3), projM(p0 + 2), s0);
+        return (fp + fm) * tmp2;
     }
-    if (br == 1) {
-        R fp = weno7(projP(p0), projP(p0 + 1), projP(p0 + 2), projP(p0 + 3), projP(p0 + 4), projP(p0 + 5),
-                     projP(p0 + 6), s0);
-        R fm = weno7(projM(p0 + 7), projM(p0 + 6), projM(p0 + 5), projM(p0 + 4), projM(p0 + 3), projM(p0 + 2),
-                     projM(p0 + 1), s0);
-        return (fp + fm) * tmp1;
-    }
-    R fp = weno5(projP(p0 + 1), projP(p0 + 2), projP(p0 + 3), projP(p0 + 4), projP(p0 + 5), s0);
-    R fm = weno5(projM(p0 + 6), projM(p0 + 5), projM(p0 + 4), projM(p0 + 3), projM(p0 + 2), s0);
-    return (fp + fm) * tmp2;
 }
 
 // Component k of the face flux R f from the five characteristic fluxes (schemes.jl:960-999):
@@ -139,8 +142,10 @@ __device__ __forceinline__ R char_right_row(const CharBasis<R>& b, int k, const 
 // Component n of a component-wise WENO7 (schemes.jl:143-230) / WENO5 (:231-276) face
 template <class R, class FPA, class FMA>
 __device__ __forceinline__ R comp_field_flux(const DevParams& P, int n, int br, int p0, R s0, FPA FP, FMA FM) {
-    const R tmp1 = R(1) / R(12), tmp2 = R(1) / R(6);
-    if constexpr (sizeof(R) == 4) {
+    if constexpr (sizeof(R) == 8) {
+        return weno_pair(br, s0, [&](int k) { return FP(n, p0 + k); }, [&](int k) { return FM(n, p0 + 7 - k); });
+    } else {
+        const R tmp1 = R(1) / R(12), tmp2 = R(1) / R(6);
         if (P.ref32) {  // the reference's Float32 reconstruction
             if (br == 1) {
                 const double fp = weno7_ref32(FP(n, p0), FP(n, p0 + 1), FP(n, p0 + 2), FP(n, p0 + 3), FP(n, p0 + 4),
@@ -153,17 +158,17 @@ __device__ __forceinline__ R comp_field_flux(const DevParams& P, int n, int br, 
                     weno5_ref32(FM(n, p0 + 6), FM(n, p0 + 5), FM(n, p0 + 4), FM(n, p0 + 3), FM(n, p0 + 2), s0)) *
                    tmp2;
         }
+        if (br == 1) {
+            R fp = weno7(FP(n, p0), FP(n, p0 + 1), FP(n, p0 + 2), FP(n, p0 + 3), FP(n, p0 + 4), FP(n, p0 + 5),
+                         FP(n, p0 + 6), s0);
+            R fm = weno7(FM(n, p0 + 7), FM(n, p0 + 6), FM(n, p0 + 5), FM(n, p0 + 4), FM(n, p0 + 3), FM(n, p0 + 2),
+                         FM(n, p0 + 1), s0);
+            return (fp + fm) * tmp1;
+        }
+        R fp = weno5(FP(n, p0 + 1), FP(n, p0 + 2), FP(n, p0 + 3), FP(n, p0 + 4), FP(n, p0 + 5), s0);
+        R fm = weno5(FM(n, p0 + 6), FM(n, p0 + 5), FM(n, p0 + 4), FM(n, p0 + 3), FM(n, p0 + 2), s0);
+        return (fp + fm) * tmp2;
     }
-    if (br == 1) {
-        R fp = weno7(FP(n, p0), FP(n, p0 + 1), FP(n, p0 + 2), FP(n, p0 + 3), FP(n, p0 + 4), FP(n, p0 + 5),
-                     FP(n, p0 + 6), s0);
-        R fm = weno7(FM(n, p0 + 7), FM(n, p0 + 6), FM(n, p0 + 5), FM(n, p0 + 4), FM(n, p0 + 3), FM(n, p0 + 2),
-                     FM(n, p0 + 1), s0);
-        return (fp + fm) * tmp1;
-    }
-    R fp = weno5(FP(n, p0 + 1), FP(n, p0 + 2), FP(n, p0 + 3), FP(n, p0 + 4), FP(n, p0 + 5), s0);
-    R fm = weno5(FM(n, p0 + 6), FM(n, p0 + 5), FM(n, p0 + 4), FM(n, p0 + 3), FM(n, p0 + 2), s0);
-    return (fp + fm) * tmp2;
 }
 
 // Face flux of one face from the split fluxes of the 8 cells around it, positions
@@ -173,7 +178,7 @@ __device__ __forceinline__ R comp_field_flux(const DevParams& P, int n, int br, 
 template <bool CHAR, class R, class FPA, class FMA>
 __device__ __forceinline__ void face_flux(const DevParams& P, const SweepArgs& a, int br, int p0, R s0,
                                           long long cl, long long cr, FPA FP, FMA FM, R out[5]) {
-    const Cst<R>& K = cst<R>(P);
+    const auto& K = cst<R>(P);
     if (br == 0) {  // UP7, schemes.jl:119-142
         const R c1 = K.lin[0], c2 = K.lin[1], c3 = K.lin[2], c4 = K.lin[3], c5 = K.lin[4], c6 = K.lin[5],
                 c7 = K.lin[6];
@@ -223,9 +228,9 @@ __device__ __forceinline__ void face_flux(const DevParams& P, const SweepArgs& a
 // Sound speed for the split: precomputed per cell in FP64; computed in place in FP32.
 template <class R> __device__ __forceinline__ R split_sound(const DevParams& P, const SweepArgs& a, long long c,
                                                             const R q[6]);
-template <> __device__ __forceinline__ double split_sound<double>(const DevParams&, const SweepArgs& a, long long c,
-                                                                  const double*) {
-    return static_cast<const double*>(a.csnd)[c];
+template <> __device__ __forceinline__ F64 split_sound<F64>(const DevParams&, const SweepArgs& a, long long c,
+                                                            const F64*) {
+    return f64(static_cast<const double*>(a.csnd)[c]);
 }
 __device__ __forceinline__ float split_sound32(const DevParams& P, const float* q) {
     return P.split == F3D_SPLIT_SW ? sqrtf(P.cf.grg * q[5]) : sqrtf(P.cf.gamma * q[4] / q[0]);

@@ -4,6 +4,7 @@
 // and the accumulation selected by out_mode (OUT_SET / OUT_ADD into acc, OUT_RHS = J *
 // (acc + d), OUT_STAGE = the RK update of div.jl plus linComb, utils.jl:57-70).
 #pragma once
+#include "f3d_f64.cuh"
 #include "f3d_kernels.cuh"
 
 namespace f3d {
@@ -48,6 +49,7 @@ template <int DIR, int TL, int TC, int NTHREADS, class R, class CellFn, class Fi
 __device__ __forceinline__ void sweep_epilogue(const SweepArgs& a, const R* sF, int c0, int l0, int other, int nc,
                                                int nl, const CellFn& cell, const FidxFn& fidx) {
     constexpr int NF = TC + 1;
+    using A = typename Arith<R>::type;
     const DevParams& P = a.P;
     const long long pl = P.plane;
     // cells t = 0..nc-1 (full position c0 + t + NG)
@@ -60,9 +62,9 @@ __device__ __forceinline__ void sweep_epilogue(const SweepArgs& a, const R* sF, 
         if (DIR == 0) { l = it / TC; t = it - l * TC; } else { t = it / TL; l = it - t * TL; }
         if (l >= nl || t >= nc) continue;
         const long long c = cell(l, c0 + t + NG);
-        R d[5];
+        A d[5];
 #pragma unroll
-        for (int n = 0; n < 5; n++) d[n] = sF[n * TL * NF + fidx(l, t)] - sF[n * TL * NF + fidx(l, t + 1)];
+        for (int n = 0; n < 5; n++) d[n] = arith(sF[n * TL * NF + fidx(l, t)]) - arith(sF[n * TL * NF + fidx(l, t + 1)]);
         if (Fvr) {
             // Fv index = full index - 2 in every dimension (viscous.jl:119, div.jl:14-39)
             long long vi, vj, vk;
@@ -72,11 +74,11 @@ __device__ __forceinline__ void sweep_epilogue(const SweepArgs& a, const R* sF, 
             else { vi = l0 + l + NG - 2; vj = other + NG - 2; vk = g; }
             const long long vc = vi + (long long)vxt * (vj + (long long)vyt * vk);
             const long long vs = DIR == 0 ? 1 : (DIR == 1 ? (long long)vxt : (long long)vxt * vyt);
-            const R k1 = R(1) / R(12), k2 = R(-2) / R(3);
+            const A k1 = A(1.0 / 12.0), k2 = A(-2.0 / 3.0);
 #pragma unroll
             for (int n = 0; n < 4; n++) {
                 const R* F = Fvr + n * vplane + vc;
-                d[n + 1] += k1 * (F[-2 * vs] - F[2 * vs]) + k2 * (F[-vs] - F[vs]);
+                d[n + 1] += k1 * (arith(F[-2 * vs]) - arith(F[2 * vs])) + k2 * (arith(F[-vs]) - arith(F[vs]));
             }
         }
         if constexpr (sizeof(R) == 4) {
@@ -105,31 +107,34 @@ __device__ __forceinline__ void sweep_epilogue(const SweepArgs& a, const R* sF, 
         // and eta sweeps' FP32 differences and this sweep's summed with compensation, so the
         // result is the exact sum rounded once to FP32 (relative to the sum, not to the terms
         // that cancel in it)
-        auto total = [&](int n) -> double {
+        auto total = [&](int n) -> F64 {
             if constexpr (sizeof(R) == 4) {
-                if (a.acc2) return to_f64(sum3_compensated(acc[c + n * pl], a.acc2[c + n * pl], d[n]));
+                if (a.acc2) return f64(to_f64(sum3_compensated(acc[c + n * pl], a.acc2[c + n * pl], d[n])));
+                return f64(to_f64(acc[c + n * pl] + d[n]));
+            } else {
+                return arith(acc[c + n * pl]) + d[n];
             }
-            return to_f64(acc[c + n * pl] + d[n]);
         };
         if (a.out_mode == OUT_SET) {
 #pragma unroll
-            for (int n = 0; n < 5; n++) acc[c + n * pl] = d[n];
+            for (int n = 0; n < 5; n++) acc[c + n * pl] = plain(d[n]);
         } else if (a.out_mode == OUT_ADD) {
 #pragma unroll
-            for (int n = 0; n < 5; n++) acc[c + n * pl] += d[n];
+            for (int n = 0; n < 5; n++) acc[c + n * pl] = plain(arith(acc[c + n * pl]) + d[n]);
         } else if (a.out_mode == OUT_RHS) {
-            const double Jc = a.J[c];
+            const F64 Jc = f64(a.J[c]);
 #pragma unroll
-            for (int n = 0; n < 5; n++) a.out[c + n * pl] = Jc * total(n);
+            for (int n = 0; n < 5; n++) a.out[c + n * pl] = F64(Jc * total(n)).v;
         } else {  // OUT_STAGE: RK state accumulation in FP64
-            const double Jact = a.J[c] * (a.dtl ? a.dtl[c] : a.dt);  // div_LTS: per-cell dt
+            const F64 Jact = f64(a.J[c]) * (a.dtl ? f64(a.dtl[c]) : F64(a.dt));  // div_LTS: per-cell dt
+            const F64 ca = a.ca, cb = a.cb;
 #pragma unroll
             for (int n = 0; n < 5; n++) {
-                const double u = a.U[c + n * pl];
-                if (a.stage1_copy) a.Un[c + n * pl] = u;
-                double un = u + total(n) * Jact;
-                if (a.combine) un = un * a.ca + a.Un[c + n * pl] * a.cb;
-                a.U[c + n * pl] = un;
+                const F64 u = f64(a.U[c + n * pl]);
+                if (a.stage1_copy) a.Un[c + n * pl] = u.v;
+                F64 un = u + total(n) * Jact;
+                if (a.combine) un = un * ca + f64(a.Un[c + n * pl]) * cb;
+                a.U[c + n * pl] = un.v;
             }
         }
     }

@@ -92,84 +92,84 @@ cudaError_t launch_face_geometry(const DevParams& P, const double* x, const doub
 // min / max that return NaN when either argument is NaN, as Julia's min and max do (the
 // reference's wave-speed estimates): fmin/fmax would drop a NaN Roe speed and hide a
 // negative reconstructed density from the non-finite check.
-__device__ __forceinline__ double nan_min(double a, double b) { return a != a ? a : (b != b ? b : (b < a ? b : a)); }
-__device__ __forceinline__ double nan_max(double a, double b) { return a != a ? a : (b != b ? b : (a < b ? b : a)); }
+__device__ __forceinline__ F64 nan_min(F64 a, F64 b) { return a != a ? a : (b != b ? b : (b < a ? b : a)); }
+__device__ __forceinline__ F64 nan_max(F64 a, F64 b) { return a != a ? a : (b != b ? b : (a < b ? b : a)); }
 
 // HLLC flux along the unit normal n of the conserved states UL, UR (FVM.jl:1224-1357)
-__device__ __forceinline__ void hllc(const DevParams& P, const double UL[5], const double UR[5], double nx,
-                                     double ny, double nz, double F[5]) {
-    const double g = P.gamma, gm = P.gm1;
-    const double rL = UL[0], irL = 1.0 / rL;
-    const double uL = UL[1] * irL, vL = UL[2] * irL, wL = UL[3] * irL, EL = UL[4];
-    const double pL = gm * (EL - 0.5 * rL * (uL * uL + vL * vL + wL * wL));
-    const double cL = sqrt(fabs(g * pL * irL));
-    const double qL = uL * nx + vL * ny + wL * nz;
-    const double rR = UR[0], irR = 1.0 / rR;
-    const double uR = UR[1] * irR, vR = UR[2] * irR, wR = UR[3] * irR, ER = UR[4];
-    const double pR = gm * (ER - 0.5 * rR * (uR * uR + vR * vR + wR * wR));
-    const double cR = sqrt(fabs(g * pR * irR));
-    const double qR = uR * nx + vR * ny + wR * nz;
-    const double sL = sqrt(rL), sR = sqrt(rR), isum = 1.0 / (sL + sR);
-    const double ur = (sL * uL + sR * uR) * isum, vr = (sL * vL + sR * vR) * isum, wr = (sL * wL + sR * wR) * isum;
-    const double qr = ur * nx + vr * ny + wr * nz;
-    const double HL = (EL + pL) * irL, HR = (ER + pR) * irR;
-    const double Hr = (sL * HL + sR * HR) * isum;
-    const double cr = sqrt(fabs(gm * (Hr - 0.5 * (ur * ur + vr * vr + wr * wr))));
-    const double SL = nan_min(qL - cL, qr - cr);
-    const double SR = nan_max(qR + cR, qr + cr);
-    const double Ss = (pR - pL + rL * qL * (SL - qL) - rR * qR * (SR - qR)) / (rL * (SL - qL) - rR * (SR - qR) + 1e-12);
-    const bool left = SL >= 0.0 || (SR > 0.0 && Ss >= 0.0);
-    const double r = left ? rL : rR, u = left ? uL : uR, v = left ? vL : vR, w = left ? wL : wR;
-    const double E = left ? EL : ER, p = left ? pL : pR, q = left ? qL : qR;
-    F[0] = r * q;
-    F[1] = r * u * q + p * nx;
-    F[2] = r * v * q + p * ny;
-    F[3] = r * w * q + p * nz;
+__device__ __forceinline__ void hllc(const DevParams& P, const F64 UL[5], const F64 UR[5], F64 nx, F64 ny, F64 nz,
+                                     F64 F[5]) {
+    const F64 g = P.gamma, gm = P.gm1, half = 0.5;
+    const F64 rL = UL[0], irL = recip(rL);
+    const F64 uL = UL[1] * irL, vL = UL[2] * irL, wL = UL[3] * irL, EL = UL[4];
+    const F64 pL = gm * (EL - (half * rL) * (uL * uL + vL * vL + wL * wL));
+    const F64 cL = sqrt(fabs((g * pL) * irL));
+    const F64 qL = uL * nx + vL * ny + wL * nz;
+    const F64 rR = UR[0], irR = recip(rR);
+    const F64 uR = UR[1] * irR, vR = UR[2] * irR, wR = UR[3] * irR, ER = UR[4];
+    const F64 pR = gm * (ER - (half * rR) * (uR * uR + vR * vR + wR * wR));
+    const F64 cR = sqrt(fabs((g * pR) * irR));
+    const F64 qR = uR * nx + vR * ny + wR * nz;
+    // Roe averages (sqrt(rL) a + sqrt(rR) b) / (sqrt(rL) + sqrt(rR)) = b + k (a - b) with
+    // k = 1 / (1 + sqrt(rR / rL)): one root and one reciprocal; two negative densities, whose roots
+    // are NaN in the reference, give NaN too
+    F64 ratio = rR * irL;
+    if ((__double2hiint(rL.v) | __double2hiint(rR.v)) < 0 && rL.v != 0.0 && rR.v != 0.0)
+        ratio = f64(__longlong_as_double(0x7ff8000000000000ll));
+    const F64 k = recip(F64(1.0) + sqrt(ratio));
+    const F64 ur = uR + k * (uL - uR), vr = vR + k * (vL - vR), wr = wR + k * (wL - wR);
+    const F64 qr = ur * nx + vr * ny + wr * nz;
+    const F64 HL = (EL + pL) * irL, HR = (ER + pR) * irR;
+    const F64 Hr = HR + k * (HL - HR);
+    const F64 cr = sqrt(fabs(gm * (Hr - half * (ur * ur + vr * vr + wr * wr))));
+    const F64 SL = nan_min(qL - cL, qr - cr);
+    const F64 SR = nan_max(qR + cR, qr + cr);
+    const F64 mL = rL * (SL - qL), mR = rR * (SR - qR);
+    const F64 Ss = (pR - pL + mL * qL - mR * qR) / (mL - mR + F64(1e-12));
+    const F64 zero = 0.0;
+    const bool left = SL >= zero || (SR > zero && Ss >= zero);
+    const F64 r = left ? rL : rR, u = left ? uL : uR, v = left ? vL : vR, w = left ? wL : wR;
+    const F64 E = left ? EL : ER, p = left ? pL : pR, q = left ? qL : qR;
+    const F64 rq = r * q;
+    F[0] = rq;
+    F[1] = rq * u + p * nx;
+    F[2] = rq * v + p * ny;
+    F[3] = rq * w + p * nz;
     F[4] = (E + p) * q;
-    if (SL >= 0.0 || SR <= 0.0) return;  // supersonic: the upwind state's physical flux
+    if (SL >= zero || SR <= zero) return;  // supersonic: the upwind state's physical flux
     // star state of the side: F* = F + S (U* - U)
-    const double S = left ? SL : SR, ir = left ? irL : irR;
-    const double* Us = left ? UL : UR;
-    const double f = r * (S - q) / (S - Ss);
-    const double st[5] = {f, f * (u + (Ss - q) * nx), f * (v + (Ss - q) * ny), f * (w + (Ss - q) * nz),
-                          f * (E * ir + (Ss - q) * (Ss + p / (r * (S - q))))};
+    const F64 S = left ? SL : SR, ir = left ? irL : irR, m = left ? mL : mR;  // m = r (S - q)
+    const F64* Us = left ? UL : UR;
+    const F64 f = m / (S - Ss), dS = Ss - q;
+    const F64 fd = f * dS;
+    const F64 st[5] = {f, f * u + fd * nx, f * v + fd * ny, f * w + fd * nz, f * (E * ir) + fd * (Ss + p / m)};
 #pragma unroll
     for (int n = 0; n < 5; n++) F[n] += S * (st[n] - Us[n]);
 }
 
-// WENO7 / WENO5 / minmod of one side on a seven-point stencil in upwind order (FVM.jl)
-__device__ __forceinline__ double fvm_weno7(const double V[7], double ss) {
-    const double V1 = V[0], V2 = V[1], V3 = V[2], V4 = V[3], V5 = V[4], V6 = V[5], V7 = V[6];
-    const double q1 = -3.0 * V1 + 13.0 * V2 - 23.0 * V3 + 25.0 * V4;
-    const double q2 = V2 - 5.0 * V3 + 13.0 * V4 + 3.0 * V5;
-    const double q3 = -V3 + 7.0 * V4 + 7.0 * V5 - V6;
-    const double q4 = 3.0 * V4 + 13.0 * V5 - 5.0 * V6 + V7;
-    double Is[4];  // the smoothness indicators in difference form (weno7_is, f3d_flux.cuh)
-    weno7_is<double>(V, Is);
-    const double I1 = Is[0], I2 = Is[1], I3 = Is[2], I4 = Is[3];
-    // alpha_k = d_k / t_k^2 with t_k = 1e-10 + IS_k ss, normalised: one divide
-    const double t1 = 1e-10 + I1 * ss, t2 = 1e-10 + I2 * ss, t3 = 1e-10 + I3 * ss, t4 = 1e-10 + I4 * ss;
-    return weno7_combine(t1, t2, t3, t4, q1, q2, q3, q4) * (1.0 / 12.0);
-}
-__device__ __forceinline__ double fvm_weno5(const double V[7], double ss) {
-    const double a = V[1], b = V[2], c = V[3], d = V[4], e = V[5];
-    double t1 = a - 2.0 * b + c, t2 = a - 4.0 * b + 3.0 * c;
-    const double s1 = 13.0 * t1 * t1 + 3.0 * t2 * t2;
-    t1 = b - 2.0 * c + d;
-    t2 = b - d;
-    const double s2 = 13.0 * t1 * t1 + 3.0 * t2 * t2;
-    t1 = c - 2.0 * d + e;
-    t2 = 3.0 * c - 4.0 * d + e;
-    const double s3 = 13.0 * t1 * t1 + 3.0 * t2 * t2;
-    const double v1 = 2.0 * a - 7.0 * b + 11.0 * c, v2 = -b + 5.0 * c + 2.0 * d, v3 = 2.0 * c + 5.0 * d - e;
-    return weno5_combine(1e-8 + s1 * ss, 1e-8 + s2 * ss, 1e-8 + s3 * ss, v1, v2, v3) * (1.0 / 6.0);
-}
-// br 1 = WENO7, 2 = WENO5, 3 = minmod; the two sides' minmod forms as FVM.jl:204-205
-__device__ __forceinline__ double fvm_side(int br, bool right, const double V[7], double ss) {
-    if (br == 1) return fvm_weno7(V, ss);
-    if (br == 2) return fvm_weno5(V, ss);
-    if (right) return V[3] - 0.5 * minmod(V[3] - V[2], V[3] - V[4]);
-    return V[3] + 0.5 * minmod(V[3] - V[2], V[4] - V[3]);
+// The two sides of a face on seven-point stencils in upwind order (FVM.jl): br 1 = WENO7 (its own
+// eps 1e-10), 2 = WENO5 (1e-8), 3 = minmod in the two sides' forms of FVM.jl:204-205. The nonlinear
+// sums are those of the finite-difference faces (f3d_flux.cuh); the two values share one reciprocal.
+__device__ __forceinline__ void fvm_sides(int br, const F64 L[7], const F64 R[7], F64 ss, F64& l, F64& r) {
+    if (br == 3) {
+        l = L[3] + F64(0.5) * minmod(F64(L[3] - L[2]), F64(L[4] - L[3]));
+        r = R[3] - F64(0.5) * minmod(F64(R[3] - R[2]), F64(R[3] - R[4]));
+        return;
+    }
+    auto VL = [&](int k) { return L[k]; };
+    auto VR = [&](int k) { return R[k]; };
+    const WenoSums a = br == 1 ? weno7_sums(VL, ss, 1e-10) : weno5_sums(VL, ss, 1e-8);
+    const WenoSums b = br == 1 ? weno7_sums(VR, ss, 1e-10) : weno5_sums(VR, ss, 1e-8);
+    const F64 unit = br == 1 ? F64(1.0 / 12.0) : F64(1.0 / 6.0);
+    const F64 D = a.D * b.D;
+    const unsigned e = ((unsigned)__double2hiint(D.v) >> 20) & 0x7ffu;
+    if (e - 23u > 1800u) {
+        l = a.base + unit * (a.N / a.D);
+        r = b.base + unit * (b.N / b.D);
+        return;
+    }
+    const F64 i = unit * recip_step(D.v);
+    l = a.base + (a.N * b.D) * i;
+    r = b.base + (b.N * a.D) * i;
 }
 
 // ------------------------------------------------------------------------------------
@@ -248,15 +248,15 @@ __global__ void __launch_bounds__(FvmLaunch<EIGEN>::NT, FvmLaunch<EIGEN>::MINB) 
     // Phase B: face t between positions t+3 (left cell, the kernels' i) and t+4
     auto face = [&](int l, int t, int br) {
         const long long cl = cell(l, c0 + t + 3);
-        auto Uv = [&](int n, int p) { return sU[n * TL * NP + sidx(l, p)]; };
-        const double nx = gnx[cl], ny = gny[cl], nz = gnz[cl];
-        double UL[5], UR[5];
+        auto Uv = [&](int n, int p) { return f64(sU[n * TL * NP + sidx(l, p)]); };
+        const F64 nx = f64(gnx[cl]), ny = f64(gny[cl]), nz = f64(gnz[cl]);
+        F64 UL[5], UR[5];
         if (br == 0) {  // linear scheme on U, FVM.jl:42-60
 #pragma unroll
             for (int n = 0; n < 5; n++) {
-                double vl = 0.0, vr = 0.0;
+                F64 vl = P.cd.lin[0] * Uv(n, t), vr = P.cd.lin[0] * Uv(n, t + 7);
 #pragma unroll
-                for (int m = 0; m < 7; m++) {
+                for (int m = 1; m < 7; m++) {
                     vl += P.cd.lin[m] * Uv(n, t + m);
                     vr += P.cd.lin[m] * Uv(n, t + 7 - m);
                 }
@@ -264,84 +264,80 @@ __global__ void __launch_bounds__(FvmLaunch<EIGEN>::NT, FvmLaunch<EIGEN>::MINB) 
                 UR[n] = vr;
             }
         } else {
-            const double ss = 2.0 / (S[cl + stride] + S[cl]);
+            const F64 ss = F64(2.0) / (f64(S[cl + stride]) + f64(S[cl]));
             if (!EIGEN) {  // Conser_reconstruct, FVM.jl:739-855
 #pragma unroll
                 for (int n = 0; n < 5; n++) {
-                    double VL[7], VR[7];
+                    F64 VL[7], VR[7];
 #pragma unroll
                     for (int m = 0; m < 7; m++) {
                         VL[m] = Uv(n, t + m);
                         VR[m] = Uv(n, t + 7 - m);
                     }
-                    UL[n] = fvm_side(br, false, VL, ss);
-                    UR[n] = fvm_side(br, true, VR, ss);
+                    fvm_sides(br, VL, VR, ss, UL[n], UR[n]);
                 }
             } else {  // Eigen_reconstruct, FVM.jl:65-228
-                const double rl = Q[cl], rr = Q[cl + stride];
-                const double srl = sqrt(rl), srr = sqrt(rr), isr = 1.0 / (srl + srr);
-                const double u = (srl * Q[cl + pl] + srr * Q[cl + stride + pl]) * isr;
-                const double v = (srl * Q[cl + 2 * pl] + srr * Q[cl + stride + 2 * pl]) * isr;
-                const double w = (srl * Q[cl + 3 * pl] + srr * Q[cl + stride + 3 * pl]) * isr;
-                const double gg = P.gamma / P.gm1;
+                auto Qv = [&](int n, long long c) { return f64(Q[c + n * pl]); };
+                const long long cr = cl + stride;
+                const F64 srl = sqrt(Qv(0, cl)), srr = sqrt(Qv(0, cr)), isr = recip(srl + srr);
+                const F64 half = 0.5;
+                auto roe = [&](F64 a, F64 b) { return F64((srl * a + srr * b) * isr); };
+                const F64 u = roe(Qv(1, cl), Qv(1, cr)), v = roe(Qv(2, cl), Qv(2, cr)), w = roe(Qv(3, cl), Qv(3, cr));
+                const F64 gg = P.gamma / P.gm1;
                 auto Hof = [&](long long c) {
-                    const double uu = Q[c + pl], vv = Q[c + 2 * pl], ww = Q[c + 3 * pl];
-                    return gg * Q[c + 4 * pl] / Q[c] + 0.5 * (uu * uu + vv * vv + ww * ww);
+                    const F64 uu = Qv(1, c), vv = Qv(2, c), ww = Qv(3, c);
+                    return gg * Qv(4, c) / Qv(0, c) + half * (uu * uu + vv * vv + ww * ww);
                 };
-                const double H = (srl * Hof(cl) + srr * Hof(cl + stride)) * isr;
-                const double v2 = 0.5 * (u * u + v * v + w * w);
-                const double c = sqrt(P.gm1 * (H - v2));
-                double lx, ly, lz;
+                const F64 H = roe(Hof(cl), Hof(cr));
+                const F64 v2 = half * (u * u + v * v + w * w);
+                const F64 c = sqrt(P.gm1 * (H - v2));
+                F64 lx, ly, lz;
                 if (fabs(nz) <= fabs(ny)) {
-                    const double id = 1.0 / sqrt(nx * nx + ny * ny + 1e-12);
-                    lx = -ny * id; ly = nx * id; lz = 0.0;
+                    const F64 id = rsq(nx * nx + ny * ny + F64(1e-12));
+                    lx = -ny * id; ly = nx * id; lz = F64(0.0);
                 } else {
-                    const double id = 1.0 / sqrt(nx * nx + nz * nz + 1e-12);
-                    lx = -nz * id; ly = 0.0; lz = nx * id;
+                    const F64 id = rsq(nx * nx + nz * nz + F64(1e-12));
+                    lx = -nz * id; ly = F64(0.0); lz = nx * id;
                 }
-                const double mx = ny * lz - nz * ly, my = nz * lx - nx * lz, mz = nx * ly - ny * lx;
-                const double invc = 1.0 / c, invc2 = invc * invc, K = P.gm1;
-                const double Ku = K * u * invc2, Kv = K * v * invc2, Kw = K * w * invc2;
-                const double Kv2 = K * v2 * invc2, Kc2 = K * invc2;
-                const double un = u * nx + v * ny + w * nz, ul = u * lx + v * ly + w * lz,
-                             um = u * mx + v * my + w * mz;
-                const double uni = un * invc, nxi = nx * invc, nyi = ny * invc, nzi = nz * invc;
+                const F64 mx = ny * lz - nz * ly, my = nz * lx - nx * lz, mz = nx * ly - ny * lx;
+                const F64 invc = recip(c), invc2 = invc * invc, K = P.gm1;
+                const F64 Kc2 = K * invc2, Ku = Kc2 * u, Kv = Kc2 * v, Kw = Kc2 * w, Kv2 = Kc2 * v2;
+                const F64 un = u * nx + v * ny + w * nz, ul = u * lx + v * ly + w * lz, um = u * mx + v * my + w * mz;
+                const F64 uni = un * invc, nxi = nx * invc, nyi = ny * invc, nzi = nz * invc;
 #pragma unroll
-                for (int q = 0; q < 5; q++) { UL[q] = 0.0; UR[q] = 0.0; }
+                for (int q = 0; q < 5; q++) { UL[q] = F64(0.0); UR[q] = F64(0.0); }
 #pragma unroll 1
                 for (int n = 0; n < 5; n++) {
-                    double ln[5], rn[5];
-                    if (n == 0) {
-                        ln[0] = 0.5 * (Kv2 + uni); ln[1] = -0.5 * (Ku + nxi); ln[2] = -0.5 * (Kv + nyi);
-                        ln[3] = -0.5 * (Kw + nzi); ln[4] = 0.5 * Kc2;
-                        rn[0] = 1.0; rn[1] = u - nx * c; rn[2] = v - ny * c; rn[3] = w - nz * c; rn[4] = H - un * c;
+                    F64 ln[5], rn[5];
+                    if (n == 0 || n == 2) {
+                        const F64 sg = n == 0 ? F64(1.0) : F64(-1.0), sc = sg * c;
+                        ln[0] = half * (Kv2 + sg * uni); ln[1] = -half * (Ku + sg * nxi); ln[2] = -half * (Kv + sg * nyi);
+                        ln[3] = -half * (Kw + sg * nzi); ln[4] = half * Kc2;
+                        rn[0] = F64(1.0); rn[1] = u - nx * sc; rn[2] = v - ny * sc; rn[3] = w - nz * sc; rn[4] = H - un * sc;
                     } else if (n == 1) {
-                        ln[0] = 1.0 - Kv2; ln[1] = Ku; ln[2] = Kv; ln[3] = Kw; ln[4] = -Kc2;
-                        rn[0] = 1.0; rn[1] = u; rn[2] = v; rn[3] = w; rn[4] = v2;
-                    } else if (n == 2) {
-                        ln[0] = 0.5 * (Kv2 - uni); ln[1] = -0.5 * (Ku - nxi); ln[2] = -0.5 * (Kv - nyi);
-                        ln[3] = -0.5 * (Kw - nzi); ln[4] = 0.5 * Kc2;
-                        rn[0] = 1.0; rn[1] = u + nx * c; rn[2] = v + ny * c; rn[3] = w + nz * c; rn[4] = H + un * c;
+                        ln[0] = F64(1.0) - Kv2; ln[1] = Ku; ln[2] = Kv; ln[3] = Kw; ln[4] = -Kc2;
+                        rn[0] = F64(1.0); rn[1] = u; rn[2] = v; rn[3] = w; rn[4] = v2;
                     } else if (n == 3) {
-                        ln[0] = -ul; ln[1] = lx; ln[2] = ly; ln[3] = lz; ln[4] = 0.0;
-                        rn[0] = 0.0; rn[1] = lx; rn[2] = ly; rn[3] = lz; rn[4] = ul;
+                        ln[0] = -ul; ln[1] = lx; ln[2] = ly; ln[3] = lz; ln[4] = F64(0.0);
+                        rn[0] = F64(0.0); rn[1] = lx; rn[2] = ly; rn[3] = lz; rn[4] = ul;
                     } else {
-                        ln[0] = -um; ln[1] = mx; ln[2] = my; ln[3] = mz; ln[4] = 0.0;
-                        rn[0] = 0.0; rn[1] = mx; rn[2] = my; rn[3] = mz; rn[4] = um;
+                        ln[0] = -um; ln[1] = mx; ln[2] = my; ln[3] = mz; ln[4] = F64(0.0);
+                        rn[0] = F64(0.0); rn[1] = mx; rn[2] = my; rn[3] = mz; rn[4] = um;
                     }
-                    double VL[7], VR[7];
+                    F64 VL[7], VR[7];
 #pragma unroll
                     for (int m = 0; m < 7; m++) {
-                        double sl = 0.0, sr = 0.0;
+                        F64 sl = ln[0] * Uv(0, t + m), sr = ln[0] * Uv(0, t + 7 - m);
 #pragma unroll
-                        for (int q = 0; q < 5; q++) {
+                        for (int q = 1; q < 5; q++) {
                             sl += ln[q] * Uv(q, t + m);
                             sr += ln[q] * Uv(q, t + 7 - m);
                         }
                         VL[m] = sl;
                         VR[m] = sr;
                     }
-                    const double vl = fvm_side(br, false, VL, ss), vr = fvm_side(br, true, VR, ss);
+                    F64 vl, vr;
+                    fvm_sides(br, VL, VR, ss, vl, vr);
 #pragma unroll
                     for (int q = 0; q < 5; q++) {
                         UL[q] += rn[q] * vl;
@@ -350,12 +346,12 @@ __global__ void __launch_bounds__(FvmLaunch<EIGEN>::NT, FvmLaunch<EIGEN>::MINB) 
                 }
             }
         }
-        double Ff[5];
+        const F64 ar = f64(gar[cl]);
+        F64 Ff[5];
         hllc(P, UL, UR, nx, ny, nz, Ff);
-        const double ar = gar[cl];
         const int f = fidx(l, t);
 #pragma unroll
-        for (int n = 0; n < 5; n++) sF[n * TL * NF + f] = Ff[n] * ar;
+        for (int n = 0; n < 5; n++) sF[n * TL * NF + f] = F64(Ff[n] * ar).v;
         if (a.faces) {  // face-flux output in the reference's Fx/Fy/Fz shape
             const long long fx = P.nx + (DIR == 0), fy = P.ny + (DIR == 1), fz = P.nz + (DIR == 2);
             long long fi, fj, fk;
@@ -364,7 +360,7 @@ __global__ void __launch_bounds__(FvmLaunch<EIGEN>::NT, FvmLaunch<EIGEN>::MINB) 
             else { fi = l0 + l; fj = other; fk = c0 + t; }
             const long long fo = fi + fx * (fj + fy * fk), nf = fx * fy * fz;
 #pragma unroll
-            for (int n = 0; n < 5; n++) a.faces[fo + n * nf] = Ff[n] * ar;
+            for (int n = 0; n < 5; n++) a.faces[fo + n * nf] = F64(Ff[n] * ar).v;
         }
     };
     for (int it = threadIdx.x; it < TL * NF; it += FVM_THREADS) {

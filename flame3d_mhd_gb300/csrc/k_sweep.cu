@@ -65,6 +65,7 @@ template <int DIR, bool CHAR, class R>
 __global__ void __launch_bounds__(Tile<DIR, R>::NT, Tile<DIR, R>::MINB) k_sweep(const SweepArgs a) {
     constexpr int TL = Tile<DIR, R>::TL, TC = Tile<DIR, R>::TC, NP = TC + 8, NF = TC + 1;
     constexpr int SWEEP_THREADS = Tile<DIR, R>::NT;
+    using A = typename Arith<R>::type;
     const DevParams& P = a.P;
     const bool hybrid = P.fixed_branch < 0;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -106,17 +107,17 @@ __global__ void __launch_bounds__(Tile<DIR, R>::NT, Tile<DIR, R>::MINB) k_sweep(
         if (DIR == 0) { l = it / NP; p = it - l * NP; } else { p = it / TL; l = it - p * TL; }
         if (l >= nl || p >= nc + 8) continue;
         const long long c = cell(l, c0 + p);
-        R q[6];
+        A q[6];
 #pragma unroll
-        for (int n = 0; n < 6; n++) q[n] = Qr[c + n * pl];
-        R fp[5], fm[5];
-        split_cell<R>(P.split, cst<R>(P), q, split_sound<R>(P, a, c, q), Ar[0][c], Ar[1][c], Ar[2][c], Hr[0][c],
-                      Hr[1][c], Hr[2][c], Sr[c], fp, fm);
+        for (int n = 0; n < 6; n++) q[n] = arith(Qr[c + n * pl]);
+        A fp[5], fm[5];
+        split_cell<A>(P.split, cst<R>(P), q, split_sound<A>(P, a, c, q), arith(Ar[0][c]), arith(Ar[1][c]),
+                      arith(Ar[2][c]), arith(Hr[0][c]), arith(Hr[1][c]), arith(Hr[2][c]), arith(Sr[c]), fp, fm);
         const int s = sidx(l, p);
 #pragma unroll
         for (int n = 0; n < 5; n++) {
-            sFp[n * TL * NP + s] = fp[n];
-            sFm[n * TL * NP + s] = fm[n];
+            sFp[n * TL * NP + s] = plain(fp[n]);
+            sFm[n * TL * NP + s] = plain(fm[n]);
         }
         if (hybrid) sPhi[s] = Phr[c];
     }
@@ -130,15 +131,15 @@ __global__ void __launch_bounds__(Tile<DIR, R>::NT, Tile<DIR, R>::MINB) k_sweep(
     // (f3d_fixed.cuh) where their coefficients allow it, others at once.
     auto do_face = [&](int l, int t, int br) {
         const long long cl = cell(l, c0 + t + 3), cr = cl + stride;
-        R out[5];
-        R s0 = R(0);
-        if (br == 1 || br == 2) s0 = R(2) / (Sr[cl] + Sr[cr]);
-        auto FP = [&](int n, int p) { return sFp[n * TL * NP + sidx(l, p)]; };
-        auto FM = [&](int n, int p) { return sFm[n * TL * NP + sidx(l, p)]; };
-        face_flux<CHAR, R>(P, a, br, t, s0, cl, cr, FP, FM, out);
+        A out[5];
+        A s0 = A(0);
+        if (br == 1 || br == 2) s0 = A(2) / (arith(Sr[cl]) + arith(Sr[cr]));
+        auto FP = [&](int n, int p) { return arith(sFp[n * TL * NP + sidx(l, p)]); };
+        auto FM = [&](int n, int p) { return arith(sFm[n * TL * NP + sidx(l, p)]); };
+        face_flux<CHAR, A>(P, a, br, t, s0, cl, cr, FP, FM, out);
         const int f = fidx(l, t);
 #pragma unroll
-        for (int n = 0; n < 5; n++) sF[n * TL * NF + f] = out[n];
+        for (int n = 0; n < 5; n++) sF[n * TL * NF + f] = plain(out[n]);
     };
     auto face_lt = [&](int it, int& l, int& t) {
         if (DIR == 0) { l = it / NF; t = it - l * NF; } else { t = it / TL; l = it - t * TL; }

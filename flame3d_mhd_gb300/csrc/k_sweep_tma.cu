@@ -276,23 +276,24 @@ __global__ void __launch_bounds__(TTile<DIR>::NT, TTile<DIR>::MINB)
                     d[n + 1] += k1 * (F[-2 * vs] - F[2 * vs]) + k2 * (F[-vs] - F[vs]);
                 }
             }
-            double L5[5];
+            F64 L5[5];
 #pragma unroll
             for (int n = 0; n < 5; n++)
-                L5[n] = to_f64(sum3_compensated(eacc[n * CELLS + it], eacc2[n * CELLS + it], d[n]));
+                L5[n] = f64(to_f64(sum3_compensated(eacc[n * CELLS + it], eacc2[n * CELLS + it], d[n])));
             if (!stage) {
-                const double Jc = eJ[it];
+                const F64 Jc = f64(eJ[it]);
 #pragma unroll
-                for (int n = 0; n < 5; n++) a.out[c + n * pl] = Jc * L5[n];
+                for (int n = 0; n < 5; n++) a.out[c + n * pl] = F64(Jc * L5[n]).v;
             } else {
-                const double Jact = eJ[it] * a.dt;
+                const F64 Jact = f64(eJ[it]) * F64(a.dt);
+                const F64 ca = a.ca, cb = a.cb;
 #pragma unroll
                 for (int n = 0; n < 5; n++) {
-                    const double u = eU[n * CELLS + it];
-                    if (a.stage1_copy) a.Un[c + n * pl] = u;
-                    double un = u + L5[n] * Jact;
-                    if (a.combine) un = un * a.ca + eUn[n * CELLS + it] * a.cb;
-                    a.U[c + n * pl] = un;
+                    const F64 u = f64(eU[n * CELLS + it]);
+                    if (a.stage1_copy) a.Un[c + n * pl] = u.v;
+                    F64 un = u + L5[n] * Jact;
+                    if (a.combine) un = un * ca + f64(eUn[n * CELLS + it]) * cb;
+                    a.U[c + n * pl] = un.v;
                 }
             }
         }

@@ -10,6 +10,9 @@
 
 namespace f3d {
 
+__device__ __forceinline__ F64 cube_root(F64 x) { return f64(cbrt(x.v)); }
+__device__ __forceinline__ float cube_root(float x) { return cbrtf(x); }
+
 template <class R>
 __global__ void __launch_bounds__(128) k_viscous(const DevParams P, const R* __restrict__ Q, const R* m0,
                                                  const R* m1, const R* m2, const R* m3, const R* m4, const R* m5,
@@ -23,94 +26,105 @@ __global__ void __launch_bounds__(128) k_viscous(const DevParams P, const R* __r
     split3(t, P.dvxt, P.dvyt, vi, vj, vk);
     const long long c = lin3(P, vi + 2, vj + 2, vk + 2);
     const long long pl = P.plane, sy = P.nxt, sz = (long long)P.nxt * P.nyt;
-    const Cst<R>& K = cst<R>(P);
-    const R xx = m0[c], xy = m1[c], xz = m2[c];
-    const R ex = m3[c], ey = m4[c], ez = m5[c];
-    const R zx = m6[c], zy = m7[c], zz = m8[c];
-    const R Jac = J[c];
-    const R T = Q[c + 5 * pl];
-    R mu = K.c_s * T * sqrt(T) / (T + K.t_s);
-    R lam = mu * K.cp_pr;
-    const R c1 = R(1) / R(12), c2 = R(-2) / R(3), c23 = R(2) / R(3);
+    const auto& K = cst<R>(P);
+    using A = typename Arith<R>::type;
+    const A xx = arith(m0[c]), xy = arith(m1[c]), xz = arith(m2[c]);
+    const A ex = arith(m3[c]), ey = arith(m4[c]), ez = arith(m5[c]);
+    const A zx = arith(m6[c]), zy = arith(m7[c]), zz = arith(m8[c]);
+    const A Jac = arith(J[c]);
+    const A T = arith(Q[c + 5 * pl]);
+    A mu;
+    if constexpr (sizeof(R) == 8) {
+        // C_s T^(3/2) / (T + T_s) = C_s T^2 (T (T + T_s)^2)^(-1/2): one reciprocal root instead of a
+        // root and a quotient (five multiplications and 368 cycles of
+        // the FP64 pipe against three and 1120)
+        const A a = T + A(K.t_s), b = (T * a) * a;
+        mu = (A(K.c_s) * T) * (T * rsq(b));
+        if (((__double_as_longlong(T.v)) << 1) == 0) mu = f64(0.0);  // T = 0, where the root has a pole
+    } else {
+        mu = K.c_s * T * sqrt(T) / (T + K.t_s);
+    }
+    A lam = mu * A(K.cp_pr);
+    const A c1 = A(1.0 / 12.0), c2 = A(-2.0 / 3.0), c23 = A(2.0 / 3.0);
     auto d4 = [&](int n, long long s) {
         const R* f = Q + n * pl + c;
-        return c1 * (f[-2 * s] - f[2 * s]) + c2 * (f[-s] - f[s]);
+        return c1 * (arith(f[-2 * s]) - arith(f[2 * s])) + c2 * (arith(f[-s]) - arith(f[s]));
     };
     // viscous.jl:29-42: the CD4 coefficients give +d/dxi
-    const R uxi = d4(1, 1), vxi = d4(2, 1), wxi = d4(3, 1), Txi = d4(5, 1);
-    const R uet = d4(1, sy), vet = d4(2, sy), wet = d4(3, sy), Tet = d4(5, sy);
-    const R uze = d4(1, sz), vze = d4(2, sz), wze = d4(3, sz), Tze = d4(5, sz);
-    const R u = Q[c + pl], v = Q[c + 2 * pl], w = Q[c + 3 * pl];
-    const R dudx = (uxi * xx + uet * ex + uze * zx) * Jac;
-    const R dudy = (uxi * xy + uet * ey + uze * zy) * Jac;
-    const R dudz = (uxi * xz + uet * ez + uze * zz) * Jac;
-    const R dvdx = (vxi * xx + vet * ex + vze * zx) * Jac;
-    const R dvdy = (vxi * xy + vet * ey + vze * zy) * Jac;
-    const R dvdz = (vxi * xz + vet * ez + vze * zz) * Jac;
-    const R dwdx = (wxi * xx + wet * ex + wze * zx) * Jac;
-    const R dwdy = (wxi * xy + wet * ey + wze * zy) * Jac;
-    const R dwdz = (wxi * xz + wet * ez + wze * zz) * Jac;
-    const R dTdx = (Txi * xx + Tet * ex + Tze * zx) * Jac;
-    const R dTdy = (Txi * xy + Tet * ey + Tze * zy) * Jac;
-    const R dTdz = (Txi * xz + Tet * ez + Tze * zz) * Jac;
-    const R dv = dudx + dvdy + dwdz;
+    const A uxi = d4(1, 1), vxi = d4(2, 1), wxi = d4(3, 1), Txi = d4(5, 1);
+    const A uet = d4(1, sy), vet = d4(2, sy), wet = d4(3, sy), Tet = d4(5, sy);
+    const A uze = d4(1, sz), vze = d4(2, sz), wze = d4(3, sz), Tze = d4(5, sz);
+    const A u = arith(Q[c + pl]), v = arith(Q[c + 2 * pl]), w = arith(Q[c + 3 * pl]);
+    const A dudx = (uxi * xx + uet * ex + uze * zx) * Jac;
+    const A dudy = (uxi * xy + uet * ey + uze * zy) * Jac;
+    const A dudz = (uxi * xz + uet * ez + uze * zz) * Jac;
+    const A dvdx = (vxi * xx + vet * ex + vze * zx) * Jac;
+    const A dvdy = (vxi * xy + vet * ey + vze * zy) * Jac;
+    const A dvdz = (vxi * xz + vet * ez + vze * zz) * Jac;
+    const A dwdx = (wxi * xx + wet * ex + wze * zx) * Jac;
+    const A dwdy = (wxi * xy + wet * ey + wze * zy) * Jac;
+    const A dwdz = (wxi * xz + wet * ez + wze * zz) * Jac;
+    const A dTdx = (Txi * xx + Tet * ex + Tze * zx) * Jac;
+    const A dTdy = (Txi * xy + Tet * ey + Tze * zy) * Jac;
+    const A dTdz = (Txi * xz + Tet * ez + Tze * zz) * Jac;
+    const A dv = dudx + dvdy + dwdz;
     if (P.les) {  // viscous.jl:66-106: eddy viscosity and conductivity, Pr_t = 0.9
-        const R rho = Q[c];
-        const R s12 = R(0.5) * (dudy + dvdx), s13 = R(0.5) * (dudz + dwdx), s23 = R(0.5) * (dvdz + dwdy);
-        const R sii = dudx * dudx + dvdy * dvdy + dwdz * dwdz;
-        const R sij = s12 * s12 + s13 * s13 + s23 * s23;
-        const R inv_d = R(1) / cbrt(Jac);  // 1 / Delta with Delta = J^(1/3) (cell size, J^-1 = volume)
-        R mut;
+        const A rho = arith(Q[c]);
+        const A s12 = A(0.5) * (dudy + dvdx), s13 = A(0.5) * (dudz + dwdx), s23 = A(0.5) * (dvdz + dwdy);
+        const A sii = dudx * dudx + dvdy * dvdy + dwdz * dwdz;
+        const A sij = s12 * s12 + s13 * s13 + s23 * s23;
+        const A inv_d = A(1) / cube_root(Jac);  // 1 / Delta with Delta = J^(1/3) (cell size, J^-1 = volume)
+        A mut;
         if (P.les == F3D_LES_SMAGORINSKY) {
-            const R Smag = sqrt(R(2) * (sii + R(2) * sij));  // sqrt(2) |S_ij|
-            const R cd = R(0.1) * inv_d;
+            const A Smag = sqrt(A(2) * (sii + A(2) * sij));  // sqrt(2) |S_ij|
+            const A cd = A(0.1) * inv_d;
             mut = rho * cd * cd * Smag;
         } else {  // WALE
-            const R S = sqrt(sii + R(2) * sij);
-            R d11 = dudx * dudx + dudy * dvdx + dudz * dwdx;
-            R d22 = dvdx * dudy + dvdy * dvdy + dvdz * dwdy;
-            R d33 = dwdx * dudz + dwdy * dvdz + dwdz * dwdz;
-            const R tr = R(1) / R(3) * (d11 + d22 + d33);
+            const A S = sqrt(sii + A(2) * sij);
+            A d11 = dudx * dudx + dudy * dvdx + dudz * dwdx;
+            A d22 = dvdx * dudy + dvdy * dvdy + dvdz * dwdy;
+            A d33 = dwdx * dudz + dwdy * dvdz + dwdz * dwdz;
+            const A tr = A(1.0 / 3.0) * (d11 + d22 + d33);
             d11 -= tr;
             d22 -= tr;
             d33 -= tr;
-            const R d12 = R(0.5) * (dudx * dvdx + dvdx * dvdy + dwdx * dvdz + dudy * dudx + dvdy * dudy + dwdy * dudz);
-            const R d13 = R(0.5) * (dudx * dwdx + dvdx * dwdy + dwdx * dwdz + dudz * dudx + dvdz * dudy + dwdz * dudz);
-            const R d23 = R(0.5) * (dudy * dwdx + dvdy * dwdy + dwdy * dwdz + dudz * dvdx + dvdz * dvdy + dwdz * dvdz);
-            const R Sd = sqrt(d11 * d11 + d22 * d22 + d33 * d33 + R(2) * (d12 * d12 + d13 * d13 + d23 * d23));
-            const R S2 = S * S;
-            const R D = Sd * Sd * Sd / (S2 * S2 * S + Sd * Sd * sqrt(Sd));
-            const R cd = R(0.325) * inv_d;
+            const A d12 = A(0.5) * (dudx * dvdx + dvdx * dvdy + dwdx * dvdz + dudy * dudx + dvdy * dudy + dwdy * dudz);
+            const A d13 = A(0.5) * (dudx * dwdx + dvdx * dwdy + dwdx * dwdz + dudz * dudx + dvdz * dudy + dwdz * dudz);
+            const A d23 = A(0.5) * (dudy * dwdx + dvdy * dwdy + dwdy * dwdz + dudz * dvdx + dvdz * dvdy + dwdz * dvdz);
+            const A Sd = sqrt(d11 * d11 + d22 * d22 + d33 * d33 + A(2) * (d12 * d12 + d13 * d13 + d23 * d23));
+            const A S2 = S * S;
+            const A D = Sd * Sd * Sd / (S2 * S2 * S + Sd * Sd * sqrt(Sd));
+            const A cd = A(0.325) * inv_d;
             mut = rho * cd * cd * D;
         }
         // min(mu_t, 2 mu) returning NaN when either is NaN, as Julia's min does (D = 0/0 where
         // the velocity gradient vanishes)
-        const R lim = R(2) * mu;
+        const A lim = A(2) * mu;
         mut = (mut != mut) ? mut : (lim < mut ? lim : mut);
         mu += mut;
-        lam += K.cp * mut / R(0.9);
+        lam += A(K.cp) * mut / A(0.9);
     }
-    const R t11 = mu * (R(2) * dudx - c23 * dv);
-    const R t12 = mu * (dudy + dvdx);
-    const R t13 = mu * (dudz + dwdx);
-    const R t22 = mu * (R(2) * dvdy - c23 * dv);
-    const R t23 = mu * (dwdy + dvdz);
-    const R t33 = mu * (R(2) * dwdz - c23 * dv);
-    const R E1 = u * t11 + v * t12 + w * t13 + lam * dTdx;
-    const R E2 = u * t12 + v * t22 + w * t23 + lam * dTdy;
-    const R E3 = u * t13 + v * t23 + w * t33 + lam * dTdz;
-    Fvx[t] = xx * t11 + xy * t12 + xz * t13;
-    Fvx[t + vpl] = xx * t12 + xy * t22 + xz * t23;
-    Fvx[t + 2 * vpl] = xx * t13 + xy * t23 + xz * t33;
-    Fvx[t + 3 * vpl] = xx * E1 + xy * E2 + xz * E3;
-    Fvy[t] = ex * t11 + ey * t12 + ez * t13;
-    Fvy[t + vpl] = ex * t12 + ey * t22 + ez * t23;
-    Fvy[t + 2 * vpl] = ex * t13 + ey * t23 + ez * t33;
-    Fvy[t + 3 * vpl] = ex * E1 + ey * E2 + ez * E3;
-    Fvz[t] = zx * t11 + zy * t12 + zz * t13;
-    Fvz[t + vpl] = zx * t12 + zy * t22 + zz * t23;
-    Fvz[t + 2 * vpl] = zx * t13 + zy * t23 + zz * t33;
-    Fvz[t + 3 * vpl] = zx * E1 + zy * E2 + zz * E3;
+    const A t11 = mu * (A(2) * dudx - c23 * dv);
+    const A t12 = mu * (dudy + dvdx);
+    const A t13 = mu * (dudz + dwdx);
+    const A t22 = mu * (A(2) * dvdy - c23 * dv);
+    const A t23 = mu * (dwdy + dvdz);
+    const A t33 = mu * (A(2) * dwdz - c23 * dv);
+    const A E1 = u * t11 + v * t12 + w * t13 + lam * dTdx;
+    const A E2 = u * t12 + v * t22 + w * t23 + lam * dTdy;
+    const A E3 = u * t13 + v * t23 + w * t33 + lam * dTdz;
+    Fvx[t] = plain(A(xx * t11 + xy * t12 + xz * t13));
+    Fvx[t + vpl] = plain(A(xx * t12 + xy * t22 + xz * t23));
+    Fvx[t + 2 * vpl] = plain(A(xx * t13 + xy * t23 + xz * t33));
+    Fvx[t + 3 * vpl] = plain(A(xx * E1 + xy * E2 + xz * E3));
+    Fvy[t] = plain(A(ex * t11 + ey * t12 + ez * t13));
+    Fvy[t + vpl] = plain(A(ex * t12 + ey * t22 + ez * t23));
+    Fvy[t + 2 * vpl] = plain(A(ex * t13 + ey * t23 + ez * t33));
+    Fvy[t + 3 * vpl] = plain(A(ex * E1 + ey * E2 + ez * E3));
+    Fvz[t] = plain(A(zx * t11 + zy * t12 + zz * t13));
+    Fvz[t + vpl] = plain(A(zx * t12 + zy * t22 + zz * t23));
+    Fvz[t + 2 * vpl] = plain(A(zx * t13 + zy * t23 + zz * t33));
+    Fvz[t + 3 * vpl] = plain(A(zx * E1 + zy * E2 + zz * E3));
 }
 
 template <class R>

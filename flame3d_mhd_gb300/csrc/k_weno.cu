@@ -62,10 +62,10 @@ __global__ void __launch_bounds__(256) k_weno_list(const DevParams P, const doub
 
 constexpr int WF_WARPS = 5, WF_FACES = 32;
 struct WenoSmem {
-    double f[10 * 8 * WF_FACES];                 // Fp (5) and Fm (5) of the eight stencil cells
-    CharBasis<double> basis[WF_FACES];
-    double flux[5 * WF_FACES];                   // characteristic fluxes
-    double s0[WF_FACES];
+    double f[10 * 8 * WF_FACES];        // Fp (5) and Fm (5) of the eight stencil cells
+    CharBasis<F64> basis[WF_FACES];
+    F64 flux[5 * WF_FACES];             // characteristic fluxes
+    F64 s0[WF_FACES];
 };
 
 template <bool CHAR>
@@ -107,38 +107,39 @@ __global__ void __launch_bounds__(WF_WARPS * 32, 4) k_weno_faces(const WenoArgs 
             for (int p = wp; p < 8; p += WF_WARPS) {
                 if (br == 2 && (p == 0 || p == 7)) continue;  // WENO5 reads positions 1 .. 6
                 const long long c = cl + (p - 3) * stride;
-                double q[6], fp[5], fm[5];
+                F64 q[6], fp[5], fm[5];
 #pragma unroll
-                for (int n = 0; n < 6; n++) q[n] = Q[c + n * pl];
-                split_cell<double>(P.split, P.cd, q, a.csnd[c], A0[c], A1[c], A2[c], a.H[3 * d][c], a.H[3 * d + 1][c],
-                                   a.H[3 * d + 2][c], S[c], fp, fm);
+                for (int n = 0; n < 6; n++) q[n] = f64(Q[c + n * pl]);
+                split_cell<F64>(P.split, P.cd, q, f64(a.csnd[c]), f64(A0[c]), f64(A1[c]), f64(A2[c]),
+                                f64(a.H[3 * d][c]), f64(a.H[3 * d + 1][c]), f64(a.H[3 * d + 2][c]), f64(S[c]), fp, fm);
 #pragma unroll
                 for (int n = 0; n < 5; n++) {
-                    sm.f[(n * 8 + p) * WF_FACES + lane] = fp[n];
-                    sm.f[((n + 5) * 8 + p) * WF_FACES + lane] = fm[n];
+                    sm.f[(n * 8 + p) * WF_FACES + lane] = fp[n].v;
+                    sm.f[((n + 5) * 8 + p) * WF_FACES + lane] = fm[n].v;
                 }
             }
             if (wp == 3) {
-                const double s0 = 2.0 / (S[cl] + S[cr]);
+                const F64 s0 = F64(2.0) / (f64(S[cl]) + f64(S[cr]));
                 sm.s0[lane] = s0;
-                if (CHAR) char_basis<double>(P, Q, A0, A1, A2, s0, cl, cr, sm.basis[lane]);
+                auto as = [](const double* p) { return reinterpret_cast<const F64*>(p); };
+                if (CHAR) char_basis<F64>(P, as(Q), as(A0), as(A1), as(A2), s0, cl, cr, sm.basis[lane]);
             }
         }
         __syncthreads();
-        auto FP = [&](int n, int p) { return sm.f[(n * 8 + p) * WF_FACES + lane]; };
-        auto FM = [&](int n, int p) { return sm.f[((n + 5) * 8 + p) * WF_FACES + lane]; };
+        auto FP = [&](int n, int p) { return f64(sm.f[(n * 8 + p) * WF_FACES + lane]); };
+        auto FM = [&](int n, int p) { return f64(sm.f[((n + 5) * 8 + p) * WF_FACES + lane]); };
         if (on) {
-            const double s0 = sm.s0[lane];
-            if (CHAR) sm.flux[wp * WF_FACES + lane] = char_field_flux<double>(P, sm.basis[lane], wp, br, 0, s0, FP, FM);
-            else *out = comp_field_flux<double>(P, wp, br, 0, s0, FP, FM);
+            const F64 s0 = sm.s0[lane];
+            if (CHAR) sm.flux[wp * WF_FACES + lane] = char_field_flux<F64>(P, sm.basis[lane], wp, br, 0, s0, FP, FM);
+            else *out = comp_field_flux<F64>(P, wp, br, 0, s0, FP, FM).v;
         }
         __syncthreads();
         if (CHAR) {
             if (on) {
-                double flux[5];
+                F64 flux[5];
 #pragma unroll
                 for (int n = 0; n < 5; n++) flux[n] = sm.flux[n * WF_FACES + lane];
-                *out = char_right_row<double>(sm.basis[lane], wp, flux);
+                *out = char_right_row<F64>(sm.basis[lane], wp, flux).v;
             }
             __syncthreads();
         }
