@@ -124,13 +124,13 @@ __device__ __forceinline__ double max_floor(double x, double e) {
 // utils.jl:2-30 c2Prim of one cell. q = (rho,u,v,w,p,T).
 __device__ __forceinline__ void c2prim_cell(const DevParams& P, const double U[5], double q[6]) {
     const double rho = max_floor(U[0], P.eps_clamp);
-    double rinv = 1.0 / rho;
+    const double rinv = recip_ieee(f64(rho)).v;
     double u = mul64(U[1], rinv), v = mul64(U[2], rinv), w = mul64(U[3], rinv);
     double ke = add64(add64(mul64(u, u), mul64(v, v)), mul64(w, w));
     double eraw = add64(U[4], -mul64(mul64(constant_here(0.5), rho), ke));
     const double ei = max_floor(eraw, P.eps_clamp);
     double p = mul64(constant_here(P.gm1), ei);
-    double T = p / mul64(rho, constant_here(P.rg));
+    double T = (f64(p) / f64(mul64(rho, constant_here(P.rg)))).v;
     q[0] = rho; q[1] = u; q[2] = v; q[3] = w; q[4] = p; q[5] = T;
 }
 

@@ -96,8 +96,15 @@ __device__ __forceinline__ F64 recip(F64 b) {
     if (!recip_range(b.v)) return f64(1.0 / b.v);
     return recip_step(b.v);
 }
-// a/b: a times the reciprocal and one residual correction, six FMAs, within 0.51 ulp where the
-// quotient and the residual are normal; the IEEE quotient elsewhere
+// 1/b with one residual correction (five FMAs): before its last rounding within 2^-105 of the
+// reciprocal, so it is the IEEE reciprocal unless that lies as near to a rounding boundary
+__device__ __forceinline__ F64 recip_ieee(F64 b) {
+    if (!recip_range(b.v)) return f64(1.0 / b.v);
+    const F64 r = recip_step(b.v);
+    return r + (f64(in_register(1.0)) - b * r) * r;
+}
+// a/b: a times the reciprocal and one residual correction (six FMAs; as near to the IEEE quotient
+// as recip_ieee) where the quotient and the residual are normal; the IEEE division elsewhere
 __device__ __forceinline__ F64 operator/(F64 a, F64 b) {
     const unsigned ha = (unsigned)__double2hiint(a.v) & 0x7fffffffu, ea = ha >> 20;
     const unsigned eb = ((unsigned)__double2hiint(b.v) >> 20) & 0x7ffu;
@@ -114,6 +121,31 @@ using ::sqrt;
 __device__ __forceinline__ F64 fabs(F64 a) { return f64(::fabs(a.v)); }
 __device__ __forceinline__ F64 sqrt(F64 a) { return f64(::sqrt(a.v)); }
 __device__ __forceinline__ F64 rsq(F64 a) { return f64(::rsqrt(a.v)); }
+
+// The square root of a normal x: an FP32 reciprocal root of x scaled by an even power of two, one
+// step of Goldschmidt's coupled iteration for g = x^(1/2), h = x^(-1/2) / 2 (relative error 2^-22 to
+// 2^-43) and the residual correction g + h (x - g^2): seven FMAs (448 cycles against 572), before
+// its last rounding within 2^-85 of the root. The library's root elsewhere.
+__device__ __forceinline__ F64 root(F64 x) {
+    const unsigned hi = (unsigned)__double2hiint(x.v), e = hi >> 20;  // sign and exponent
+    if (e - 64u > 1900u) return sqrt(x);
+    const unsigned lo = (unsigned)__double2loint(x.v);
+    // mantissa times 1 (odd biased exponent) or 2, as binary32 in [1, 4)
+    const unsigned odd = (e & 1u) ^ 1u;
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;"
+        : "=f"(y) : "f"(__uint_as_float(((127u + odd) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29))));
+    const unsigned f = __float_as_uint(y);  // in (1/2, 1]
+    // times 2^-((e - odd - 1023) / 2)
+    const unsigned yh = (f >> 3) + (896u << 20) - ((((e - odd) - 1023u) << 19) & 0xfff00000u);
+    const F64 y0 = f64(__hiloint2double((int)yh, (int)(f << 29)));
+    const F64 half = f64(in_register(0.5));
+    F64 g = x * y0, h = y0 * half;
+    const F64 r = half - g * h;
+    g = g + g * r;
+    h = h + h * r;
+    return g + (x - g * g) * h;
+}
 
 // The arithmetic type of a kernel's element type, and values between the two
 template <class R> struct Arith { using type = R; };

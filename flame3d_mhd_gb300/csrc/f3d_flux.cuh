@@ -253,11 +253,17 @@ __device__ __forceinline__ double weno7_ref32(float V1, float V2, float V3, floa
                                               float s0) {
     float q[4], Is[4];
     weno7_parts<float>(V1, V2, V3, V4, V5, V6, V7, q, Is);
+    // alpha_k over their common denominator (one FP64 division a side instead of five): the
+    // reference's values to within FP64 rounding, far below the Float32 the result is rounded to.
+    // Bases from 1e-20 to 3e38: the triple products stay within 1e-120 .. 1e231. Plain double
+    // expressions: branches here change how the compiler contracts the mixed form's FP32 faces in
+    // the same kernels
     const double e1 = 1e-20;
-    const double a1 = 1.0 / sq(e1 + (double)(Is[0] * s0)), a2 = 12.0 / sq(e1 + (double)(Is[1] * s0));
-    const double a3 = 18.0 / sq(e1 + (double)(Is[2] * s0)), a4 = 4.0 / sq(e1 + (double)(Is[3] * s0));
-    const double invsum = 1.0 / (a1 + a2 + a3 + a4);
-    return invsum * (a1 * (double)q[0] + a2 * (double)q[1] + a3 * (double)q[2] + a4 * (double)q[3]);
+    const double b1 = sq(e1 + (double)(Is[0] * s0)), b2 = sq(e1 + (double)(Is[1] * s0));
+    const double b3 = sq(e1 + (double)(Is[2] * s0)), b4 = sq(e1 + (double)(Is[3] * s0));
+    const double p12 = b1 * b2, p34 = b3 * b4;
+    const double a1 = b2 * p34, a2 = 12.0 * b1 * p34, a3 = 18.0 * p12 * b4, a4 = 4.0 * p12 * b3;
+    return (a1 * (double)q[0] + a2 * (double)q[1] + a3 * (double)q[2] + a4 * (double)q[3]) / (a1 + a2 + a3 + a4);
 }
 // WENO5 in Float32 with one division per alpha and one for their sum (schemes.jl:233-252).
 __device__ __forceinline__ float weno5_ref32(float V1, float V2, float V3, float V4, float V5, float s0) {

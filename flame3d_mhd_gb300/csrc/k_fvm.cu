@@ -92,8 +92,27 @@ cudaError_t launch_face_geometry(const DevParams& P, const double* x, const doub
 // min / max that return NaN when either argument is NaN, as Julia's min and max do (the
 // reference's wave-speed estimates): fmin/fmax would drop a NaN Roe speed and hide a
 // negative reconstructed density from the non-finite check.
-__device__ __forceinline__ F64 nan_min(F64 a, F64 b) { return a != a ? a : (b != b ? b : (b < a ? b : a)); }
-__device__ __forceinline__ F64 nan_max(F64 a, F64 b) { return a != a ? a : (b != b ? b : (a < b ? b : a)); }
+// Comparisons on the bit patterns with integer instructions (an FP64 comparison takes the FP64 pipe
+// as long as an addition): two's complement order for the signs, the NaN patterns lie beyond both
+// infinities.
+__device__ __forceinline__ long long order_of(F64 a) {
+    const long long b = __double_as_longlong(a.v);
+    return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ bool is_nan(F64 a) {
+    return (__double_as_longlong(a.v) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll;
+}
+__device__ __forceinline__ F64 nan_min(F64 a, F64 b) {
+    return is_nan(a) ? a : (is_nan(b) ? b : (order_of(b) < order_of(a) ? b : a));
+}
+__device__ __forceinline__ F64 nan_max(F64 a, F64 b) {
+    return is_nan(a) ? a : (is_nan(b) ? b : (order_of(a) < order_of(b) ? b : a));
+}
+// a >= 0 and a <= 0, either zero included, false for NaN
+__device__ __forceinline__ bool not_below_zero(F64 a) {
+    return !is_nan(a) && (__double2hiint(a.v) >= 0 || (__double_as_longlong(a.v) << 1) == 0);
+}
+__device__ __forceinline__ bool not_above_zero(F64 a) { return not_below_zero(-a); }
 
 // HLLC flux along the unit normal n of the conserved states UL, UR (FVM.jl:1224-1357)
 __device__ __forceinline__ void hllc(const DevParams& P, const F64 UL[5], const F64 UR[5], F64 nx, F64 ny, F64 nz,
@@ -102,12 +121,12 @@ __device__ __forceinline__ void hllc(const DevParams& P, const F64 UL[5], const 
     const F64 rL = UL[0], irL = recip(rL);
     const F64 uL = UL[1] * irL, vL = UL[2] * irL, wL = UL[3] * irL, EL = UL[4];
     const F64 pL = gm * (EL - (half * rL) * (uL * uL + vL * vL + wL * wL));
-    const F64 cL = sqrt(fabs((g * pL) * irL));
+    const F64 cL = root(fabs((g * pL) * irL));
     const F64 qL = uL * nx + vL * ny + wL * nz;
     const F64 rR = UR[0], irR = recip(rR);
     const F64 uR = UR[1] * irR, vR = UR[2] * irR, wR = UR[3] * irR, ER = UR[4];
     const F64 pR = gm * (ER - (half * rR) * (uR * uR + vR * vR + wR * wR));
-    const F64 cR = sqrt(fabs((g * pR) * irR));
+    const F64 cR = root(fabs((g * pR) * irR));
     const F64 qR = uR * nx + vR * ny + wR * nz;
     // Roe averages (sqrt(rL) a + sqrt(rR) b) / (sqrt(rL) + sqrt(rR)) = b + k (a - b) with
     // k = 1 / (1 + sqrt(rR / rL)): one root and one reciprocal; two negative densities, whose roots
@@ -115,18 +134,18 @@ __device__ __forceinline__ void hllc(const DevParams& P, const F64 UL[5], const 
     F64 ratio = rR * irL;
     if ((__double2hiint(rL.v) | __double2hiint(rR.v)) < 0 && rL.v != 0.0 && rR.v != 0.0)
         ratio = f64(__longlong_as_double(0x7ff8000000000000ll));
-    const F64 k = recip(F64(1.0) + sqrt(ratio));
+    const F64 k = recip(F64(1.0) + root(ratio));
     const F64 ur = uR + k * (uL - uR), vr = vR + k * (vL - vR), wr = wR + k * (wL - wR);
     const F64 qr = ur * nx + vr * ny + wr * nz;
     const F64 HL = (EL + pL) * irL, HR = (ER + pR) * irR;
     const F64 Hr = HR + k * (HL - HR);
-    const F64 cr = sqrt(fabs(gm * (Hr - half * (ur * ur + vr * vr + wr * wr))));
+    const F64 cr = root(fabs(gm * (Hr - half * (ur * ur + vr * vr + wr * wr))));
     const F64 SL = nan_min(qL - cL, qr - cr);
     const F64 SR = nan_max(qR + cR, qr + cr);
     const F64 mL = rL * (SL - qL), mR = rR * (SR - qR);
     const F64 Ss = (pR - pL + mL * qL - mR * qR) / (mL - mR + F64(1e-12));
-    const F64 zero = 0.0;
-    const bool left = SL >= zero || (SR > zero && Ss >= zero);
+    const bool SLp = not_below_zero(SL), SRm = not_above_zero(SR);
+    const bool left = SLp || (!SRm && !is_nan(SR) && not_below_zero(Ss));
     const F64 r = left ? rL : rR, u = left ? uL : uR, v = left ? vL : vR, w = left ? wL : wR;
     const F64 E = left ? EL : ER, p = left ? pL : pR, q = left ? qL : qR;
     const F64 rq = r * q;
@@ -135,7 +154,7 @@ __device__ __forceinline__ void hllc(const DevParams& P, const F64 UL[5], const 
     F[2] = rq * v + p * ny;
     F[3] = rq * w + p * nz;
     F[4] = (E + p) * q;
-    if (SL >= zero || SR <= zero) return;  // supersonic: the upwind state's physical flux
+    if (SLp || SRm) return;  // supersonic: the upwind state's physical flux
     // star state of the side: F* = F + S (U* - U)
     const F64 S = left ? SL : SR, ir = left ? irL : irR, m = left ? mL : mR;  // m = r (S - q)
     const F64* Us = left ? UL : UR;
@@ -182,7 +201,7 @@ template <> struct FTile<2> { static constexpr int TL = 16, TC = 16; };
 // registers a thread, the component-wise one ~120. Small blocks let several blocks share an
 // SM, so one block's barrier waits overlap another's face work.
 #ifndef FVM_E_THREADS
-#define FVM_E_THREADS 64
+#define FVM_E_THREADS 96
 #define FVM_E_BLOCKS 4
 #define FVM_C_THREADS 128
 #define FVM_C_BLOCKS 2
@@ -279,7 +298,7 @@ __global__ void __launch_bounds__(FvmLaunch<EIGEN>::NT, FvmLaunch<EIGEN>::MINB) 
             } else {  // Eigen_reconstruct, FVM.jl:65-228
                 auto Qv = [&](int n, long long c) { return f64(Q[c + n * pl]); };
                 const long long cr = cl + stride;
-                const F64 srl = sqrt(Qv(0, cl)), srr = sqrt(Qv(0, cr)), isr = recip(srl + srr);
+                const F64 srl = root(Qv(0, cl)), srr = root(Qv(0, cr)), isr = recip(srl + srr);
                 const F64 half = 0.5;
                 auto roe = [&](F64 a, F64 b) { return F64((srl * a + srr * b) * isr); };
                 const F64 u = roe(Qv(1, cl), Qv(1, cr)), v = roe(Qv(2, cl), Qv(2, cr)), w = roe(Qv(3, cl), Qv(3, cr));
@@ -290,7 +309,7 @@ __global__ void __launch_bounds__(FvmLaunch<EIGEN>::NT, FvmLaunch<EIGEN>::MINB) 
                 };
                 const F64 H = roe(Hof(cl), Hof(cr));
                 const F64 v2 = half * (u * u + v * v + w * w);
-                const F64 c = sqrt(P.gm1 * (H - v2));
+                const F64 c = root(P.gm1 * (H - v2));
                 F64 lx, ly, lz;
                 if (fabs(nz) <= fabs(ny)) {
                     const F64 id = rsq(nx * nx + ny * ny + F64(1e-12));

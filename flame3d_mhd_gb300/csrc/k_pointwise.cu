@@ -22,7 +22,7 @@ __device__ __forceinline__ bool is_interior(const DevParams& P, int i, int j, in
 
 __device__ __forceinline__ double sound_speed(const DevParams& P, const double q[6]) {
     // split.jl:22 (SW) and split.jl:90,130,205 (LF, VL, AUSM)
-    return P.split == F3D_SPLIT_SW ? ::sqrt(mul64(constant_here(P.grg), q[5])) : ::sqrt(mul64(constant_here(P.gamma), q[4]) / q[0]);
+    return root(P.split == F3D_SPLIT_SW ? F64(F64(P.grg) * f64(q[5])) : F64(F64(P.gamma) * f64(q[4])) / f64(q[0])).v;
 }
 
 // c2Prim at interior cells (k_prim_interior), then the composed ghost rules (k_prim_ghost):
