@@ -13,28 +13,27 @@ namespace f3d {
 // ---- c2Prim (utils.jl:2-30): q = (rho,u,v,w,p,T) from U; qb -> Ub ----------------------
 __device__ __forceinline__ void c2prim_vjp(const DevParams& P, const double U[5], const double qb[6], double Ub[5]) {
     const bool rho_free = U[0] > P.eps_clamp;
-    const double rho = rho_free ? U[0] : P.eps_clamp;
-    const double rinv = 1.0 / rho;
-    const double u = U[1] * rinv, v = U[2] * rinv, w = U[3] * rinv;
-    const double ke = u * u + v * v + w * w;
-    const double eraw = U[4] - 0.5 * rho * ke;
-    const bool e_free = eraw > P.eps_clamp;
-    const double ei = e_free ? eraw : P.eps_clamp;
-    const double p = P.gm1 * ei;
-    const double Tr = qb[5] * rinv * P.inv_rg;  // T = p/(rho Rg)
-    double pb = qb[4] + Tr;
-    double rhob = qb[0] - Tr * p * rinv;
-    const double eb = e_free ? P.gm1 * pb : 0.0;
-    Ub[4] = eb;
-    rhob += -0.5 * ke * eb;
-    const double keb = -0.5 * rho * eb;
-    const double ub = qb[1] + 2.0 * u * keb, vb = qb[2] + 2.0 * v * keb, wb = qb[3] + 2.0 * w * keb;
-    Ub[1] = ub * rinv;
-    Ub[2] = vb * rinv;
-    Ub[3] = wb * rinv;
-    const double rinvb = ub * U[1] + vb * U[2] + wb * U[3];
-    rhob += -rinvb * rinv * rinv;
-    Ub[0] = rho_free ? rhob : 0.0;
+    const F64 rho = f64(rho_free ? U[0] : P.eps_clamp);
+    const F64 rinv = recip(rho);
+    const F64 m1 = f64(U[1]), m2 = f64(U[2]), m3 = f64(U[3]), half = 0.5, gm1 = P.gm1;
+    const F64 u = m1 * rinv, v = m2 * rinv, w = m3 * rinv;
+    const F64 ke = u * u + v * v + w * w;
+    const F64 hr = half * rho;
+    const F64 eraw = f64(U[4]) - hr * ke;
+    const bool e_free = eraw.v > P.eps_clamp;
+    const F64 p = gm1 * (e_free ? eraw : f64(P.eps_clamp));
+    const F64 Tr = (f64(qb[5]) * rinv) * F64(P.inv_rg);  // T = p/(rho Rg)
+    const F64 pb = f64(qb[4]) + Tr;
+    const F64 eb = e_free ? F64(gm1 * pb) : f64(0.0);
+    const F64 k2 = (hr + hr) * eb;  // -2 times the cotangent of ke
+    const F64 ub = f64(qb[1]) - u * k2, vb = f64(qb[2]) - v * k2, wb = f64(qb[3]) - w * k2;
+    Ub[4] = eb.v;
+    Ub[1] = F64(ub * rinv).v;
+    Ub[2] = F64(vb * rinv).v;
+    Ub[3] = F64(wb * rinv).v;
+    const F64 rinvb = ub * m1 + vb * m2 + wb * m3;
+    const F64 rhob = f64(qb[0]) - (half * ke) * eb - (Tr * p + rinvb * rinv) * rinv;
+    Ub[0] = rho_free ? rhob.v : 0.0;
 }
 
 // ---- flux splitting (split.jl) -------------------------------------------------------
@@ -46,89 +45,93 @@ __device__ __forceinline__ void c2prim_vjp(const DevParams& P, const double U[5]
 // and routed by their sign pattern, the eigenvectors' velocities u -+ c Ah and enthalpies
 // H -+ c Un. The metric enters only through Ah and |A| (A's own cotangent stays 0; the caller
 // folds Ah and |A| back onto A).
-__device__ __forceinline__ void split_sw_vjp(const Cst<double>& K, const double q[6], double c, double A1, double A2,
-                                             double A3, double H1, double H2, double H3, double ss,
-                                             const double fpb[5], const double fmb[5], double qb[6],
-                                             double* mg = nullptr) {
-    (void)A1; (void)A2; (void)A3;
-    const double rho = q[0], u = q[1], v = q[2], w = q[3];
-    const double tss = (rho * ss) * K.inv_2g;
-    const double Un = H1 * u + H2 * v + H3 * w;
-    const double e1 = tss * Un, tcs = tss * c;
-    const double e2 = e1 - tcs, e3 = e1 + tcs;
-    const double q2 = u * u + v * v + w * w;
-    const double vv = K.gm1 * q2;
-    const double Hh = 0.5 * q2 + (K.inv_gm1 * c) * c;
-    const double cUn = c * Un;
-    const bool e2pos = __double2hiint(e2) >= 0, e3pos = __double2hiint(e3) >= 0;
-    double ub = 0, vb = 0, wb = 0, cb = 0, Hb1 = 0, Hb2 = 0, Hb3 = 0, vvb = 0, Hhb = 0, cUnb = 0;
-    double e1b, e2b, e3b;
+__device__ __forceinline__ void split_sw_vjp(const Cst<double>& K, const F64 q[6], F64 c, F64 H1, F64 H2, F64 H3, F64 ss,
+                                             const F64 fpb[5], const F64 fmb[5], F64 qb[6], F64* mg = nullptr) {
+    const F64 rho = q[0], u = q[1], v = q[2], w = q[3], i2g = K.inv_2g, gm1 = K.gm1, two_gm1 = K.two_gm1;
+    const F64 tss = (rho * ss) * i2g;
+    const F64 Un = H1 * u + H2 * v + H3 * w;
+    const F64 e1 = tss * Un, tcs = tss * c;
+    const F64 e2 = e1 - tcs, e3 = e1 + tcs;
+    const F64 q2 = u * u + v * v + w * w;
+    const F64 vv = gm1 * q2, cg = F64(K.inv_gm1) * c;
+    const F64 Hh = F64(0.5) * q2 + cg * c;
+    const F64 cUn = c * Un;
+    const bool e2pos = sign_plus(e2), e3pos = sign_plus(e3);
+    F64 ub, vb, wb, cb, Hb1, Hb2, Hb3, vvb, Hhb, cUnb;
+    F64 e1b, e2b, e3b;
     if (e2pos || !e3pos) {  // f = a1 + e2 + e3, (a1 + e2 + e3) u + c (e3 - e2) Ah, e1 vv + (e2 + e3) H + (e3 - e2) c Un
-        const double* g = e2pos ? fpb : fmb;
-        const double a1 = K.two_gm1 * e1, s23 = e2 + e3, d23 = e3 - e2;
-        const double f0 = a1 + s23, dc = d23 * c;
-        const double f0b = g[0] + g[1] * u + g[2] * v + g[3] * w;
-        const double dcb = g[1] * H1 + g[2] * H2 + g[3] * H3;
-        ub += g[1] * f0; vb += g[2] * f0; wb += g[3] * f0;
-        Hb1 += g[1] * dc; Hb2 += g[2] * dc; Hb3 += g[3] * dc;
-        vvb += g[4] * e1;
-        Hhb += g[4] * s23;
-        cUnb += g[4] * d23;
-        cb += dcb * d23;
-        const double s23b = g[4] * Hh + f0b, d23b = g[4] * cUn + dcb * c;
-        e1b = g[4] * vv + K.two_gm1 * f0b;
+        F64 g[5];
+#pragma unroll
+        for (int n = 0; n < 5; n++) g[n] = e2pos ? fpb[n] : fmb[n];
+        const F64 s23 = e2 + e3, d23 = e3 - e2;
+        const F64 f0 = two_gm1 * e1 + s23, dc = d23 * c;
+        const F64 f0b = g[0] + g[1] * u + g[2] * v + g[3] * w;
+        const F64 dcb = g[1] * H1 + g[2] * H2 + g[3] * H3;
+        ub = g[1] * f0; vb = g[2] * f0; wb = g[3] * f0;
+        Hb1 = g[1] * dc; Hb2 = g[2] * dc; Hb3 = g[3] * dc;
+        vvb = g[4] * e1;
+        Hhb = g[4] * s23;
+        cUnb = g[4] * d23;
+        cb = dcb * d23;
+        const F64 s23b = g[4] * Hh + f0b, d23b = g[4] * cUn + dcb * c;
+        e1b = g[4] * vv + two_gm1 * f0b;
         e2b = s23b - d23b;
         e3b = s23b + d23b;
     } else {  // e2 < 0 <= e3: Fp from e3 (and e1 >= 0), Fm from e2 (and e1 < 0)
-        const bool e1pos = __double2hiint(e1) >= 0;
-        const double e1p = e1pos ? e1 : 0.0, e1m = e1pos ? 0.0 : e1;
-        const double fp0 = K.two_gm1 * e1p + e3, e3c = e3 * c;
-        const double fm0 = K.two_gm1 * e1m + e2, e2c = e2 * c;
-        const double* g = fpb;
-        const double* h = fmb;
-        const double fp0b = g[0] + g[1] * u + g[2] * v + g[3] * w;
-        const double fm0b = h[0] + h[1] * u + h[2] * v + h[3] * w;
-        const double e3cb = g[1] * H1 + g[2] * H2 + g[3] * H3;
-        const double e2cb = -(h[1] * H1 + h[2] * H2 + h[3] * H3);
-        ub += g[1] * fp0 + h[1] * fm0;
-        vb += g[2] * fp0 + h[2] * fm0;
-        wb += g[3] * fp0 + h[3] * fm0;
-        Hb1 += g[1] * e3c - h[1] * e2c;
-        Hb2 += g[2] * e3c - h[2] * e2c;
-        Hb3 += g[3] * e3c - h[3] * e2c;
-        vvb += g[4] * e1p + h[4] * e1m;
-        Hhb += g[4] * e3 + h[4] * e2;
-        cUnb += g[4] * e3 - h[4] * e2;
-        cb += e3cb * e3 + e2cb * e2;
-        e3b = fp0b + e3cb * c + g[4] * (Hh + cUn);
-        e2b = fm0b + e2cb * c + h[4] * (Hh - cUn);
+        const bool e1pos = sign_plus(e1);
+        F64 e1p, e1m;
+        sign_split(e1, e1p, e1m);
+        const F64 fp0 = two_gm1 * e1p + e3, e3c = e3 * c;
+        const F64 fm0 = two_gm1 * e1m + e2, e2c = e2 * c;
+        const F64* g = fpb;
+        const F64* h = fmb;
+        const F64 fp0b = g[0] + g[1] * u + g[2] * v + g[3] * w;
+        const F64 fm0b = h[0] + h[1] * u + h[2] * v + h[3] * w;
+        const F64 e3cb = g[1] * H1 + g[2] * H2 + g[3] * H3;
+        const F64 e2cb = -(h[1] * H1 + h[2] * H2 + h[3] * H3);
+        ub = g[1] * fp0 + h[1] * fm0;
+        vb = g[2] * fp0 + h[2] * fm0;
+        wb = g[3] * fp0 + h[3] * fm0;
+        Hb1 = g[1] * e3c - h[1] * e2c;
+        Hb2 = g[2] * e3c - h[2] * e2c;
+        Hb3 = g[3] * e3c - h[3] * e2c;
+        vvb = g[4] * e1p + h[4] * e1m;
+        const F64 g3 = g[4] * e3;
+        Hhb = h[4] * e2 + g3;
+        cUnb = g3 - h[4] * e2;
+        cb = e3cb * e3 + e2cb * e2;
+        e3b = (fp0b + e3cb * c) + g[4] * (Hh + cUn);
+        e2b = (fm0b + e2cb * c) + h[4] * (Hh - cUn);
         // e1+ = max(e1, 0), e1- = min(e1, 0): the cotangent of the side e1 lies on
-        e1b = e1pos ? g[4] * vv + K.two_gm1 * fp0b : h[4] * vv + K.two_gm1 * fm0b;
+        const F64 ge = e1pos ? g[4] : h[4], fe = e1pos ? fp0b : fm0b;
+        e1b = ge * vv + two_gm1 * fe;
     }
     // e2 = e1 - tcs, e3 = e1 + tcs; e1 = tss Un, tcs = tss c; cUn = c Un
     e1b += e2b + e3b;
-    const double tcsb = e3b - e2b;
-    const double tssb = e1b * Un + tcsb * c;
-    const double Unb = e1b * tss + cUnb * c;
-    cb += tcsb * tss + cUnb * Un;
+    const F64 tcsb = e3b - e2b;
+    const F64 tssb = e1b * Un + tcsb * c;
+    const F64 Unb = e1b * tss + cUnb * c;
+    cb = cb + tcsb * tss + cUnb * Un;
     // Hh = q2/2 + c^2/(gamma-1), vv = (gamma-1) q2, q2 = |u|^2, Un = Ah.u
-    const double q2b = 0.5 * Hhb + K.gm1 * vvb;
-    cb += 2.0 * (K.inv_gm1 * c) * Hhb;
-    ub += 2.0 * u * q2b + H1 * Unb;
-    vb += 2.0 * v * q2b + H2 * Unb;
-    wb += 2.0 * w * q2b + H3 * Unb;
+    const F64 q2b = Hhb + F64(2.0 * K.gm1) * vvb;  // twice the cotangent of q2
+    cb += (cg + cg) * Hhb;
+    ub = ub + u * q2b + H1 * Unb;
+    vb = vb + v * q2b + H2 * Unb;
+    wb = wb + w * q2b + H3 * Unb;
+    const F64 ts = tssb * i2g;
     if (mg) {
         mg[3] += Hb1 + u * Unb;
         mg[4] += Hb2 + v * Unb;
         mg[5] += Hb3 + w * Unb;
-        mg[6] += tssb * rho * K.inv_2g;
+        mg[6] += ts * rho;
     }
-    qb[0] += tssb * ss * K.inv_2g;
-    qb[1] += ub;
-    qb[2] += vb;
-    qb[3] += wb;
+    qb[0] = ts * ss;
+    qb[1] = ub;
+    qb[2] = vb;
+    qb[3] = wb;
+    qb[4] = f64(0.0);
     // c = sqrt(gamma Rg T)
-    qb[5] += cb * K.grg / (2.0 * c);
+    qb[5] = (cb * F64(0.5 * K.grg)) * recip(c);
 }
 
 __device__ __forceinline__ void split_lf_vjp(const Cst<double>& K, const double q[6], double c, double A1, double A2,

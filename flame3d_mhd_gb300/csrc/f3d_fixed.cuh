@@ -67,6 +67,63 @@ __device__ __forceinline__ double fixed_to_f64(long long T, unsigned r, int E) {
     return __longlong_as_double((long long)(b | (neg ? 0x8000000000000000ull : 0ull)));
 }
 
+// The two one-sided linear combinations of one array on a strip: up[f] = sum_k lin[k] V(t0 + f + k) and
+// down[f] = sum_k lin[k] V(t0 + f + 7 - k), f = 0..4 (the left and right states of finite-volume faces;
+// the transpose of the linear faces in the reverse sweeps). V(p) is read at p = t0 .. t0 + 11;
+// the windows share positions t0 + 4 .. t0 + 7.
+template <class VF>
+__device__ __forceinline__ void linear_strip_both(const DevParams& P, int t0, VF V, double up[LIN_STRIP],
+                                                  double down[LIN_STRIP]) {
+    constexpr int NV = LIN_STRIP + 7;
+    unsigned top = 0u, mid = 0u;
+#pragma unroll
+    for (int p = 0; p < NV; p++) {
+        const unsigned a = (unsigned)__double2hiint(V(t0 + p)) & 0x7fffffffu;
+        top = max(top, a);
+        if (p >= LIN_STRIP - 1 && p <= 7) mid = max(mid, a);
+    }
+    if (top == 0u) {  // all zero (or below 2^-1042)
+#pragma unroll
+        for (int f = 0; f < LIN_STRIP; f++) up[f] = down[f] = 0.0;
+        return;
+    }
+    const int E = (int)(top >> 20), Em = (int)(mid >> 20);
+    if (E < 200 || E > 1900 || E - Em > LIN_SPREAD) {
+#pragma unroll
+        for (int f = 0; f < LIN_STRIP; f++) {
+            double a = 0.0, b = 0.0;
+#pragma unroll
+            for (int k = 0; k < 7; k++) {
+                a += P.cd.lin[k] * V(t0 + f + k);
+                b += P.cd.lin[k] * V(t0 + f + 7 - k);
+            }
+            up[f] = a;
+            down[f] = b;
+        }
+        return;
+    }
+    long long x[NV];
+#pragma unroll
+    for (int p = 0; p < NV; p++) x[p] = fixed_of(V(t0 + p), E);
+#pragma unroll
+    for (int f = 0; f < LIN_STRIP; f++)
+#pragma unroll
+        for (int side = 0; side < 2; side++) {
+            long long h = 0;
+            unsigned long long lp = 0ull, ln = 0ull;
+#pragma unroll
+            for (int k = 0; k < 7; k++) {
+                const long long v = x[side == 0 ? f + k : f + 7 - k];
+                h += (long long)(int)(v >> 32) * P.lin_c[k];
+                if (k == 0 || k == 2 || k == 5) ln += (unsigned long long)(unsigned)v * (unsigned)(-P.lin_c[k]);
+                else lp += (unsigned long long)(unsigned)v * (unsigned)P.lin_c[k];
+            }
+            const long long l = (long long)(lp - ln);
+            const double r = F64(f64(fixed_to_f64(h + (l >> 32), (unsigned)l, E)) * F64(P.lin_s)).v;
+            if (side == 0) up[f] = r; else down[f] = r;
+        }
+}
+
 // The five faces t0 .. t0+4 of one line and component: out[f] = sum_k lin[k] (Fp(t+k) + Fm(t+7-k)),
 // t = t0 + f. FP / FM(p) read the split fluxes at position p; positions past `last` were not
 // filled and count as zero (no face that is kept reads them).
@@ -127,7 +184,7 @@ __device__ __forceinline__ void linear_strip(const DevParams& P, int t0, int las
 #pragma unroll
     for (int f = 0; f < LIN_STRIP; f++) {
         const long long l = (long long)(lp[f] - ln[f]);
-        out[f] = fixed_to_f64(hs[f] + (l >> 32), (unsigned)l, E) * P.lin_s;
+        out[f] = F64(f64(fixed_to_f64(hs[f] + (l >> 32), (unsigned)l, E)) * F64(P.lin_s)).v;
     }
 }
 

@@ -15,7 +15,7 @@
 // Contributions that cross tile boundaries are added with FP64 atomics, so gradients are
 // accurate but their last bits depend on the order of those additions.
 #include "f3d_adjoint.cuh"
-#include "f3d_kernels.cuh"
+#include "f3d_fixed.cuh"
 
 namespace f3d {
 
@@ -110,13 +110,13 @@ __global__ void __launch_bounds__(VTile<DIR, CHAR>::NT, VTile<DIR, CHAR>::MINB) 
         }
         if (l >= nl || p >= nc + 8) continue;
         const long long c = cell(l, c0 + p);
-        double q[6], fp[5], fm[5];
-        for (int n = 0; n < 6; n++) q[n] = a.Q[c + n * pl];
-        split_cell<double>(P.split, P.cd, q, a.csnd[c], a.A[0][c], a.A[1][c], a.A[2][c], a.Ah[0][c], a.Ah[1][c],
-                           a.Ah[2][c], a.S[c], fp, fm);
+        F64 q[6], fp[5], fm[5];
+        for (int n = 0; n < 6; n++) q[n] = f64(a.Q[c + n * pl]);
+        split_cell<F64>(P.split, P.cd, q, f64(a.csnd[c]), f64(a.A[0][c]), f64(a.A[1][c]), f64(a.A[2][c]),
+                        f64(a.Ah[0][c]), f64(a.Ah[1][c]), f64(a.Ah[2][c]), f64(a.S[c]), fp, fm);
         for (int n = 0; n < 5; n++) {
-            sFp[n * TL * NP + s] = fp[n];
-            sFm[n * TL * NP + s] = fm[n];
+            sFp[n * TL * NP + s] = fp[n].v;
+            sFm[n * TL * NP + s] = fm[n].v;
         }
         if (hybrid) sPhi[s] = a.phi[c];
     }
@@ -128,15 +128,14 @@ __global__ void __launch_bounds__(VTile<DIR, CHAR>::NT, VTile<DIR, CHAR>::MINB) 
         const int f = c0 + t;  // interior face index 0..Nd
         // L_c = J_c (F[left face of c] - F[right face of c]): face f is the left face of
         // interior cell f and the right face of interior cell f-1
-        double Fb[5] = {0, 0, 0, 0, 0};
+        double Fb[5];
         const long long cr = cell(l, f + NG), cl = cr - stride;
-        if (f < Nd) {
-            const double j = a.J[cr];
-            for (int n = 0; n < 5; n++) Fb[n] += j * a.Lb[cr + n * pl];
-        }
-        if (f >= 1) {
-            const double j = a.J[cl];
-            for (int n = 0; n < 5; n++) Fb[n] -= j * a.Lb[cl + n * pl];
+        {
+            const F64 jr = f64(f < Nd ? a.J[cr] : 0.0), jl = f64(f >= 1 ? a.J[cl] : 0.0);
+            for (int n = 0; n < 5; n++) {
+                const F64 r = f64(f < Nd ? a.Lb[cr + n * pl] : 0.0), g = f64(f >= 1 ? a.Lb[cl + n * pl] : 0.0);
+                Fb[n] = (jr * r - jl * g).v;
+            }
         }
         if (br == 0) {  // UP7 (schemes.jl:119-142): the face cotangent, gathered in Phase C
             for (int n = 0; n < 5; n++) sG[n * TL * NFV + gidx(l, t)] = Fb[n];
@@ -266,46 +265,83 @@ __global__ void __launch_bounds__(VTile<DIR, CHAR>::NT, VTile<DIR, CHAR>::MINB) 
     }
     __syncthreads();
 
+    // The transpose of the linear faces: position p takes Fp from the faces t = p - k with
+    // coefficient lin[k] and Fm from the faces t = p - 7 + k (face t reads positions t..t+6 and
+    // t+7..t+1), i.e. the two one-sided combinations of the face cotangents G over p-7..p, as integer
+    // sums over strips of five positions and one component (f3d_fixed.cuh): 20 FP64 instructions a
+    // position instead of 80
+    if (P.lin_int && P.fixed_branch <= 0) {
+        const int np = nc + 8, ns = (np + LIN_STRIP - 1) / LIN_STRIP, per = ns * (DIR == 0 ? nl : TL);
+        for (int k = threadIdx.x; k < 5 * per; k += NT) {
+            const int n = k / per, r = k - n * per;
+            int l, sp;
+            if (DIR == 0) { l = r / ns; sp = r - l * ns; } else { sp = r / TL; l = r - sp * TL; }
+            if (l >= nl) continue;
+            const int p0 = sp * LIN_STRIP;
+            const double* G = sG + n * TL * NFV;
+            double gm[LIN_STRIP], gp[LIN_STRIP];
+            linear_strip_both(P, p0 - 7, [&](int t) { return t >= 0 && t < NFV ? G[gidx(l, t)] : 0.0; }, gm, gp);
+#pragma unroll
+            for (int f = 0; f < LIN_STRIP; f++)
+                if (p0 + f < np) {
+                    const int s = n * TL * NP + sidx(l, p0 + f);
+                    // linear faces alone leave the cotangents at zero so far
+                    if (__double_as_longlong(gp[f]) << 1) sFpb[s] = (f64(sFpb[s]) + f64(gp[f])).v;
+                    if (__double_as_longlong(gm[f]) << 1) sFmb[s] = (f64(sFmb[s]) + f64(gm[f])).v;
+                }
+        }
+        __syncthreads();
+    }
+
     // Phase C: reverse of the split at every position, into Qb
     for (int it = threadIdx.x; it < TL * NP; it += NT) {
         int l, p;
         if (DIR == 0) { l = it / NP; p = it - l * NP; } else { p = it / TL; l = it - p * TL; }
         if (l >= nl || p >= nc + 8) continue;
         const int s = sidx(l, p);
-        double fpb[5], fmb[5];
+        F64 fpb[5], fmb[5];
         bool any = false;
         for (int n = 0; n < 5; n++) {
-            // UP7 faces t = p - k take Fp here with coefficient lin[k], faces t = p - 7 + k
-            // take Fm here with lin[k] (positions t..t+6 and t+7..t+1 of face t)
-            const double* G = sG + n * TL * NFV;
-            double gp = 0.0, gm = 0.0;
+            const int o = n * TL * NP + s;
+            fpb[n] = f64(sFpb[o]);
+            fmb[n] = f64(sFmb[o]);
+            if (!P.lin_int) {  // the linear faces' transpose in FP64
+                const double* G = sG + n * TL * NFV;
 #pragma unroll
-            for (int k = 0; k < 7; k++) {
-                const int tp = p - k, tm = p - 7 + k;
-                if (tp >= 0 && tp < NFV) gp += P.cd.lin[k] * G[gidx(l, tp)];
-                if (tm >= 0 && tm < NFV) gm += P.cd.lin[k] * G[gidx(l, tm)];
+                for (int k = 0; k < 7; k++) {
+                    const int tp = p - k, tm = p - 7 + k;
+                    if (tp >= 0 && tp < NFV) fpb[n] += P.cd.lin[k] * f64(G[gidx(l, tp)]);
+                    if (tm >= 0 && tm < NFV) fmb[n] += P.cd.lin[k] * f64(G[gidx(l, tm)]);
+                }
             }
-            fpb[n] = sFpb[n * TL * NP + s] + gp;
-            fmb[n] = sFmb[n * TL * NP + s] + gm;
-            any |= fpb[n] != 0.0 || fmb[n] != 0.0;
+            any |= ((__double_as_longlong(fpb[n].v) | __double_as_longlong(fmb[n].v)) << 1) != 0;
         }
         if (!any) continue;
         const long long c = cell(l, c0 + p);
-        double q[6], qb[6] = {0, 0, 0, 0, 0, 0};
+        double qb[6] = {0, 0, 0, 0, 0, 0};
         double mg[7] = {0, 0, 0, 0, 0, 0, 0};
         double* mgp = a.mb[0] ? mg : nullptr;
-        for (int n = 0; n < 6; n++) q[n] = a.Q[c + n * pl];
         const double A3[3] = {a.A[0][c], a.A[1][c], a.A[2][c]};
         const double S = a.S[c];
-        if (P.split == F3D_SPLIT_SW)
-            split_sw_vjp(P.cd, q, a.csnd[c], A3[0], A3[1], A3[2], a.Ah[0][c], a.Ah[1][c], a.Ah[2][c], S, fpb, fmb, qb,
-                         mgp);
-        else if (P.split == F3D_SPLIT_LF)
-            split_lf_vjp(P.cd, q, a.csnd[c], A3[0], A3[1], A3[2], S, fpb, fmb, qb, mgp);
-        else  // van Leer, AUSM
-            split_mach_vjp(P.split, P.cd, q, a.csnd[c], A3[0], A3[1], A3[2], S, fpb, fmb, qb, mgp);
+        if (P.split == F3D_SPLIT_SW) {
+            F64 q[6], qs[6], ms[7];
+            for (int n = 0; n < 6; n++) q[n] = f64(a.Q[c + n * pl]);
+            for (int n = 0; n < 7; n++) ms[n] = f64(0.0);
+            split_sw_vjp(P.cd, q, f64(a.csnd[c]), f64(a.Ah[0][c]), f64(a.Ah[1][c]), f64(a.Ah[2][c]), f64(S), fpb, fmb,
+                         qs, mgp ? ms : nullptr);
+            for (int n = 0; n < 6; n++) qb[n] = qs[n].v;
+            for (int n = 0; n < 7; n++) mg[n] = ms[n].v;
+        } else {
+            double q[6], fp[5], fm[5];
+            for (int n = 0; n < 6; n++) q[n] = a.Q[c + n * pl];
+            for (int n = 0; n < 5; n++) { fp[n] = fpb[n].v; fm[n] = fmb[n].v; }
+            if (P.split == F3D_SPLIT_LF)
+                split_lf_vjp(P.cd, q, a.csnd[c], A3[0], A3[1], A3[2], S, fp, fm, qb, mgp);
+            else  // van Leer, AUSM
+                split_mach_vjp(P.split, P.cd, q, a.csnd[c], A3[0], A3[1], A3[2], S, fp, fm, qb, mgp);
+        }
         for (int n = 0; n < 6; n++)
-            if (qb[n] != 0.0) atomicAdd(&a.Qb[c + n * pl], qb[n]);
+            if (__double_as_longlong(qb[n]) << 1) atomicAdd(&a.Qb[c + n * pl], qb[n]);
         if (mgp) {
             // A/|A| and |A| derive from A: A_j-bar += H_j-bar/S - (H-bar . A) A_j/S^3 + S-bar A_j/S
             const double iS = 1.0 / S;
@@ -330,7 +366,7 @@ __global__ void k_visc_fvb(const DevParams P, const double* __restrict__ Lb, con
     int vi, vj, vk;
     split3(t, P.dvxt, P.dvyt, vi, vj, vk);
     const int gi = vi + 2, gj = vj + 2, gk = vk + 2;  // full cell index
-    const double k1 = 1.0 / 12.0, k2 = -2.0 / 3.0;
+    const F64 k1 = 1.0 / 12.0, k2 = -2.0 / 3.0;
     const int g[3] = {gi, gj, gk};
     const int N[3] = {P.nx, P.ny, P.nz};
     const long long st[3] = {1, (long long)P.nxt, (long long)P.nxt * P.nyt};
@@ -342,19 +378,19 @@ __global__ void k_visc_fvb(const DevParams P, const double* __restrict__ Lb, con
         bool tr = true;
         for (int e = 0; e < 3; e++)
             if (e != d && !inside(e, g[e])) tr = false;
-        double acc[4] = {0, 0, 0, 0};
+        F64 acc[4] = {f64(0.0), f64(0.0), f64(0.0), f64(0.0)};
         if (tr) {
             const int offs[4] = {2, -2, 1, -1};
-            const double coef[4] = {k1, -k1, k2, -k2};  // F[c'] enters cell c'+2 with +k1, c'-2 with -k1, ...
+            const F64 coef[4] = {k1, -k1, k2, -k2};  // F[c'] enters cell c'+2 with +k1, c'-2 with -k1, ...
             for (int o = 0; o < 4; o++) {
                 const int gg = g[d] + offs[o];
                 if (!inside(d, gg)) continue;
                 const long long cc = c + offs[o] * st[d];
-                const double w = coef[o] * J[cc];
-                for (int n = 0; n < 4; n++) acc[n] += w * Lb[cc + (n + 1) * P.plane];
+                const F64 w = coef[o] * f64(J[cc]);
+                for (int n = 0; n < 4; n++) acc[n] += w * f64(Lb[cc + (n + 1) * P.plane]);
             }
         }
-        for (int n = 0; n < 4; n++) out[d][t + n * vpl] = acc[n];
+        for (int n = 0; n < 4; n++) out[d][t + n * vpl] = acc[n].v;
     }
 }
 
@@ -373,44 +409,45 @@ __global__ void k_visc_vjp(const DevParams P, const double* __restrict__ Q, cons
     split3(t, P.dvxt, P.dvyt, vi, vj, vk);
     const long long c = lin3(P, vi + 2, vj + 2, vk + 2);
     const long long pl = P.plane, sy = P.nxt, sz = (long long)P.nxt * P.nyt;
-    const double M[3][3] = {{m0[c], m1[c], m2[c]}, {m3[c], m4[c], m5[c]}, {m6[c], m7[c], m8[c]}};  // M[d][x]
-    const double Jac = J[c];
-    const double T = Q[c + 5 * pl];
-    const double sT = sqrt(T);
-    const double rTs = 1.0 / (T + P.t_s);
-    const double mu = P.c_s * T * sT * rTs;
-    const double lam = mu * P.cd.cp_pr;
-    const double c1 = 1.0 / 12.0, c2 = -2.0 / 3.0, c23 = 2.0 / 3.0;
+    const F64 M[3][3] = {{f64(m0[c]), f64(m1[c]), f64(m2[c])}, {f64(m3[c]), f64(m4[c]), f64(m5[c])}, {f64(m6[c]), f64(m7[c]), f64(m8[c])}};  // M[d][x]
+    const F64 Jac = f64(J[c]);
+    const F64 T = f64(Q[c + 5 * pl]);
+    const F64 sT = root(T);
+    const F64 rTs = recip(T + F64(P.t_s));
+    const F64 mu = ((F64(P.c_s) * T) * sT) * rTs;
+    const F64 lam = mu * F64(P.cd.cp_pr);
+    const F64 c1 = 1.0 / 12.0, c2 = -2.0 / 3.0, c23 = 2.0 / 3.0, two = 2.0;
     // forward: computational gradients G[var][d] of (u, v, w, T) and physical D[var][x]
     const int vars[4] = {1, 2, 3, 5};
     const long long st[3] = {1, sy, sz};
-    double G[4][3], D[4][3];
+    F64 G[4][3], D[4][3];
     for (int a = 0; a < 4; a++)
         for (int d = 0; d < 3; d++) {
             const double* f = Q + vars[a] * pl + c;
-            G[a][d] = c1 * (f[-2 * st[d]] - f[2 * st[d]]) + c2 * (f[-st[d]] - f[st[d]]);
+            G[a][d] = c1 * (f64(f[-2 * st[d]]) - f64(f[2 * st[d]])) + c2 * (f64(f[-st[d]]) - f64(f[st[d]]));
         }
     for (int a = 0; a < 4; a++)
         for (int x = 0; x < 3; x++) D[a][x] = (G[a][0] * M[0][x] + G[a][1] * M[1][x] + G[a][2] * M[2][x]) * Jac;
-    const double uvw[3] = {Q[c + pl], Q[c + 2 * pl], Q[c + 3 * pl]};
-    const double dv = D[0][0] + D[1][1] + D[2][2];
-    double tau[3][3];
+    const F64 uvw[3] = {f64(Q[c + pl]), f64(Q[c + 2 * pl]), f64(Q[c + 3 * pl])};
+    const F64 dv = D[0][0] + D[1][1] + D[2][2];
+    F64 tau[3][3];
     for (int x = 0; x < 3; x++)
         for (int y = 0; y < 3; y++) tau[x][y] = mu * (D[x][y] + D[y][x]);
-    for (int x = 0; x < 3; x++) tau[x][x] = mu * (2.0 * D[x][x] - c23 * dv);
+    for (int x = 0; x < 3; x++) tau[x][x] = mu * (two * D[x][x] - c23 * dv);
     // E_x = sum_y u_y tau[y][x] + lam dT/dx
     // reverse: Fv_d[n] = sum_x M[d][x] tau[x][n] (n < 3), Fv_d[3] = sum_x M[d][x] E_x
     const double* Fvb[3] = {Fvbx, Fvby, Fvbz};
-    double taub[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, Eb[3] = {0, 0, 0};
+    const F64 zero = f64(0.0);
+    F64 taub[3][3] = {{zero, zero, zero}, {zero, zero, zero}, {zero, zero, zero}}, Eb[3] = {zero, zero, zero};
     for (int d = 0; d < 3; d++) {
-        const double fb[4] = {Fvb[d][t], Fvb[d][t + vpl], Fvb[d][t + 2 * vpl], Fvb[d][t + 3 * vpl]};
+        const F64 fb[4] = {f64(Fvb[d][t]), f64(Fvb[d][t + vpl]), f64(Fvb[d][t + 2 * vpl]), f64(Fvb[d][t + 3 * vpl])};
         for (int x = 0; x < 3; x++) {
             for (int n = 0; n < 3; n++) taub[x][n] += M[d][x] * fb[n];
             Eb[x] += M[d][x] * fb[3];
         }
     }
-    double ub[3] = {0, 0, 0}, lamb = 0, mub = 0;
-    double Db[4][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+    F64 ub[3] = {zero, zero, zero}, lamb = zero, mub = zero;
+    F64 Db[4][3] = {{zero, zero, zero}, {zero, zero, zero}, {zero, zero, zero}, {zero, zero, zero}};
     for (int x = 0; x < 3; x++) {
         for (int y = 0; y < 3; y++) {
             ub[y] += Eb[x] * tau[y][x];
@@ -420,54 +457,53 @@ __global__ void k_visc_vjp(const DevParams P, const double* __restrict__ Q, cons
         Db[3][x] += Eb[x] * lam;
     }
     // tau is symmetric in the forward; taub holds the cotangent of each (x,y) entry as used
-    double dvb = 0;
+    F64 dvb = zero;
     for (int x = 0; x < 3; x++)
         for (int y = 0; y < 3; y++) {
-            const double g = taub[x][y];
+            const F64 g = taub[x][y], gmu = g * mu;
             if (x == y) {
-                mub += g * (2.0 * D[x][x] - c23 * dv);
-                Db[x][x] += g * mu * 2.0;
-                dvb += -g * mu * c23;
+                mub += g * (two * D[x][x] - c23 * dv);
+                Db[x][x] += gmu * two;
+                dvb -= gmu * c23;
             } else {
                 mub += g * (D[x][y] + D[y][x]);
-                Db[x][y] += g * mu;
-                Db[y][x] += g * mu;
+                Db[x][y] += gmu;
+                Db[y][x] += gmu;
             }
         }
     Db[0][0] += dvb;
     Db[1][1] += dvb;
     Db[2][2] += dvb;
     // lambda = cp mu / Pr; mu = C_s T^1.5 / (T + T_s)
-    mub += lamb * P.cd.cp_pr;
-    const double Tb_mu = mub * P.c_s * (1.5 * sT * (T + P.t_s) - T * sT) * (rTs * rTs);
+    mub += lamb * F64(P.cd.cp_pr);
+    const F64 Tb_mu = ((mub * F64(P.c_s)) * (F64(1.5) * sT * (T + F64(P.t_s)) - T * sT)) * (rTs * rTs);
     // D[a][x] = (sum_d G[a][d] M[d][x]) J
     for (int a = 0; a < 4; a++)
         for (int d = 0; d < 3; d++) {
-            double g = 0;
-            for (int x = 0; x < 3; x++) g += Db[a][x] * M[d][x];
-            gb[t + (a * 3 + d) * vpl] = g * Jac;
+            const F64 g = Db[a][0] * M[d][0] + Db[a][1] * M[d][1] + Db[a][2] * M[d][2];
+            gb[t + (a * 3 + d) * vpl] = F64(g * Jac).v;
         }
-    atomicAdd(&Qb[c + pl], ub[0]);
-    atomicAdd(&Qb[c + 2 * pl], ub[1]);
-    atomicAdd(&Qb[c + 3 * pl], ub[2]);
-    atomicAdd(&Qb[c + 5 * pl], Tb_mu);
+    atomicAdd(&Qb[c + pl], ub[0].v);
+    atomicAdd(&Qb[c + 2 * pl], ub[1].v);
+    atomicAdd(&Qb[c + 3 * pl], ub[2].v);
+    atomicAdd(&Qb[c + 5 * pl], Tb_mu.v);
     if (mbar.m[0]) {
         // metric cotangents of this cell: the projections Fv_d = sum_x M[d][x] (tau, E)[x] and
         // the gradients D[a][x] = (sum_d G[a][d] M[d][x]) J
-        double E[3];
+        F64 E[3];
         for (int x = 0; x < 3; x++) E[x] = uvw[0] * tau[0][x] + uvw[1] * tau[1][x] + uvw[2] * tau[2][x] + lam * D[3][x];
-        double Jb = 0.0;
+        F64 Jb = zero;
         for (int a = 0; a < 4; a++)
             for (int x = 0; x < 3; x++) Jb += Db[a][x] * D[a][x];
         for (int d = 0; d < 3; d++) {
-            const double fb[4] = {Fvb[d][t], Fvb[d][t + vpl], Fvb[d][t + 2 * vpl], Fvb[d][t + 3 * vpl]};
+            const F64 fb[4] = {f64(Fvb[d][t]), f64(Fvb[d][t + vpl]), f64(Fvb[d][t + 2 * vpl]), f64(Fvb[d][t + 3 * vpl])};
             for (int x = 0; x < 3; x++) {
-                double b = fb[0] * tau[x][0] + fb[1] * tau[x][1] + fb[2] * tau[x][2] + fb[3] * E[x];
-                for (int a = 0; a < 4; a++) b += Db[a][x] * G[a][d] * Jac;
-                mbar.m[3 * d + x][c] += mbar.scale * b;  // one thread per cell, after the sweeps
+                F64 b = fb[0] * tau[x][0] + fb[1] * tau[x][1] + fb[2] * tau[x][2] + fb[3] * E[x];
+                for (int a = 0; a < 4; a++) b += (Db[a][x] * G[a][d]) * Jac;
+                mbar.m[3 * d + x][c] += mbar.scale * b.v;  // one thread per cell, after the sweeps
             }
         }
-        mbar.J[c] += mbar.scale * Jb / Jac;
+        mbar.J[c] += mbar.scale * Jb.v / Jac.v;
     }
 }
 
@@ -493,11 +529,11 @@ __global__ void k_visc_gather(const DevParams P, const double* __restrict__ gb, 
     split3(c, P.dnxt, P.dnyt, i, j, k);
     const int vxt = P.nxt - 4, vyt = P.nyt - 4, vzt = P.nzt - 4;
     const long long vpl = (long long)vxt * vyt * vzt;
-    const double c1 = 1.0 / 12.0, c2 = -2.0 / 3.0;
+    const F64 c1 = 1.0 / 12.0, c2 = -2.0 / 3.0;
     const int g[3] = {i, j, k};
     const int vn[3] = {vxt, vyt, vzt};
     const int vars[4] = {1, 2, 3, 5};
-    double acc[4] = {0, 0, 0, 0};
+    F64 acc[4] = {f64(0.0), f64(0.0), f64(0.0), f64(0.0)};
     for (int d = 0; d < 3; d++) {
         // box index of c along the other dimensions must be valid
         bool ok = true;
@@ -509,17 +545,17 @@ __global__ void k_visc_gather(const DevParams P, const double* __restrict__ gb, 
         if (!ok) continue;
         // c = c' - 2 gets +c1, c = c' + 2 gets -c1, c = c' - 1 gets +c2, c = c' + 1 gets -c2
         const int offs[4] = {2, -2, 1, -1};
-        const double coef[4] = {c1, -c1, c2, -c2};
+        const F64 coef[4] = {c1, -c1, c2, -c2};
         for (int o = 0; o < 4; o++) {
             int vv[3] = {vb[0], vb[1], vb[2]};
             vv[d] += offs[o];
             if (vv[d] < 0 || vv[d] >= vn[d]) continue;
             const long long tc = vv[0] + (long long)vxt * (vv[1] + (long long)vyt * vv[2]);
-            for (int a = 0; a < 4; a++) acc[a] += coef[o] * gb[tc + (a * 3 + d) * vpl];
+            for (int a = 0; a < 4; a++) acc[a] += coef[o] * f64(gb[tc + (a * 3 + d) * vpl]);
         }
     }
     for (int a = 0; a < 4; a++)
-        if (acc[a] != 0.0) Qb[c + vars[a] * P.plane] += acc[a];
+        if (__double_as_longlong(acc[a].v) << 1) Qb[c + vars[a] * P.plane] += acc[a].v;
 }
 
 // ---- ghost fill and c2Prim -----------------------------------------------------------
@@ -586,8 +622,8 @@ __global__ void k_c2prim_vjp(const DevParams P, const double* __restrict__ U, co
     for (int n = 0; n < 6; n++) qb[n] = Qb[c + n * pl];
     c2prim_vjp(P, u, qb, ub);
     for (int n = 0; n < 5; n++) {
-        const double o = beta == 0.0 ? 0.0 : beta * out[c + n * pl];
-        out[c + n * pl] = o + alpha * ub[n];
+        const F64 r = F64(alpha) * f64(ub[n]);
+        out[c + n * pl] = beta == 0.0 ? r.v : (F64(beta) * f64(out[c + n * pl]) + r).v;
     }
 }
 
@@ -600,7 +636,7 @@ __global__ void k_axpby(const DevParams P, double* out, const double* x, double 
     const bool in = i >= NG && i < P.nx + NG && j >= NG && j < P.ny + NG && k >= NG && k < P.nz + NG;
     for (int n = 0; n < 5; n++) {
         const long long o = c + n * P.plane;
-        out[o] = in ? a * x[o] + (y ? b * y[o] : 0.0) : 0.0;
+        out[o] = in ? (y ? (F64(a) * f64(x[o]) + F64(b) * f64(y[o])).v : F64(F64(a) * f64(x[o])).v) : 0.0;
     }
 }
 

@@ -16,7 +16,7 @@
 //   shared epilogue (differences, viscous CD4, accumulation).
 // k_stage_update: the RK update U = ca (U + dt J acc) + cb Un at interior cells. The
 //   finite-volume sweeps read U, so the stage cannot update it inside the last sweep.
-#include "f3d_kernels.cuh"
+#include "f3d_fixed.cuh"
 #include "f3d_sweep_epilogue.cuh"
 
 namespace f3d {
@@ -212,7 +212,7 @@ template <> struct FvmLaunch<false> { static constexpr int NT = FVM_C_THREADS, M
 
 template <int DIR> constexpr size_t fvm_smem_bytes() {
     constexpr int TL = FTile<DIR>::TL, TC = FTile<DIR>::TC, NP = TC + 8, NF = TC + 1;
-    return sizeof(double) * ((size_t)TL * NP * 6 + (size_t)TL * NF * 5) + sizeof(int) * ((size_t)TL * NF + 2);
+    return sizeof(double) * ((size_t)TL * NP * 6 + (size_t)TL * NF * 15) + sizeof(int) * ((size_t)TL * NF + 2);
 }
 
 template <int DIR, bool EIGEN>
@@ -227,7 +227,8 @@ __global__ void __launch_bounds__(FvmLaunch<EIGEN>::NT, FvmLaunch<EIGEN>::MINB) 
     double* sU = reinterpret_cast<double*>(smem_raw);  // [5][TL*NP]
     double* sPhi = sU + 5 * TL * NP;                    // [TL*NP]
     double* sF = sPhi + TL * NP;                        // [5][TL*NF]
-    int* list = reinterpret_cast<int*>(sF + 5 * TL * NF);
+    double* sL = sF + 5 * TL * NF;                      // [10][TL*NF] left and right linear states
+    int* list = reinterpret_cast<int*>(sL + 10 * TL * NF);
     int* count = list + TL * NF;
     const double* Q = static_cast<const double*>(a.Q);
     const double* S = static_cast<const double*>(a.S);
@@ -264,13 +265,43 @@ __global__ void __launch_bounds__(FvmLaunch<EIGEN>::NT, FvmLaunch<EIGEN>::MINB) 
     }
     __syncthreads();
 
+    // The linear scheme's left and right states of every face as integer sums over strips of five
+    // faces and one component (f3d_fixed.cuh): 10 FP64 instructions a face instead of 70
+    if (P.lin_int && P.fixed_branch <= 0) {
+        const int ns = (nc + LIN_STRIP) / LIN_STRIP, per = ns * (DIR == 0 ? nl : TL), last = nc + 7;
+        for (int k = threadIdx.x; k < 5 * per; k += FVM_THREADS) {
+            const int n = k / per, r = k - n * per;
+            int l, st;
+            if (DIR == 0) { l = r / ns; st = r - l * ns; } else { st = r / TL; l = r - st * TL; }
+            if (l >= nl) continue;
+            const int t0 = st * LIN_STRIP;
+            const double* u = sU + n * TL * NP;
+            double up[LIN_STRIP], down[LIN_STRIP];
+            linear_strip_both(P, t0, [&](int p) { return p <= last ? u[sidx(l, p)] : 0.0; }, up, down);
+#pragma unroll
+            for (int f = 0; f < LIN_STRIP; f++)
+                if (t0 + f <= nc) {
+                    sL[n * TL * NF + fidx(l, t0 + f)] = up[f];
+                    sL[(n + 5) * TL * NF + fidx(l, t0 + f)] = down[f];
+                }
+        }
+        __syncthreads();
+    }
+
     // Phase B: face t between positions t+3 (left cell, the kernels' i) and t+4
     auto face = [&](int l, int t, int br) {
         const long long cl = cell(l, c0 + t + 3);
         auto Uv = [&](int n, int p) { return f64(sU[n * TL * NP + sidx(l, p)]); };
         const F64 nx = f64(gnx[cl]), ny = f64(gny[cl]), nz = f64(gnz[cl]);
         F64 UL[5], UR[5];
-        if (br == 0) {  // linear scheme on U, FVM.jl:42-60
+        if (br == 0 && P.lin_int) {  // linear scheme on U, FVM.jl:42-60, summed by the strips
+            const int f = fidx(l, t);
+#pragma unroll
+            for (int n = 0; n < 5; n++) {
+                UL[n] = f64(sL[n * TL * NF + f]);
+                UR[n] = f64(sL[(n + 5) * TL * NF + f]);
+            }
+        } else if (br == 0) {
 #pragma unroll
             for (int n = 0; n < 5; n++) {
                 F64 vl = P.cd.lin[0] * Uv(n, t), vr = P.cd.lin[0] * Uv(n, t + 7);
