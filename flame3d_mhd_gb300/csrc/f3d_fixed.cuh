@@ -67,6 +67,27 @@ __device__ __forceinline__ double fixed_to_f64(long long T, unsigned r, int E) {
     return __longlong_as_double((long long)(b | (neg ? 0x8000000000000000ull : 0ull)));
 }
 
+// 12 times the fourth-order central difference, (a - d) - 8 (b - c) for a, b, c, d = f[-2], f[-1], f[1],
+// f[2] (viscous.jl:29-42), rounded once: no FP64 instruction instead of four (the 1/12 goes into a
+// metric factor). Values within 2^9 of the largest enter exactly. `plain` is cleared for values
+// outside 2^-823 .. 2^877 (infinities and NaN among them): the caller then takes difference12_fp64 for
+// all of its differences, in a block of its own (a fallback beside each call is turned into predicated
+// FP64 instructions, which hold the pipe although no lane runs them).
+__device__ __forceinline__ F64 difference12(double a, double b, double c, double d, bool& plain) {
+    unsigned top = 0u;
+    top = max(max((unsigned)__double2hiint(a) & 0x7fffffffu, (unsigned)__double2hiint(b) & 0x7fffffffu),
+              max((unsigned)__double2hiint(c) & 0x7fffffffu, (unsigned)__double2hiint(d) & 0x7fffffffu));
+    const int E = (int)(top >> 20);
+    plain = plain && (top == 0u || (E >= 200 && E <= 1900));
+    const long long x = fixed_of(a, E) - fixed_of(d, E), y = fixed_of(b, E) - fixed_of(c, E);  // below 2^63
+    const long long l = (long long)(unsigned)x - 8ll * (long long)(unsigned)y;
+    const double r = fixed_to_f64((x >> 32) - 8ll * (y >> 32) + (l >> 32), (unsigned)l, E);
+    return f64(top == 0u ? 0.0 : r);
+}
+__device__ __forceinline__ F64 difference12_fp64(double a, double b, double c, double d) {
+    return (f64(a) - f64(d)) - F64(8.0) * (f64(b) - f64(c));
+}
+
 // The two one-sided linear combinations of one array on a strip: up[f] = sum_k lin[k] V(t0 + f + k) and
 // down[f] = sum_k lin[k] V(t0 + f + 7 - k), f = 0..4 (the left and right states of finite-volume faces;
 // the transpose of the linear faces in the reverse sweeps). V(p) is read at p = t0 .. t0 + 11;

@@ -416,18 +416,34 @@ __global__ void k_visc_vjp(const DevParams P, const double* __restrict__ Q, cons
     const F64 rTs = recip(T + F64(P.t_s));
     const F64 mu = ((F64(P.c_s) * T) * sT) * rTs;
     const F64 lam = mu * F64(P.cd.cp_pr);
-    const F64 c1 = 1.0 / 12.0, c2 = -2.0 / 3.0, c23 = 2.0 / 3.0, two = 2.0;
+    const F64 c1 = 1.0 / 12.0, c23 = 2.0 / 3.0, two = 2.0;
+    const F64 j12 = Jac * c1;
+    F64 B[3][3];  // the metrics times J/12: G holds 12 times the differences
+    for (int d = 0; d < 3; d++)
+        for (int x = 0; x < 3; x++) B[d][x] = M[d][x] * j12;
     // forward: computational gradients G[var][d] of (u, v, w, T) and physical D[var][x]
     const int vars[4] = {1, 2, 3, 5};
     const long long st[3] = {1, sy, sz};
     F64 G[4][3], D[4][3];
+    bool plain_values = true;
+#pragma unroll
     for (int a = 0; a < 4; a++)
+#pragma unroll
         for (int d = 0; d < 3; d++) {
             const double* f = Q + vars[a] * pl + c;
-            G[a][d] = c1 * (f64(f[-2 * st[d]]) - f64(f[2 * st[d]])) + c2 * (f64(f[-st[d]]) - f64(f[st[d]]));
+            G[a][d] = difference12(f[-2 * st[d]], f[-st[d]], f[st[d]], f[2 * st[d]], plain_values);  // 12 times
         }
+    if (!plain_values) {
+#pragma unroll
+        for (int a = 0; a < 4; a++)
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                const volatile double* f = Q + vars[a] * pl + c;  // read again: not held meanwhile
+                G[a][d] = difference12_fp64(f[-2 * st[d]], f[-st[d]], f[st[d]], f[2 * st[d]]);
+            }
+    }
     for (int a = 0; a < 4; a++)
-        for (int x = 0; x < 3; x++) D[a][x] = (G[a][0] * M[0][x] + G[a][1] * M[1][x] + G[a][2] * M[2][x]) * Jac;
+        for (int x = 0; x < 3; x++) D[a][x] = G[a][0] * B[0][x] + G[a][1] * B[1][x] + G[a][2] * B[2][x];
     const F64 uvw[3] = {f64(Q[c + pl]), f64(Q[c + 2 * pl]), f64(Q[c + 3 * pl])};
     const F64 dv = D[0][0] + D[1][1] + D[2][2];
     F64 tau[3][3];
@@ -480,8 +496,8 @@ __global__ void k_visc_vjp(const DevParams P, const double* __restrict__ Q, cons
     // D[a][x] = (sum_d G[a][d] M[d][x]) J
     for (int a = 0; a < 4; a++)
         for (int d = 0; d < 3; d++) {
-            const F64 g = Db[a][0] * M[d][0] + Db[a][1] * M[d][1] + Db[a][2] * M[d][2];
-            gb[t + (a * 3 + d) * vpl] = F64(g * Jac).v;
+            // of 12 times the difference: k_visc_gather applies the integer coefficients 1 and -8
+            gb[t + (a * 3 + d) * vpl] = (Db[a][0] * B[d][0] + Db[a][1] * B[d][1] + Db[a][2] * B[d][2]).v;
         }
     atomicAdd(&Qb[c + pl], ub[0].v);
     atomicAdd(&Qb[c + 2 * pl], ub[1].v);
@@ -499,7 +515,7 @@ __global__ void k_visc_vjp(const DevParams P, const double* __restrict__ Q, cons
             const F64 fb[4] = {f64(Fvb[d][t]), f64(Fvb[d][t + vpl]), f64(Fvb[d][t + 2 * vpl]), f64(Fvb[d][t + 3 * vpl])};
             for (int x = 0; x < 3; x++) {
                 F64 b = fb[0] * tau[x][0] + fb[1] * tau[x][1] + fb[2] * tau[x][2] + fb[3] * E[x];
-                for (int a = 0; a < 4; a++) b += (Db[a][x] * G[a][d]) * Jac;
+                for (int a = 0; a < 4; a++) b += (Db[a][x] * G[a][d]) * j12;
                 mbar.m[3 * d + x][c] += mbar.scale * b.v;  // one thread per cell, after the sweeps
             }
         }
@@ -520,7 +536,7 @@ __global__ void k_jbar(const DevParams P, const double* __restrict__ Lb, const d
     Jbar[c] += scale * s / J[c];
 }
 
-// Transpose of the CD4 gradients: G[c'] = c1 (f[c'-2] - f[c'+2]) + c2 (f[c'-1] - f[c'+1]),
+// Transpose of 12 times the CD4 gradients: G[c'] = c1 (f[c'-2] - f[c'+2]) + c2 (f[c'-1] - f[c'+1]), c1 = 1, c2 = -8,
 // gathered at every cell c from the box cells c' = c -+ 1, 2 that used it.
 __global__ void k_visc_gather(const DevParams P, const double* __restrict__ gb, double* Qb) {
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -529,7 +545,7 @@ __global__ void k_visc_gather(const DevParams P, const double* __restrict__ gb, 
     split3(c, P.dnxt, P.dnyt, i, j, k);
     const int vxt = P.nxt - 4, vyt = P.nyt - 4, vzt = P.nzt - 4;
     const long long vpl = (long long)vxt * vyt * vzt;
-    const F64 c1 = 1.0 / 12.0, c2 = -2.0 / 3.0;
+    const F64 c1 = 1.0, c2 = -8.0;
     const int g[3] = {i, j, k};
     const int vn[3] = {vxt, vyt, vzt};
     const int vars[4] = {1, 2, 3, 5};

@@ -6,7 +6,7 @@
 // chain rule with the J^-1-scaled metrics and J, Sutherland viscosity, Stokes stress and
 // Fourier heat flux, projected on the three metric rows. Output arrays have the
 // reference's Fv_x/Fv_y/Fv_z shape ((Nt-4)^3 x 4) with Fv index = cell index - 2.
-#include "f3d_kernels.cuh"
+#include "f3d_fixed.cuh"
 
 namespace f3d {
 
@@ -45,28 +45,68 @@ __global__ void __launch_bounds__(128) k_viscous(const DevParams P, const R* __r
         mu = K.c_s * T * sqrt(T) / (T + K.t_s);
     }
     A lam = mu * A(K.cp_pr);
-    const A c1 = A(1.0 / 12.0), c2 = A(-2.0 / 3.0), c23 = A(2.0 / 3.0);
-    auto d4 = [&](int n, long long s) {
-        const R* f = Q + n * pl + c;
-        return c1 * (arith(f[-2 * s]) - arith(f[2 * s])) + c2 * (arith(f[-s]) - arith(f[s]));
-    };
-    // viscous.jl:29-42: the CD4 coefficients give +d/dxi
-    const A uxi = d4(1, 1), vxi = d4(2, 1), wxi = d4(3, 1), Txi = d4(5, 1);
-    const A uet = d4(1, sy), vet = d4(2, sy), wet = d4(3, sy), Tet = d4(5, sy);
-    const A uze = d4(1, sz), vze = d4(2, sz), wze = d4(3, sz), Tze = d4(5, sz);
+    const A c23 = A(2.0 / 3.0);
+    // viscous.jl:29-42: the CD4 coefficients give +d/dxi. FP64: 12 times the differences as integer
+    // sums, and the metrics times J/12 once instead of J on each physical gradient (120 FP64
+    // instructions a cell instead of 190: the kernel keeps the FP64 pipe 98% busy)
+    const A c1 = A(1.0 / 12.0), c2 = A(-2.0 / 3.0);
+    const int vars[4] = {1, 2, 3, 5};
+    const long long st[3] = {1, sy, sz};
+    A g[4][3];  // u, v, w, T in xi, eta, zeta
+    if constexpr (sizeof(R) == 8) {
+        bool plain_values = true;
+#pragma unroll
+        for (int n = 0; n < 4; n++)
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                const R* f = Q + vars[n] * pl + c;
+                g[n][d] = difference12(f[-2 * st[d]], f[-st[d]], f[st[d]], f[2 * st[d]], plain_values);
+            }
+        if (!plain_values) {
+#pragma unroll
+            for (int n = 0; n < 4; n++)
+#pragma unroll
+                for (int d = 0; d < 3; d++) {
+                    const volatile double* f = Q + vars[n] * pl + c;  // read again: not held meanwhile
+                    g[n][d] = difference12_fp64(f[-2 * st[d]], f[-st[d]], f[st[d]], f[2 * st[d]]);
+                }
+        }
+    } else {
+        auto d4 = [&](int n, long long s) {
+            const R* f = Q + n * pl + c;
+            return c1 * (f[-2 * s] - f[2 * s]) + c2 * (f[-s] - f[s]);
+        };
+        g[0][0] = d4(1, 1); g[1][0] = d4(2, 1); g[2][0] = d4(3, 1); g[3][0] = d4(5, 1);
+        g[0][1] = d4(1, sy); g[1][1] = d4(2, sy); g[2][1] = d4(3, sy); g[3][1] = d4(5, sy);
+        g[0][2] = d4(1, sz); g[1][2] = d4(2, sz); g[2][2] = d4(3, sz); g[3][2] = d4(5, sz);
+    }
+    const A uxi = g[0][0], vxi = g[1][0], wxi = g[2][0], Txi = g[3][0];
+    const A uet = g[0][1], vet = g[1][1], wet = g[2][1], Tet = g[3][1];
+    const A uze = g[0][2], vze = g[1][2], wze = g[2][2], Tze = g[3][2];
     const A u = arith(Q[c + pl]), v = arith(Q[c + 2 * pl]), w = arith(Q[c + 3 * pl]);
-    const A dudx = (uxi * xx + uet * ex + uze * zx) * Jac;
-    const A dudy = (uxi * xy + uet * ey + uze * zy) * Jac;
-    const A dudz = (uxi * xz + uet * ez + uze * zz) * Jac;
-    const A dvdx = (vxi * xx + vet * ex + vze * zx) * Jac;
-    const A dvdy = (vxi * xy + vet * ey + vze * zy) * Jac;
-    const A dvdz = (vxi * xz + vet * ez + vze * zz) * Jac;
-    const A dwdx = (wxi * xx + wet * ex + wze * zx) * Jac;
-    const A dwdy = (wxi * xy + wet * ey + wze * zy) * Jac;
-    const A dwdz = (wxi * xz + wet * ez + wze * zz) * Jac;
-    const A dTdx = (Txi * xx + Tet * ex + Tze * zx) * Jac;
-    const A dTdy = (Txi * xy + Tet * ey + Tze * zy) * Jac;
-    const A dTdz = (Txi * xz + Tet * ez + Tze * zz) * Jac;
+    A dudx, dudy, dudz, dvdx, dvdy, dvdz, dwdx, dwdy, dwdz, dTdx, dTdy, dTdz;
+    if constexpr (sizeof(R) == 8) {
+        const A j = Jac * c1;
+        const A ax = xx * j, ay = xy * j, az = xz * j, bx = ex * j, by = ey * j, bz = ez * j, gx = zx * j, gy = zy * j,
+                gz = zz * j;
+        dudx = uxi * ax + uet * bx + uze * gx; dudy = uxi * ay + uet * by + uze * gy; dudz = uxi * az + uet * bz + uze * gz;
+        dvdx = vxi * ax + vet * bx + vze * gx; dvdy = vxi * ay + vet * by + vze * gy; dvdz = vxi * az + vet * bz + vze * gz;
+        dwdx = wxi * ax + wet * bx + wze * gx; dwdy = wxi * ay + wet * by + wze * gy; dwdz = wxi * az + wet * bz + wze * gz;
+        dTdx = Txi * ax + Tet * bx + Tze * gx; dTdy = Txi * ay + Tet * by + Tze * gy; dTdz = Txi * az + Tet * bz + Tze * gz;
+    } else {
+        dudx = (uxi * xx + uet * ex + uze * zx) * Jac;
+        dudy = (uxi * xy + uet * ey + uze * zy) * Jac;
+        dudz = (uxi * xz + uet * ez + uze * zz) * Jac;
+        dvdx = (vxi * xx + vet * ex + vze * zx) * Jac;
+        dvdy = (vxi * xy + vet * ey + vze * zy) * Jac;
+        dvdz = (vxi * xz + vet * ez + vze * zz) * Jac;
+        dwdx = (wxi * xx + wet * ex + wze * zx) * Jac;
+        dwdy = (wxi * xy + wet * ey + wze * zy) * Jac;
+        dwdz = (wxi * xz + wet * ez + wze * zz) * Jac;
+        dTdx = (Txi * xx + Tet * ex + Tze * zx) * Jac;
+        dTdy = (Txi * xy + Tet * ey + Tze * zy) * Jac;
+        dTdz = (Txi * xz + Tet * ez + Tze * zz) * Jac;
+    }
     const A dv = dudx + dvdy + dwdz;
     if (P.les) {  // viscous.jl:66-106: eddy viscosity and conductivity, Pr_t = 0.9
         const A rho = arith(Q[c]);
