@@ -242,6 +242,7 @@ struct f3d_ctx {
     void* adj_slab = nullptr;
     double *Qb = nullptr, *Lt = nullptr, *U1 = nullptr, *U2 = nullptr, *Xb = nullptr, *Yb = nullptr;
     double *Qst[3] = {}, *cst_[3] = {}, *phst[3] = {};  // Q, sound speed and sensor of the stage states
+    double* Sb = nullptr;  // split-flux cotangents of the listed WENO faces (10 planes, zero between calls)
     double *Fvb[3] = {}, *gb = nullptr;
     // metric and Jacobian cotangents (borrowed; f3d_set_metrics_cotangent) and the forward
     // RHS of the first two stage states kept for the Jacobian's term (10 arrays, owned)
@@ -544,6 +545,10 @@ int adjoint_supported(f3d_ctx* ctx) {
     return F3D_OK;
 }
 
+// Planes of the split-flux cotangents of listed WENO faces: of the three directions at once (one
+// launch a stage), or, on grids above 2^23 cells, of one after the other to save memory
+size_t sb_planes(const f3d_ctx* ctx) { return ctx->dp.plane <= (1ll << 23) ? 30 : 10; }
+
 int adjoint_alloc(f3d_ctx* ctx) {
     if (ctx->adj_slab) return F3D_OK;
     const size_t nc = (size_t)ctx->dp.plane;
@@ -552,10 +557,11 @@ int adjoint_alloc(f3d_ctx* ctx) {
     const size_t b1 = up(nc * 8);
     const size_t bv = up(nv * 8);
     const int ncache = ctx->params.adjoint_lean ? 1 : 3;
-    size_t total = b1 * (6 + 5 * 5 + 8 * ncache) + (ctx->params.viscous ? bv * (12 + 12) : 0);
+    size_t total = b1 * (6 + 5 * 5 + 8 * ncache) + (ctx->weno.list ? up(sb_planes(ctx) * nc * 8) : 0) + (ctx->params.viscous ? bv * (12 + 12) : 0);
     cudaError_t e = cudaMalloc(&ctx->adj_slab, total);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc (adjoint scratch)");
     char* q = (char*)ctx->adj_slab;
+    if (ctx->weno.list) { ctx->Sb = (double*)q; q += up(sb_planes(ctx) * nc * 8); }
     ctx->Qb = (double*)q; q += 6 * b1;
     ctx->Lt = (double*)q; q += 5 * b1;
     ctx->U1 = (double*)q; q += 5 * b1;
@@ -617,6 +623,30 @@ int rhs_vjp_prepared(f3d_ctx* ctx, const double* U, const double* Q, const doubl
     const DevParams& P = ctx->dp;
     const bool hybrid = P.fixed_branch < 0;
     F3D_CUDA(ctx, cudaMemsetAsync(ctx->Qb, 0, (size_t)P.plane * 6 * sizeof(double), st));
+    // the WENO faces from their lists, unless metric cotangents are wanted (formed in the tiles)
+    const bool listed = ctx->Sb && !mbar;
+    WenoVjpArgs w;
+    const bool at_once = sb_planes(ctx) == 30;
+    if (listed) {
+        w.P = P;
+        w.w = ctx->weno;
+        w.Q = Q;
+        w.csnd = csnd;
+        w.J = ctx->J;
+        w.Lb = Lb;
+        for (int n = 0; n < 9; n++) {
+            w.A[n] = ctx->m[n];
+            w.H[n] = ctx->Ah[n];
+        }
+        for (int d = 0; d < 3; d++) w.S[d] = ctx->S[d];
+        w.Qb = ctx->Qb;
+        w.Sb = ctx->Sb;
+        w.any = ctx->weno.count + 8;
+        w.d0 = 0;
+        w.d1 = 3;
+        F3D_CUDA(ctx, launch_weno_list(P, ctx->weno, phi, st));
+        if (at_once) F3D_CUDA(ctx, launch_weno_vjp(w, ctx->sms, st));
+    }
     for (int d = 0; d < 3; d++) {
         AdjArgs a;
         std::memset(&a, 0, sizeof(a));
@@ -635,6 +665,15 @@ int rhs_vjp_prepared(f3d_ctx* ctx, const double* U, const double* Q, const doubl
         if (mbar) {
             for (int n = 0; n < 3; n++) a.mb[n] = ctx->mbar[3 * d + n];
             a.mscale = alpha;
+        }
+        if (listed) {
+            a.Sb = ctx->Sb + (at_once ? 10 * d * P.plane : 0);
+            a.any = w.any + d;
+            if (!at_once) {
+                w.d0 = d;
+                w.d1 = d + 1;
+                F3D_CUDA(ctx, launch_weno_vjp(w, ctx->sms, st));
+            }
         }
         F3D_CUDA(ctx, launch_sweep_vjp(d, a, st));
     }

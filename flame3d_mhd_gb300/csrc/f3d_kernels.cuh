@@ -55,6 +55,7 @@ struct WenoArgs {
     const double* H[9];
     const double* S[3];
 };
+cudaError_t launch_weno_list(const DevParams& P, const WenoList& w, const double* phi, cudaStream_t st);
 cudaError_t launch_weno(const WenoArgs& a, const double* phi, int sms, cudaStream_t st);
 
 // Arguments of one sweep. The field pointers are typed by the sweep's arithmetic: double
@@ -113,9 +114,27 @@ struct AdjArgs {
     const double* J;
     const double* Lb;     // cotangent of the RHS (U layout, interior cells)
     double* Qb;           // accumulated cotangent of Q (6 x Nt^3)
+    double* Sb;           // listed WENO faces: cotangents of Fp, Fm (10 planes, k_weno_vjp.cu), else null
+    const unsigned* any;  //   and whether this direction has any
     double* mb[3];        // optional: accumulated cotangent of this direction's metric row
     double mscale;        //   (scaled by mscale, the VJP's alpha)
 };
+
+// Reverse of the listed WENO faces of directions d0 .. d1-1 into the split-flux cotangents Sb (ten
+// planes a direction) and Qb; any[d] receives whether direction d has listed faces
+struct WenoVjpArgs {
+    DevParams P;
+    WenoList w;
+    const double *Q, *csnd, *J, *Lb;
+    const double* A[9];
+    const double* H[9];
+    const double* S[3];
+    double *Qb, *Sb;
+    unsigned* any;
+    int d0, d1;
+};
+cudaError_t weno_vjp_configure();
+cudaError_t launch_weno_vjp(const WenoVjpArgs& a, int sms, cudaStream_t st);
 
 cudaError_t adjoint_configure();
 cudaError_t launch_sweep_vjp(int dir, const AdjArgs& a, cudaStream_t st);

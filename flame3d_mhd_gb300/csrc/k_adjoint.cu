@@ -246,6 +246,7 @@ __global__ void __launch_bounds__(VTile<DIR, CHAR>::NT, VTile<DIR, CHAR>::MINB) 
             }
             br = m < P.phib[0] ? 0 : (m < P.phib[1] ? 1 : (m < P.phib[2] ? 2 : 3));
             if (br == 1 || br == 2) {
+                if (a.Sb) continue;  // reversed from its list
                 const int k = atomicAdd(&counts[br - 1], 1);
                 (br == 1 ? list7 : list5)[k] = it;
                 continue;
@@ -294,6 +295,7 @@ __global__ void __launch_bounds__(VTile<DIR, CHAR>::NT, VTile<DIR, CHAR>::MINB) 
     }
 
     // Phase C: reverse of the split at every position, into Qb
+    const bool shared = a.Sb && *a.any != 0u;
     for (int it = threadIdx.x; it < TL * NP; it += NT) {
         int l, p;
         if (DIR == 0) { l = it / NP; p = it - l * NP; } else { p = it / TL; l = it - p * TL; }
@@ -301,10 +303,20 @@ __global__ void __launch_bounds__(VTile<DIR, CHAR>::NT, VTile<DIR, CHAR>::MINB) 
         const int s = sidx(l, p);
         F64 fpb[5], fmb[5];
         bool any = false;
+        // the tile that takes a position's global cotangents: its own cells, and the ghost cells at
+        // the line's ends
+        const bool owned = (p >= NG || c0 == 0) && (p < nc + NG || last_tile);
         for (int n = 0; n < 5; n++) {
             const int o = n * TL * NP + s;
             fpb[n] = f64(sFpb[o]);
             fmb[n] = f64(sFmb[o]);
+            if (shared && owned) {  // the listed faces' share, cleared for the next use
+                double* sp = a.Sb + cell(l, c0 + p) + n * pl;
+                double* sn = sp + 5 * pl;
+                const double x = *sp, y = *sn;
+                if (__double_as_longlong(x) << 1) { fpb[n] += f64(x); *sp = 0.0; }
+                if (__double_as_longlong(y) << 1) { fmb[n] += f64(y); *sn = 0.0; }
+            }
             if (!P.lin_int) {  // the linear faces' transpose in FP64
                 const double* G = sG + n * TL * NFV;
 #pragma unroll
@@ -359,6 +371,7 @@ __global__ void __launch_bounds__(VTile<DIR, CHAR>::NT, VTile<DIR, CHAR>::MINB) 
 // J_c [k1 (F[c-2] - F[c+2]) + k2 (F[c-1] - F[c+1])] to momentum/energy (div.jl:14-48).
 __global__ void k_visc_fvb(const DevParams P, const double* __restrict__ Lb, const double* __restrict__ J,
                            double* Fvbx, double* Fvby, double* Fvbz) {
+    after_previous();
     const int vxt = P.nxt - 4, vyt = P.nyt - 4, vzt = P.nzt - 4;
     const long long vpl = (long long)vxt * vyt * vzt;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -401,6 +414,7 @@ __global__ void k_visc_vjp(const DevParams P, const double* __restrict__ Q, cons
                            const double* m2, const double* m3, const double* m4, const double* m5, const double* m6,
                            const double* m7, const double* m8, const double* __restrict__ J, const double* Fvbx,
                            const double* Fvby, const double* Fvbz, double* gb, double* Qb, MetricBar mbar) {
+    after_previous();
     const int vxt = P.nxt - 4, vyt = P.nyt - 4, vzt = P.nzt - 4;
     const long long vpl = (long long)vxt * vyt * vzt;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -539,6 +553,7 @@ __global__ void k_jbar(const DevParams P, const double* __restrict__ Lb, const d
 // Transpose of 12 times the CD4 gradients: G[c'] = c1 (f[c'-2] - f[c'+2]) + c2 (f[c'-1] - f[c'+1]), c1 = 1, c2 = -8,
 // gathered at every cell c from the box cells c' = c -+ 1, 2 that used it.
 __global__ void k_visc_gather(const DevParams P, const double* __restrict__ gb, double* Qb) {
+    after_previous();
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= P.plane) return;
     int i, j, k;
@@ -581,6 +596,7 @@ __global__ void k_visc_gather(const DevParams P, const double* __restrict__ gb, 
 // Inflow-profile cotangents (when a buffer is set) receive pscale times theirs: the RHS VJP
 // scales its state cotangent by alpha after c2Prim, and the profile enters before it.
 __global__ void k_fill_vjp(const DevParams P, const double* __restrict__ Q, double* Qb, double pscale) {
+    after_previous();
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= P.plane) return;
     int i, j, k;
@@ -627,6 +643,7 @@ __global__ void k_fill_vjp(const DevParams P, const double* __restrict__ Q, doub
 
 __global__ void k_c2prim_vjp(const DevParams P, const double* __restrict__ U, const double* __restrict__ Qb,
                              double* out, double alpha, double beta) {
+    after_previous();
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= P.plane) return;
     int i, j, k;
@@ -645,6 +662,7 @@ __global__ void k_c2prim_vjp(const DevParams P, const double* __restrict__ U, co
 
 // out = a x + b y over interior cells of U-layout arrays (RK3 adjoint combinations)
 __global__ void k_axpby(const DevParams P, double* out, const double* x, double a, const double* y, double b) {
+    after_previous();
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= P.plane) return;
     int i, j, k;
@@ -679,11 +697,14 @@ cudaError_t adjoint_configure() {
         (e = configure_vjp<2, false>()) != cudaSuccess || (e = configure_vjp<0, true>()) != cudaSuccess ||
         (e = configure_vjp<1, true>()) != cudaSuccess)
         return e;
-    return configure_vjp<2, true>();
+    if ((e = configure_vjp<2, true>()) != cudaSuccess) return e;
+    return weno_vjp_configure();
 }
 
+// With listed WENO faces the tiles hold linear and NND2 faces alone: the component-wise instance
+// serves both reconstructions (137 registers, three blocks of 96 threads per SM, against 234)
 cudaError_t launch_sweep_vjp(int dir, const AdjArgs& a, cudaStream_t st) {
-    const bool ch = a.P.character != 0;
+    const bool ch = a.P.character != 0 && !a.Sb;
     if (dir == 0) return ch ? launch_vjp_dir<0, true>(a, st) : launch_vjp_dir<0, false>(a, st);
     if (dir == 1) return ch ? launch_vjp_dir<1, true>(a, st) : launch_vjp_dir<1, false>(a, st);
     return ch ? launch_vjp_dir<2, true>(a, st) : launch_vjp_dir<2, false>(a, st);
@@ -699,10 +720,10 @@ cudaError_t launch_viscous_vjp(const DevParams& P, const double* Q, const double
     for (int n = 0; n < 9; n++) mb.m[n] = mbar ? mbar[n] : nullptr;
     mb.J = Jbar;
     mb.scale = mscale;
-    k_visc_fvb<<<blocks_for(nv, 256), 256, 0, st>>>(P, Lb, J, Fvb[0], Fvb[1], Fvb[2]);
-    k_visc_vjp<<<blocks_for(nv, 128), 128, 0, st>>>(P, Q, m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[7], m[8], J,
+    launch_after(P, k_visc_fvb, blocks_for(nv, 256), 256, st, P, Lb, J, Fvb[0], Fvb[1], Fvb[2]);
+    launch_after(P, k_visc_vjp, blocks_for(nv, 128), 128, st, P, Q, m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[7], m[8], J,
                                                      Fvb[0], Fvb[1], Fvb[2], gb, Qb, mb);
-    k_visc_gather<<<blocks_for(P.plane, 256), 256, 0, st>>>(P, gb, Qb);
+    launch_after(P, k_visc_gather, blocks_for(P.plane, 256), 256, st, P, gb, Qb);
     return cudaGetLastError();
 }
 
@@ -713,19 +734,19 @@ cudaError_t launch_jbar(const DevParams& P, const double* Lb, const double* L, c
 }
 
 cudaError_t launch_fill_vjp(const DevParams& P, const double* Q, double* Qb, double pscale, cudaStream_t st) {
-    k_fill_vjp<<<blocks_for(P.plane, 256), 256, 0, st>>>(P, Q, Qb, pscale);
+    launch_after(P, k_fill_vjp, blocks_for(P.plane, 256), 256, st, P, Q, Qb, pscale);
     return cudaGetLastError();
 }
 
 cudaError_t launch_c2prim_vjp(const DevParams& P, const double* U, const double* Qb, double* out, double alpha,
                               double beta, cudaStream_t st) {
-    k_c2prim_vjp<<<blocks_for(P.plane, 256), 256, 0, st>>>(P, U, Qb, out, alpha, beta);
+    launch_after(P, k_c2prim_vjp, blocks_for(P.plane, 256), 256, st, P, U, Qb, out, alpha, beta);
     return cudaGetLastError();
 }
 
 cudaError_t launch_axpby(const DevParams& P, double* out, const double* x, double a, const double* y, double b,
                          cudaStream_t st) {
-    k_axpby<<<blocks_for(P.plane, 256), 256, 0, st>>>(P, out, x, a, y, b);
+    launch_after(P, k_axpby, blocks_for(P.plane, 256), 256, st, P, out, x, a, y, b);
     return cudaGetLastError();
 }
 

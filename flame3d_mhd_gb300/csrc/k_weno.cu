@@ -154,12 +154,17 @@ __global__ void __launch_bounds__(WF_WARPS * 32, 4) k_weno_faces(const WenoArgs 
     }
 }
 
+cudaError_t launch_weno_list(const DevParams& P, const WenoList& w, const double* phi, cudaStream_t st) {
+    launch_after(P, k_weno_list, cdiv(P.plane, 256), 256, st, P, phi, w);
+    return cudaGetLastError();
+}
+
 // Four blocks of k_weno_faces per SM stay resident and share the lists out among themselves; a grid
 // too small to fill them gets one block per 32 of its cells.
 cudaError_t launch_weno(const WenoArgs& a, const double* phi, int sms, cudaStream_t st) {
     const long long most = (long long)a.P.nx * a.P.ny * a.P.nz / WF_FACES + 1;
     const int blocks = most < 4 * sms ? (int)most : 4 * sms;
-    launch_after(a.P, k_weno_list, cdiv(a.P.plane, 256), 256, st, a.P, phi, a.w);
+    launch_weno_list(a.P, a.w, phi, st);
     if (a.P.character) k_weno_faces<true><<<blocks, WF_WARPS * 32, 0, st>>>(a);
     else k_weno_faces<false><<<blocks, WF_WARPS * 32, 0, st>>>(a);
     return cudaGetLastError();

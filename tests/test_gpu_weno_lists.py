@@ -52,3 +52,51 @@ def test_rhs_equals_differences_of_tile_faces(gpu_lib, n, which, character, spli
         tol = 2048 * EPS * scale.max(0)
         assert (np.abs(got - want).max(0) <= tol).all(), float((np.abs(got - want).max(0) / tol).max())
     s.close()
+
+
+@pytest.mark.parametrize("n", [(4, 4, 4), (33, 5, 9), (70, 9, 31), (520, 130, 120)])
+@pytest.mark.parametrize("which", ["all", "weno7", "weno5", "none"])
+@pytest.mark.parametrize("character,split", [(1, "SW"), (0, "LF")])
+def test_reverse_equals_the_tiles_reverse(gpu_lib, n, which, character, split):
+    """The RHS VJP, whose WENO faces are reversed from their lists (k_weno_vjp.cu), against the same
+    call with metric cotangents requested, which reverses them within the tiles. The largest grid is
+    above the size up to which the three directions are taken at once."""
+    import torch
+
+    from flame3d_mhd_gb300.solver import Flame3D
+    nx, ny, nz = n
+    if nx > 500 and (which != "all" or not character):
+        pytest.skip("one case of the largest grid is enough")
+    per = dict(kind=abi.BC_PERIODIC)
+    p1, p2, p3 = THRESHOLDS[which]
+    s = Flame3D(abi.make_params(nx, ny, nz, phi1=p1, phi2=p2, phi3=p3, viscous=0, character=character, split=split,
+                                bc=[per] * 6))
+    shape = (nz + 8, ny + 8, nx + 8)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    uni = lambda *sh: torch.rand(sh, generator=g, dtype=torch.float64, device="cuda")  # noqa: E731
+    eye = [1.0, 0.0, 0.0, 0.0, 1.0, 0.0, 0.0, 0.0, 1.0]
+    # periodic inputs: the metrics are smooth functions of the cell indices
+    z, y, x = torch.meshgrid(*[torch.arange(m, dtype=torch.float64, device="cuda") - 4 for m in shape], indexing="ij")
+    w = [torch.sin(2 * np.pi * (x / nx + k * y / ny + z / nz)) for k in range(1, 10)]
+    s.set_metrics([e + 0.1 * v for e, v in zip(eye, w)], torch.ones(shape, dtype=torch.float64, device="cuda"))
+    Q = torch.empty((6, *shape), dtype=torch.float64, device="cuda")
+    Q[0] = 0.7 + 0.6 * uni(*shape)
+    Q[1:4] = 1.2 * uni(3, *shape) - 0.6
+    Q[4] = (0.3 + 1.2 * uni(*shape)) ** 2
+    Q[5] = Q[4] / (Q[0] * 287.0)
+    U = s.field(5)
+    s.prim2c(U, Q)
+    s.fillGhost(Q, U)
+    Lbar = s.field(5)
+    Lbar[:, 4:-4, 4:-4, 4:-4] = 2.0 * uni(5, nz, ny, nx) - 1.0
+    runs = [s.rhs_vjp(U, Lbar).clone() for _ in range(2)]  # the second finds the planes cleared
+    bars = [s.field(1) for _ in range(10)]
+    s.set_metrics_cotangent(bars[:9], bars[9])
+    want = s.rhs_vjp(U, Lbar)
+    # both are sums of the same ~1e4 rounded products in another order: the derivative of a WENO face
+    # is formed with relative error ~1e3 eps of its largest terms, which are O(1/(1 - w)) of the result
+    scale = want.abs().max()
+    for got in runs:
+        assert torch.isfinite(got).all()
+        assert (got - want).abs().max() <= 1e-11 * scale, float((got - want).abs().max() / scale)
+    s.close()
