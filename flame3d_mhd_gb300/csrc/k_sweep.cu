@@ -21,18 +21,24 @@
 namespace f3d {
 
 // Tile (lines TL x cells TC), threads and resident blocks per SM of a sweep, by type.
-// FP64: 4 x 64 in every direction on 160 threads, four blocks per SM (~38 KB of shared memory
-// each, 96 registers a thread): 20 warps an SM hide each other's loads, barriers and FP64
-// latencies better than two blocks of nine warps on 8 x 64 tiles, at the same halo. Measured on
-// one box (RK3 step): shock tube 256x64x64 3.03 -> 2.91 ms, ramp 512x256x128 61.1 -> 58.7 ms,
-// plate 125x61x37 1.67 -> 1.55 ms. 32-cell tiles split a quarter of their cells twice (tube 3.2
-// ms, ramp 63.6 ms); 128 threads x 5 blocks and 192 x 3 on this tile: 3.04 / 3.22 ms.
+// FP64: 4 x 64 in every direction on 288 threads (~38 KB of shared memory a block): Phase B's
+// 260 faces and Phase A's 288 split cells are one pass of the block, so that no warp waits for
+// others' second pass. Four blocks per SM where the tiles hold no WENO code (WENO_LISTED, 56
+// registers, 36 warps an SM hide the loads, barriers and FP64 latencies), three where they do
+// (72 registers). Measured on one box (RK3 step; 160 threads x 4 blocks with WENO code -> 288 x 4
+// without): shock tube 256x64x64 5.38 -> 4.56 ms, ramp 512x256x128 49.8 -> 45.5 ms, plate
+// 125x61x37 1.29 -> 1.18 ms, RHS of a 16^3 vortex 50.9 -> 43.7 us. Without WENO code 288 x 3 takes
+// 4.82 / 47.5 / 1.23 ms, 288 x 2 5.69 / 54.5 / 1.37, 288 x 5 (45 registers) 5.07 / 48.7 / 1.27,
+// 320 x 4 4.77 / 46.9 / 1.22, 192 x 6 5.19 / 48.7 / 1.23, 160 x 5 4.87 / 46.5 / 1.21. With it (the WENO5 vortex 64^3):
+// 160 x 4 4.74 -> 288 x 3 4.64 ms, 320 x 3 4.67, 192 x 5 4.82. Tiles of eight lines or of
+// 32 cells lose more on the smaller grids than the ramp gains.
 // FP32: half-height tiles on 128 threads, six blocks per SM (~20 KB each): the same step time as
 // three 256-thread blocks on that tube, 6% less per RHS on the component-wise tube and on
 // the viscous vortex.
 #ifndef SW_D_THREADS
-#define SW_D_THREADS 160
-#define SW_D_BLOCKS 4
+#define SW_D_THREADS 288
+#define SW_D_BLOCKS 3
+#define SW_D_LISTED_BLOCKS 4
 #define SW_D_TL0 4
 #define SW_D_TL12 4
 #endif
@@ -40,19 +46,29 @@ namespace f3d {
 #define SW_D_TC0 64
 #define SW_D_TC12 64
 #endif
-template <int DIR, class R> struct Tile;
+enum { WENO_COMP, WENO_CHAR, WENO_LISTED };  // WENO faces: component-, characteristic-wise, from k_weno.cu
+template <int DIR, class R, int FACES = WENO_COMP> struct Tile;
 #ifndef SW_F_THREADS
 #define SW_F_THREADS 128
 #define SW_F_BLOCKS 6
 #define SW_F_TL0 4
 #define SW_F_TL12 8
 #endif
-template <> struct Tile<0, float> { static constexpr int TL = SW_F_TL0, TC = 64, NT = SW_F_THREADS, MINB = SW_F_BLOCKS; };
-template <> struct Tile<1, float> { static constexpr int TL = SW_F_TL12, TC = 32, NT = SW_F_THREADS, MINB = SW_F_BLOCKS; };
-template <> struct Tile<2, float> { static constexpr int TL = SW_F_TL12, TC = 32, NT = SW_F_THREADS, MINB = SW_F_BLOCKS; };
-template <> struct Tile<0, double> { static constexpr int TL = SW_D_TL0, TC = SW_D_TC0, NT = SW_D_THREADS, MINB = SW_D_BLOCKS; };
-template <> struct Tile<1, double> { static constexpr int TL = SW_D_TL12, TC = SW_D_TC12, NT = SW_D_THREADS, MINB = SW_D_BLOCKS; };
-template <> struct Tile<2, double> { static constexpr int TL = SW_D_TL12, TC = SW_D_TC12, NT = SW_D_THREADS, MINB = SW_D_BLOCKS; };
+template <int FACES> struct Tile<0, float, FACES> { static constexpr int TL = SW_F_TL0, TC = 64, NT = SW_F_THREADS, MINB = SW_F_BLOCKS; };
+template <int FACES> struct Tile<1, float, FACES> { static constexpr int TL = SW_F_TL12, TC = 32, NT = SW_F_THREADS, MINB = SW_F_BLOCKS; };
+template <int FACES> struct Tile<2, float, FACES> { static constexpr int TL = SW_F_TL12, TC = 32, NT = SW_F_THREADS, MINB = SW_F_BLOCKS; };
+template <int FACES> struct Tile<0, double, FACES> {
+    static constexpr int TL = SW_D_TL0, TC = SW_D_TC0, NT = SW_D_THREADS,
+                         MINB = FACES == WENO_LISTED ? SW_D_LISTED_BLOCKS : SW_D_BLOCKS;
+};
+template <int FACES> struct Tile<1, double, FACES> {
+    static constexpr int TL = SW_D_TL12, TC = SW_D_TC12, NT = SW_D_THREADS,
+                         MINB = FACES == WENO_LISTED ? SW_D_LISTED_BLOCKS : SW_D_BLOCKS;
+};
+template <int FACES> struct Tile<2, double, FACES> {
+    static constexpr int TL = SW_D_TL12, TC = SW_D_TC12, NT = SW_D_THREADS,
+                         MINB = FACES == WENO_LISTED ? SW_D_LISTED_BLOCKS : SW_D_BLOCKS;
+};
 
 template <int DIR, class R> constexpr size_t sweep_smem_bytes(bool hybrid) {
     using T = Tile<DIR, R>;
@@ -61,10 +77,10 @@ template <int DIR, class R> constexpr size_t sweep_smem_bytes(bool hybrid) {
            (sizeof(R) == 8 ? (((size_t)T::TL * (T::TC + 1) + 7) & ~(size_t)7) : 0);  // faces of the linear strips
 }
 
-template <int DIR, bool CHAR, class R>
-__global__ void __launch_bounds__(Tile<DIR, R>::NT, Tile<DIR, R>::MINB) k_sweep(const SweepArgs a) {
+template <int DIR, int FACES, class R>
+__global__ void __launch_bounds__(Tile<DIR, R, FACES>::NT, Tile<DIR, R, FACES>::MINB) k_sweep(const SweepArgs a) {
     constexpr int TL = Tile<DIR, R>::TL, TC = Tile<DIR, R>::TC, NP = TC + 8, NF = TC + 1;
-    constexpr int SWEEP_THREADS = Tile<DIR, R>::NT;
+    constexpr int SWEEP_THREADS = Tile<DIR, R, FACES>::NT;
     using A = typename Arith<R>::type;
     const DevParams& P = a.P;
     const bool hybrid = P.fixed_branch < 0;
@@ -133,10 +149,10 @@ __global__ void __launch_bounds__(Tile<DIR, R>::NT, Tile<DIR, R>::MINB) k_sweep(
         const long long cl = cell(l, c0 + t + 3), cr = cl + stride;
         A out[5];
         A s0 = A(0);
-        if (br == 1 || br == 2) s0 = A(2) / (arith(Sr[cl]) + arith(Sr[cr]));
+        if (FACES != WENO_LISTED && (br == 1 || br == 2)) s0 = A(2) / (arith(Sr[cl]) + arith(Sr[cr]));
         auto FP = [&](int n, int p) { return arith(sFp[n * TL * NP + sidx(l, p)]); };
         auto FM = [&](int n, int p) { return arith(sFm[n * TL * NP + sidx(l, p)]); };
-        face_flux<CHAR, A>(P, a, br, t, s0, cl, cr, FP, FM, out);
+        face_flux<FACES == WENO_CHAR, A>(P, a, br, t, s0, cl, cr, FP, FM, out);
         const int f = fidx(l, t);
 #pragma unroll
         for (int n = 0; n < 5; n++) sF[n * TL * NF + f] = plain(out[n]);
@@ -161,14 +177,14 @@ __global__ void __launch_bounds__(Tile<DIR, R>::NT, Tile<DIR, R>::MINB) k_sweep(
             for (int o = 0; o < 6; o++) ph[o] = sPhi[sidx(l, t + 1 + o)];
             br = branch_of(P, ph);
             if (br == 1 || br == 2) {
-                if (sizeof(R) == 8 && a.wflux) {  // its flux is known (k_weno.cu)
+                if constexpr (FACES == WENO_LISTED) {  // its flux is known (k_weno.cu)
                     const double* w = a.wflux + cell(l, c0 + t + 3);
 #pragma unroll
                     for (int n = 0; n < 5; n++) sF[n * TL * NF + fidx(l, t)] = (R)w[n * pl];
-                    continue;
+                } else {
+                    const int k = atomicAdd(&counts[br - 1], 1);
+                    (br == 1 ? list7 : list5)[k] = it;
                 }
-                const int k = atomicAdd(&counts[br - 1], 1);
-                (br == 1 ? list7 : list5)[k] = it;
                 continue;
             }
         }
@@ -176,7 +192,7 @@ __global__ void __launch_bounds__(Tile<DIR, R>::NT, Tile<DIR, R>::MINB) k_sweep(
             sLin[it] = 1;
             continue;
         }
-        do_face(l, t, br);
+        do_face(l, t, FACES == WENO_LISTED && br != 0 ? 3 : br);
     }
     if (hybrid || strips) {
         __syncthreads();
@@ -199,7 +215,7 @@ __global__ void __launch_bounds__(Tile<DIR, R>::NT, Tile<DIR, R>::MINB) k_sweep(
                 if (lane == 0) ch = atomicAdd(&counts[2], 1);
                 ch = __shfl_sync(0xffffffffu, ch, 0);
                 if (ch >= ch7 + ch5 + chs) break;
-                if (ch < ch7 + ch5) {
+                if (FACES != WENO_LISTED && ch < ch7 + ch5) {
                     const bool w7 = ch < ch7;
                     const int k = (w7 ? ch : ch - ch7) * 32 + lane;
                     if (k < (w7 ? n7 : n5)) {
@@ -254,29 +270,29 @@ __global__ void __launch_bounds__(Tile<DIR, R>::NT, Tile<DIR, R>::MINB) k_sweep(
     sweep_epilogue<DIR, TL, TC, SWEEP_THREADS, R>(a, sF, c0, l0, other, nc, nl, cell, fidx);
 }
 
-template <int DIR, bool CHAR, class R> static cudaError_t configure_dir() {
-    return cudaFuncSetAttribute(k_sweep<DIR, CHAR, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+template <int DIR, int FACES, class R> static cudaError_t configure_dir() {
+    return cudaFuncSetAttribute(k_sweep<DIR, FACES, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)sweep_smem_bytes<DIR, R>(true));
 }
 
-template <class R> static cudaError_t configure_type() {
-    cudaError_t e;
-    if ((e = configure_dir<0, false, R>()) != cudaSuccess) return e;
-    if ((e = configure_dir<0, true, R>()) != cudaSuccess) return e;
-    if ((e = configure_dir<1, false, R>()) != cudaSuccess) return e;
-    if ((e = configure_dir<1, true, R>()) != cudaSuccess) return e;
-    if ((e = configure_dir<2, false, R>()) != cudaSuccess) return e;
-    return configure_dir<2, true, R>();
+template <int FACES, class R> static cudaError_t configure_faces() {
+    cudaError_t e = configure_dir<0, FACES, R>();
+    if (e == cudaSuccess) e = configure_dir<1, FACES, R>();
+    return e == cudaSuccess ? configure_dir<2, FACES, R>() : e;
 }
 
 // Dynamic shared memory above 48 KB must be enabled per kernel before the first launch
 // (and outside stream capture): called from f3d_create.
 cudaError_t sweep_configure() {
-    cudaError_t e = configure_type<double>();
-    return e != cudaSuccess ? e : configure_type<float>();
+    cudaError_t e;
+    if ((e = configure_faces<WENO_COMP, double>()) != cudaSuccess) return e;
+    if ((e = configure_faces<WENO_CHAR, double>()) != cudaSuccess) return e;
+    if ((e = configure_faces<WENO_LISTED, double>()) != cudaSuccess) return e;
+    if ((e = configure_faces<WENO_COMP, float>()) != cudaSuccess) return e;
+    return configure_faces<WENO_CHAR, float>();
 }
 
-template <int DIR, bool CHAR, class R> static cudaError_t launch_dir(const SweepArgs& a, cudaStream_t st) {
+template <int DIR, int FACES, class R> static cudaError_t launch_dir(const SweepArgs& a, cudaStream_t st) {
     constexpr int TL = Tile<DIR, R>::TL, TC = Tile<DIR, R>::TC;
     const DevParams& P = a.P;
     const size_t smem = sweep_smem_bytes<DIR, R>(true);
@@ -284,19 +300,23 @@ template <int DIR, bool CHAR, class R> static cudaError_t launch_dir(const Sweep
     if (DIR == 0) grid = dim3(cdiv(P.nx, TC), cdiv(P.ny, TL), P.nz);
     else if (DIR == 1) grid = dim3(cdiv(P.nx, TL), cdiv(P.ny, TC), P.nz);
     else grid = dim3(cdiv(P.nx, TL), cdiv(P.nz, TC), P.ny);
-    k_sweep<DIR, CHAR, R><<<grid, Tile<DIR, R>::NT, smem, st>>>(a);
+    k_sweep<DIR, FACES, R><<<grid, Tile<DIR, R, FACES>::NT, smem, st>>>(a);
     return cudaGetLastError();
 }
 
-template <class R> static cudaError_t launch_typed(int dir, const SweepArgs& a, cudaStream_t st) {
-    const bool ch = a.P.character != 0;
-    if (dir == 0) return ch ? launch_dir<0, true, R>(a, st) : launch_dir<0, false, R>(a, st);
-    if (dir == 1) return ch ? launch_dir<1, true, R>(a, st) : launch_dir<1, false, R>(a, st);
-    return ch ? launch_dir<2, true, R>(a, st) : launch_dir<2, false, R>(a, st);
+template <int FACES, class R> static cudaError_t launch_faces(int dir, const SweepArgs& a, cudaStream_t st) {
+    if (dir == 0) return launch_dir<0, FACES, R>(a, st);
+    return dir == 1 ? launch_dir<1, FACES, R>(a, st) : launch_dir<2, FACES, R>(a, st);
 }
 
+// With the WENO faces listed (the hybrid switch in FP64), or a scheme without any, the sweep holds
+// no WENO code: 56 registers a thread, and one instance for component- and characteristic-wise faces.
 cudaError_t launch_sweep(int dir, const SweepArgs& a, cudaStream_t st) {
-    return a.fp32 ? launch_typed<float>(dir, a, st) : launch_typed<double>(dir, a, st);
+    const bool ch = a.P.character != 0;
+    if (a.fp32) return ch ? launch_faces<WENO_CHAR, float>(dir, a, st) : launch_faces<WENO_COMP, float>(dir, a, st);
+    const int fb = a.P.fixed_branch;
+    if (fb == 0 || fb == 3 || (a.wflux && fb < 0)) return launch_faces<WENO_LISTED, double>(dir, a, st);
+    return ch ? launch_faces<WENO_CHAR, double>(dir, a, st) : launch_faces<WENO_COMP, double>(dir, a, st);
 }
 
 }  // namespace f3d
