@@ -20,16 +20,16 @@
 namespace f3d {
 
 // Tile of TL lines x TC cells; NT threads cover the TL x (TC + 8) stencil positions of
-// phases A and C. About 140 registers a thread (component-wise) and 59.5 KB of shared
-// memory a block for 4-line tiles (the split fluxes, their cotangents, the sensor and the UP7
-// face cotangents gathered in Phase C): three blocks per SM.
-#ifndef V_TL0
-#define V_TL0 4
-#define V_NT0 96
-#define V_MB0 3
-#define V_TL12 4
-#define V_NT12 96
-#define V_MB12 3
+// phases A and C. ~59.5 KB of shared memory a block for 4-line tiles (the split fluxes, their
+// cotangents, the sensor and the linear faces' cotangents): three blocks per SM, ~120 registers a
+// thread on 160 threads. Measured on one box (step VJP): 96 threads x 3 -> 160 x 3: viscous vortex
+// 128^3 18.7 -> 18.0 ms, shock tube 256x64x64 9.14 -> 8.55 ms (192 x 3 18.3 / 8.74, 288 x 2
+// 18.6 / 8.93, 256 x 2 19.5 / 9.70). Tiles without WENO faces (VJP_NONE) split the cells of Phase A
+// only where an NND2 face reads them, since the reverse of a linear face needs no split: 17.8 ->
+// 16.2 and 8.37 -> 7.58 ms (288 x 3 at 72 registers, with spills, 16.2 / 7.50; 192 x 3 16.5 / 7.75).
+#ifndef V_NT
+#define V_NT 160
+#define V_MB 3
 #endif
 // characteristic-wise reverse sweeps: the reverse of a characteristic WENO face holds more
 // state (its eigenvectors, a side's stencil of one field and its cotangents). Smaller blocks
@@ -44,23 +44,24 @@ namespace f3d {
 #define V_C_NT12 96
 #define V_C_MB12 2
 #endif
-template <int DIR, bool CHAR = false> struct VTile;
-template <> struct VTile<0, false> { static constexpr int TL = V_TL0, TC = 64, NT = V_NT0, MINB = V_MB0; };
-template <> struct VTile<1, false> { static constexpr int TL = V_TL12, TC = 64, NT = V_NT12, MINB = V_MB12; };
-template <> struct VTile<2, false> { static constexpr int TL = V_TL12, TC = 64, NT = V_NT12, MINB = V_MB12; };
-template <> struct VTile<0, true> { static constexpr int TL = V_C_TL0, TC = 64, NT = V_C_NT0, MINB = V_C_MB0; };
-template <> struct VTile<1, true> { static constexpr int TL = V_C_TL12, TC = 64, NT = V_C_NT12, MINB = V_C_MB12; };
-template <> struct VTile<2, true> { static constexpr int TL = V_C_TL12, TC = 64, NT = V_C_NT12, MINB = V_C_MB12; };
+enum { VJP_COMP, VJP_CHAR, VJP_NONE };  // the tiles' WENO faces: component-, characteristic-wise, none
+template <int DIR, int FACES> struct VTile {
+    static constexpr int TL = 4, TC = 64, NT = V_NT, MINB = V_MB;
+};
+template <> struct VTile<0, VJP_CHAR> { static constexpr int TL = V_C_TL0, TC = 64, NT = V_C_NT0, MINB = V_C_MB0; };
+template <> struct VTile<1, VJP_CHAR> { static constexpr int TL = V_C_TL12, TC = 64, NT = V_C_NT12, MINB = V_C_MB12; };
+template <> struct VTile<2, VJP_CHAR> { static constexpr int TL = V_C_TL12, TC = 64, NT = V_C_NT12, MINB = V_C_MB12; };
 
-template <int DIR, bool CHAR> constexpr size_t vjp_smem_bytes() {
-    using T = VTile<DIR, CHAR>;
+template <int DIR, int FACES> constexpr size_t vjp_smem_bytes() {
+    using T = VTile<DIR, FACES>;
     return sizeof(double) * ((size_t)T::TL * (T::TC + 8) * 21 + 5 * (size_t)T::TL * (T::TC + 1)) +
            sizeof(int) * (2 * (size_t)T::TL * (T::TC + 1) + 4);
 }
 
-template <int DIR, bool CHAR>
-__global__ void __launch_bounds__(VTile<DIR, CHAR>::NT, VTile<DIR, CHAR>::MINB) k_sweep_vjp(const AdjArgs a) {
-    constexpr int TL = VTile<DIR, CHAR>::TL, TC = VTile<DIR, CHAR>::TC, NP = TC + 8, NT = VTile<DIR, CHAR>::NT;
+template <int DIR, int FACES>
+__global__ void __launch_bounds__(VTile<DIR, FACES>::NT, VTile<DIR, FACES>::MINB) k_sweep_vjp(const AdjArgs a) {
+    constexpr int TL = VTile<DIR, FACES>::TL, TC = VTile<DIR, FACES>::TC, NP = TC + 8, NT = VTile<DIR, FACES>::NT;
+    constexpr bool CHAR = FACES == VJP_CHAR, WENO = FACES != VJP_NONE;
     const DevParams& P = a.P;
     const bool hybrid = P.fixed_branch < 0;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -94,21 +95,22 @@ __global__ void __launch_bounds__(VTile<DIR, CHAR>::NT, VTile<DIR, CHAR>::MINB) 
     auto sidx = [&](int l, int p) { return DIR == 0 ? l * NP + p : p * TL + l; };
     const long long pl = P.plane;
 
-    int* list7 = reinterpret_cast<int*>(sG + 5 * TL * NFV);
-    int* list5 = list7 + TL * (TC + 1);
-    int* counts = list5 + TL * (TC + 1);
-    if (threadIdx.x < 2) counts[threadIdx.x] = 0;
-    for (int it = threadIdx.x; it < 5 * TL * NFV; it += NT) sG[it] = 0.0;
-    // Phase A: forward split at positions 0..nc+7 (full index c0 + p); zero the cotangents
-    for (int it = threadIdx.x; it < TL * NP; it += NT) {
-        int l, p;
+    auto pos_lp = [&](int it, int& l, int& p) {
         if (DIR == 0) { l = it / NP; p = it - l * NP; } else { p = it / TL; l = it - p * TL; }
-        const int s = sidx(l, p);
-        for (int n = 0; n < 5; n++) {
-            sFpb[n * TL * NP + s] = 0.0;
-            sFmb[n * TL * NP + s] = 0.0;
+    };
+    auto face_lt = [&](int it, int& l, int& t) {
+        if (DIR == 0) { l = it / NFV; t = it - l * NFV; } else { t = it / TL; l = it - t * TL; }
+    };
+    auto branch = [&](int l, int t) {
+        unsigned long long m = __double_as_longlong(sPhi[sidx(l, t + 1)]);
+        for (int o = 2; o <= 6; o++) {
+            const unsigned long long b = __double_as_longlong(sPhi[sidx(l, t + o)]);
+            m = b > m ? b : m;
         }
-        if (l >= nl || p >= nc + 8) continue;
+        return m < P.phib[0] ? 0 : (m < P.phib[1] ? 1 : (m < P.phib[2] ? 2 : 3));
+    };
+    auto split = [&](int l, int p) {
+        const int s = sidx(l, p);
         const long long c = cell(l, c0 + p);
         F64 q[6], fp[5], fm[5];
         for (int n = 0; n < 6; n++) q[n] = f64(a.Q[c + n * pl]);
@@ -118,9 +120,46 @@ __global__ void __launch_bounds__(VTile<DIR, CHAR>::NT, VTile<DIR, CHAR>::MINB) 
             sFp[n * TL * NP + s] = fp[n].v;
             sFm[n * TL * NP + s] = fm[n].v;
         }
-        if (hybrid) sPhi[s] = a.phi[c];
+    };
+
+    int* list7 = reinterpret_cast<int*>(sG + 5 * TL * NFV);
+    int* list5 = list7 + TL * (TC + 1);
+    int* counts = list5 + TL * (TC + 1);
+    if (threadIdx.x < 2) counts[threadIdx.x] = 0;
+    for (int it = threadIdx.x; it < 5 * TL * NFV; it += NT) sG[it] = 0.0;
+    // Phase A: forward split at positions 0..nc+7 (full index c0 + p), without WENO faces only in
+    // tiles with an NND2 face; zero the cotangents
+    for (int it = threadIdx.x; it < TL * NP; it += NT) {
+        int l, p;
+        pos_lp(it, l, p);
+        const int s = sidx(l, p);
+        for (int n = 0; n < 5; n++) {
+            sFpb[n * TL * NP + s] = 0.0;
+            sFmb[n * TL * NP + s] = 0.0;
+        }
+        if (l >= nl || p >= nc + 8) continue;
+        if (hybrid) sPhi[s] = a.phi[cell(l, c0 + p)];
+        if (!WENO) continue;
+        split(l, p);
     }
     __syncthreads();
+    if (!WENO) {
+        bool nnd = P.fixed_branch > 0;
+        if (hybrid)
+            for (int it = threadIdx.x; it < TL * NFV; it += NT) {
+                int l, t;
+                face_lt(it, l, t);
+                if (l < nl && t < nfaces) nnd |= branch(l, t) == 3;
+            }
+        if (__syncthreads_or(nnd)) {
+            for (int it = threadIdx.x; it < TL * NP; it += NT) {
+                int l, p;
+                pos_lp(it, l, p);
+                if (l < nl && p < nc + 8) split(l, p);
+            }
+            __syncthreads();
+        }
+    }
 
     // Phase B: owned faces t (interior face c0+t, between positions t+3 and t+4). UP7 and
     // NND2 faces at once; WENO7 / WENO5 faces queued and done by consecutive threads.
@@ -141,7 +180,7 @@ __global__ void __launch_bounds__(VTile<DIR, CHAR>::NT, VTile<DIR, CHAR>::MINB) 
             for (int n = 0; n < 5; n++) sG[n * TL * NFV + gidx(l, t)] = Fb[n];
             return;
         }
-        const double s0 = (br == 1 || br == 2) ? 2.0 / (a.S[cl] + a.S[cr]) : 0.0;
+        const double s0 = WENO && (br == 1 || br == 2) ? 2.0 / (a.S[cl] + a.S[cr]) : 0.0;
         double s0b_ = 0.0;
         double* s0b = a.mb[0] ? &s0b_ : nullptr;  // metric cotangent wanted
         if (CHAR && (br == 1 || br == 2)) {
@@ -180,7 +219,7 @@ __global__ void __launch_bounds__(VTile<DIR, CHAR>::NT, VTile<DIR, CHAR>::MINB) 
             const double* vm = sFm + n * TL * NP;
             auto P_ = [&](int pos) { return vp[sidx(l, pos)]; };
             auto M_ = [&](int pos) { return vm[sidx(l, pos)]; };
-            if (br == 1) {  // WENO7, (fp + fm)/12
+            if (WENO && br == 1) {  // WENO7, (fp + fm)/12
                 double V[7], Vb[7];
                 for (int k = 0; k < 7; k++) V[k] = P_(t + k);
                 weno7_vjp(V, s0, g * (1.0 / 12.0), Vb, s0b);
@@ -188,7 +227,7 @@ __global__ void __launch_bounds__(VTile<DIR, CHAR>::NT, VTile<DIR, CHAR>::MINB) 
                 for (int k = 0; k < 7; k++) V[k] = M_(t + 7 - k);
                 weno7_vjp(V, s0, g * (1.0 / 12.0), Vb, s0b);
                 for (int k = 0; k < 7; k++) atomicAdd(&mb[sidx(l, t + 7 - k)], Vb[k]);
-            } else if (br == 2) {  // WENO5, (fp + fm)/6: Fp at t+1..t+5, Fm at t+6..t+2
+            } else if (WENO && br == 2) {  // WENO5, (fp + fm)/6: Fp at t+1..t+5, Fm at t+6..t+2
                 double V[5], Vb[5];
                 for (int k = 0; k < 5; k++) V[k] = P_(t + 1 + k);
                 weno5_vjp(V, s0, g * (1.0 / 6.0), Vb, s0b);
@@ -223,7 +262,7 @@ __global__ void __launch_bounds__(VTile<DIR, CHAR>::NT, VTile<DIR, CHAR>::MINB) 
                 }
             }
         }
-        if (s0b && s0b_ != 0.0) {
+        if (WENO && s0b && s0b_ != 0.0) {
             // s0 = 2 / (S_l + S_r): both |A| get -s0^2/2 s0-bar, and |A| passes A_j / |A| to A_j
             const double Sb = -0.5 * s0 * s0 * s0b_ * a.mscale;
             const long long cc[2] = {cl, cr};
@@ -235,18 +274,13 @@ __global__ void __launch_bounds__(VTile<DIR, CHAR>::NT, VTile<DIR, CHAR>::MINB) 
     };
     for (int it = threadIdx.x; it < TL * (TC + 1); it += NT) {
         int l, t;
-        if (DIR == 0) { l = it / (TC + 1); t = it - l * (TC + 1); } else { t = it / TL; l = it - t * TL; }
+        face_lt(it, l, t);
         if (l >= nl || t >= nfaces) continue;
         int br = P.fixed_branch;
         if (hybrid) {
-            unsigned long long m = __double_as_longlong(sPhi[sidx(l, t + 1)]);
-            for (int o = 2; o <= 6; o++) {
-                unsigned long long b = __double_as_longlong(sPhi[sidx(l, t + o)]);
-                m = b > m ? b : m;
-            }
-            br = m < P.phib[0] ? 0 : (m < P.phib[1] ? 1 : (m < P.phib[2] ? 2 : 3));
+            br = branch(l, t);
             if (br == 1 || br == 2) {
-                if (a.Sb) continue;  // reversed from its list
+                if (!WENO) continue;  // reversed from its list
                 const int k = atomicAdd(&counts[br - 1], 1);
                 (br == 1 ? list7 : list5)[k] = it;
                 continue;
@@ -254,13 +288,13 @@ __global__ void __launch_bounds__(VTile<DIR, CHAR>::NT, VTile<DIR, CHAR>::MINB) 
         }
         face_vjp(l, t, br);
     }
-    if (hybrid) {
+    if (WENO && hybrid) {
         __syncthreads();
         const int n7 = counts[0], n5 = counts[1];
         for (int k = threadIdx.x; k < n7 + n5; k += NT) {
             const int it = k < n7 ? list7[k] : list5[k - n7];
             int l, t;
-            if (DIR == 0) { l = it / (TC + 1); t = it - l * (TC + 1); } else { t = it / TL; l = it - t * TL; }
+            face_lt(it, l, t);
             face_vjp(l, t, k < n7 ? 1 : 2);
         }
     }
@@ -298,7 +332,7 @@ __global__ void __launch_bounds__(VTile<DIR, CHAR>::NT, VTile<DIR, CHAR>::MINB) 
     const bool shared = a.Sb && *a.any != 0u;
     for (int it = threadIdx.x; it < TL * NP; it += NT) {
         int l, p;
-        if (DIR == 0) { l = it / NP; p = it - l * NP; } else { p = it / TL; l = it - p * TL; }
+        pos_lp(it, l, p);
         if (l >= nl || p >= nc + 8) continue;
         const int s = sidx(l, p);
         F64 fpb[5], fmb[5];
@@ -675,39 +709,45 @@ __global__ void k_axpby(const DevParams P, double* out, const double* x, double 
 }
 
 // ---- launchers --------------------------------------------------------------------------
-template <int DIR, bool CHAR> static cudaError_t launch_vjp_dir(const AdjArgs& a, cudaStream_t st) {
-    constexpr int TL = VTile<DIR, CHAR>::TL, TC = VTile<DIR, CHAR>::TC;
+template <int DIR, int FACES> static cudaError_t launch_vjp_dir(const AdjArgs& a, cudaStream_t st) {
+    constexpr int TL = VTile<DIR, FACES>::TL, TC = VTile<DIR, FACES>::TC;
     const DevParams& P = a.P;
     dim3 grid;
     if (DIR == 0) grid = dim3(cdiv(P.nx, TC), cdiv(P.ny, TL), P.nz);
     else if (DIR == 1) grid = dim3(cdiv(P.nx, TL), cdiv(P.ny, TC), P.nz);
     else grid = dim3(cdiv(P.nx, TL), cdiv(P.nz, TC), P.ny);
-    k_sweep_vjp<DIR, CHAR><<<grid, VTile<DIR, CHAR>::NT, vjp_smem_bytes<DIR, CHAR>(), st>>>(a);
+    k_sweep_vjp<DIR, FACES><<<grid, VTile<DIR, FACES>::NT, vjp_smem_bytes<DIR, FACES>(), st>>>(a);
     return cudaGetLastError();
 }
 
-template <int DIR, bool CHAR> static cudaError_t configure_vjp() {
-    return cudaFuncSetAttribute(k_sweep_vjp<DIR, CHAR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)vjp_smem_bytes<DIR, CHAR>());
+template <int DIR, int FACES> static cudaError_t configure_vjp() {
+    return cudaFuncSetAttribute(k_sweep_vjp<DIR, FACES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)vjp_smem_bytes<DIR, FACES>());
+}
+
+template <int FACES> static cudaError_t configure_faces() {
+    cudaError_t e = configure_vjp<0, FACES>();
+    if (e == cudaSuccess) e = configure_vjp<1, FACES>();
+    return e == cudaSuccess ? configure_vjp<2, FACES>() : e;
 }
 
 cudaError_t adjoint_configure() {
     cudaError_t e;
-    if ((e = configure_vjp<0, false>()) != cudaSuccess || (e = configure_vjp<1, false>()) != cudaSuccess ||
-        (e = configure_vjp<2, false>()) != cudaSuccess || (e = configure_vjp<0, true>()) != cudaSuccess ||
-        (e = configure_vjp<1, true>()) != cudaSuccess)
+    if ((e = configure_faces<VJP_COMP>()) != cudaSuccess || (e = configure_faces<VJP_CHAR>()) != cudaSuccess ||
+        (e = configure_faces<VJP_NONE>()) != cudaSuccess)
         return e;
-    if ((e = configure_vjp<2, true>()) != cudaSuccess) return e;
     return weno_vjp_configure();
 }
 
-// With listed WENO faces the tiles hold linear and NND2 faces alone: the component-wise instance
-// serves both reconstructions (137 registers, three blocks of 96 threads per SM, against 234)
+template <int FACES> static cudaError_t launch_vjp_faces(int dir, const AdjArgs& a, cudaStream_t st) {
+    if (dir == 0) return launch_vjp_dir<0, FACES>(a, st);
+    return dir == 1 ? launch_vjp_dir<1, FACES>(a, st) : launch_vjp_dir<2, FACES>(a, st);
+}
+
+// With listed WENO faces, or a scheme without any, the tiles hold linear and NND2 faces alone.
 cudaError_t launch_sweep_vjp(int dir, const AdjArgs& a, cudaStream_t st) {
-    const bool ch = a.P.character != 0 && !a.Sb;
-    if (dir == 0) return ch ? launch_vjp_dir<0, true>(a, st) : launch_vjp_dir<0, false>(a, st);
-    if (dir == 1) return ch ? launch_vjp_dir<1, true>(a, st) : launch_vjp_dir<1, false>(a, st);
-    return ch ? launch_vjp_dir<2, true>(a, st) : launch_vjp_dir<2, false>(a, st);
+    if (a.Sb || a.P.fixed_branch == 0 || a.P.fixed_branch == 3) return launch_vjp_faces<VJP_NONE>(dir, a, st);
+    return a.P.character ? launch_vjp_faces<VJP_CHAR>(dir, a, st) : launch_vjp_faces<VJP_COMP>(dir, a, st);
 }
 
 static unsigned blocks_for(long long n, int t) { return (unsigned)((n + t - 1) / t); }
