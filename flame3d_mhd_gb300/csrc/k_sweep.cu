@@ -32,9 +32,10 @@ namespace f3d {
 // 320 x 4 4.77 / 46.9 / 1.22, 192 x 6 5.19 / 48.7 / 1.23, 160 x 5 4.87 / 46.5 / 1.21. With it (the WENO5 vortex 64^3):
 // 160 x 4 4.74 -> 288 x 3 4.64 ms, 320 x 3 4.67, 192 x 5 4.82. Tiles of eight lines or of
 // 32 cells lose more on the smaller grids than the ramp gains.
-// FP32: half-height tiles on 128 threads, six blocks per SM (~20 KB each): the same step time as
-// three 256-thread blocks on that tube, 6% less per RHS on the component-wise tube and on
-// the viscous vortex.
+// FP32: the same tile sizes (~20 KB) on 320 threads, five blocks per SM (40 registers, the
+// characteristic form spills ~150 bytes): one pass per phase and 50 warps an SM for the
+// latencies of the FP64 WENO7 weights. RK3 step of the FP32 shock tube 256x64x64, 128 threads x 6 ->
+// 320 x 5: 4.80 -> 4.07 ms (288 x 6 4.12, 288 x 5 4.19, 160 x 7 4.40, 224 x 6 4.47, 288 x 3 5.06).
 #ifndef SW_D_THREADS
 #define SW_D_THREADS 288
 #define SW_D_BLOCKS 3
@@ -49,8 +50,8 @@ namespace f3d {
 enum { WENO_COMP, WENO_CHAR, WENO_LISTED };  // WENO faces: component-, characteristic-wise, from k_weno.cu
 template <int DIR, class R, int FACES = WENO_COMP> struct Tile;
 #ifndef SW_F_THREADS
-#define SW_F_THREADS 128
-#define SW_F_BLOCKS 6
+#define SW_F_THREADS 320
+#define SW_F_BLOCKS 5
 #define SW_F_TL0 4
 #define SW_F_TL12 8
 #endif
