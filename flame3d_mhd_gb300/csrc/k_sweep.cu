@@ -32,10 +32,12 @@ namespace f3d {
 // 320 x 4 4.77 / 46.9 / 1.22, 192 x 6 5.19 / 48.7 / 1.23, 160 x 5 4.87 / 46.5 / 1.21. With it (the WENO5 vortex 64^3):
 // 160 x 4 4.74 -> 288 x 3 4.64 ms, 320 x 3 4.67, 192 x 5 4.82. Tiles of eight lines or of
 // 32 cells lose more on the smaller grids than the ramp gains.
-// FP32: the same tile sizes (~20 KB) on 320 threads, five blocks per SM (40 registers, the
-// characteristic form spills ~150 bytes): one pass per phase and 50 warps an SM for the
-// latencies of the FP64 WENO7 weights. RK3 step of the FP32 shock tube 256x64x64, 128 threads x 6 ->
-// 320 x 5: 4.80 -> 4.07 ms (288 x 6 4.12, 288 x 5 4.19, 160 x 7 4.40, 224 x 6 4.47, 288 x 3 5.06).
+// FP32: the same tile sizes (~20 KB). The Float32 form (FP64 WENO7 weights) on 320 threads, five
+// blocks per SM (32 registers, the characteristic form spills ~270 bytes): one pass per phase and 50
+// warps an SM for the latencies of the weights. RK3 step of its shock tube 256x64x64, 128 threads x
+// 6 -> 320 x 5: 4.80 -> 4.07 ms (288 x 6 4.12, 288 x 5 4.19, 160 x 7 4.40, 224 x 6 4.47, 288 x 3 5.06).
+// The mixed form (grids without TMA rows) keeps 128 x 6, 80 registers: on small grids the spills
+// would lengthen its faces' chains (RHS of 30x10x9: 53 us, 59 us at 320 x 5).
 #ifndef SW_D_THREADS
 #define SW_D_THREADS 288
 #define SW_D_BLOCKS 3
@@ -47,17 +49,24 @@ namespace f3d {
 #define SW_D_TC0 64
 #define SW_D_TC12 64
 #endif
-enum { WENO_COMP, WENO_CHAR, WENO_LISTED };  // WENO faces: component-, characteristic-wise, from k_weno.cu
+// WENO faces: component-, characteristic-wise, from k_weno.cu, the first two with the FP64 WENO7 weights of the Float32 form
+enum { WENO_COMP, WENO_CHAR, WENO_LISTED, WENO_COMP_REF32, WENO_CHAR_REF32 };
 template <int DIR, class R, int FACES = WENO_COMP> struct Tile;
 #ifndef SW_F_THREADS
-#define SW_F_THREADS 320
-#define SW_F_BLOCKS 5
+#define SW_F_THREADS 128
+#define SW_F_BLOCKS 6
+#define SW_R_THREADS 320
+#define SW_R_BLOCKS 5
 #define SW_F_TL0 4
 #define SW_F_TL12 8
 #endif
-template <int FACES> struct Tile<0, float, FACES> { static constexpr int TL = SW_F_TL0, TC = 64, NT = SW_F_THREADS, MINB = SW_F_BLOCKS; };
-template <int FACES> struct Tile<1, float, FACES> { static constexpr int TL = SW_F_TL12, TC = 32, NT = SW_F_THREADS, MINB = SW_F_BLOCKS; };
-template <int FACES> struct Tile<2, float, FACES> { static constexpr int TL = SW_F_TL12, TC = 32, NT = SW_F_THREADS, MINB = SW_F_BLOCKS; };
+template <int FACES> struct FloatTile {
+    static constexpr bool REF32 = FACES == WENO_COMP_REF32 || FACES == WENO_CHAR_REF32;
+    static constexpr int NT = REF32 ? SW_R_THREADS : SW_F_THREADS, MINB = REF32 ? SW_R_BLOCKS : SW_F_BLOCKS;
+};
+template <int FACES> struct Tile<0, float, FACES> { static constexpr int TL = SW_F_TL0, TC = 64, NT = FloatTile<FACES>::NT, MINB = FloatTile<FACES>::MINB; };
+template <int FACES> struct Tile<1, float, FACES> { static constexpr int TL = SW_F_TL12, TC = 32, NT = FloatTile<FACES>::NT, MINB = FloatTile<FACES>::MINB; };
+template <int FACES> struct Tile<2, float, FACES> { static constexpr int TL = SW_F_TL12, TC = 32, NT = FloatTile<FACES>::NT, MINB = FloatTile<FACES>::MINB; };
 template <int FACES> struct Tile<0, double, FACES> {
     static constexpr int TL = SW_D_TL0, TC = SW_D_TC0, NT = SW_D_THREADS,
                          MINB = FACES == WENO_LISTED ? SW_D_LISTED_BLOCKS : SW_D_BLOCKS;
@@ -153,7 +162,7 @@ __global__ void __launch_bounds__(Tile<DIR, R, FACES>::NT, Tile<DIR, R, FACES>::
         if (FACES != WENO_LISTED && (br == 1 || br == 2)) s0 = A(2) / (arith(Sr[cl]) + arith(Sr[cr]));
         auto FP = [&](int n, int p) { return arith(sFp[n * TL * NP + sidx(l, p)]); };
         auto FM = [&](int n, int p) { return arith(sFm[n * TL * NP + sidx(l, p)]); };
-        face_flux<FACES == WENO_CHAR, A>(P, a, br, t, s0, cl, cr, FP, FM, out);
+        face_flux<FACES == WENO_CHAR || FACES == WENO_CHAR_REF32, A>(P, a, br, t, s0, cl, cr, FP, FM, out);
         const int f = fidx(l, t);
 #pragma unroll
         for (int n = 0; n < 5; n++) sF[n * TL * NF + f] = plain(out[n]);
@@ -290,7 +299,9 @@ cudaError_t sweep_configure() {
     if ((e = configure_faces<WENO_CHAR, double>()) != cudaSuccess) return e;
     if ((e = configure_faces<WENO_LISTED, double>()) != cudaSuccess) return e;
     if ((e = configure_faces<WENO_COMP, float>()) != cudaSuccess) return e;
-    return configure_faces<WENO_CHAR, float>();
+    if ((e = configure_faces<WENO_CHAR, float>()) != cudaSuccess) return e;
+    if ((e = configure_faces<WENO_COMP_REF32, float>()) != cudaSuccess) return e;
+    return configure_faces<WENO_CHAR_REF32, float>();
 }
 
 template <int DIR, int FACES, class R> static cudaError_t launch_dir(const SweepArgs& a, cudaStream_t st) {
@@ -314,6 +325,8 @@ template <int FACES, class R> static cudaError_t launch_faces(int dir, const Swe
 // no WENO code: 56 registers a thread, and one instance for component- and characteristic-wise faces.
 cudaError_t launch_sweep(int dir, const SweepArgs& a, cudaStream_t st) {
     const bool ch = a.P.character != 0;
+    if (a.fp32 && a.P.ref32)
+        return ch ? launch_faces<WENO_CHAR_REF32, float>(dir, a, st) : launch_faces<WENO_COMP_REF32, float>(dir, a, st);
     if (a.fp32) return ch ? launch_faces<WENO_CHAR, float>(dir, a, st) : launch_faces<WENO_COMP, float>(dir, a, st);
     const int fb = a.P.fixed_branch;
     if (fb == 0 || fb == 3 || (a.wflux && fb < 0)) return launch_faces<WENO_LISTED, double>(dir, a, st);
