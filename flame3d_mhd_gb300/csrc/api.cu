@@ -30,18 +30,18 @@ static int fixed_branch_of(const f3d_params& p) {
 }
 
 // The linear coefficients as integers over a common denominator D (f3d_fixed.cuh): 420 m with
-// the smallest m <= 500 that makes 420 m (up7 phi + cd6 (1 - phi)) whole for the given blend
+// the smallest m <= 500 that makes 420 m (up7_420 phi + cd6_420 (1 - phi)) whole for the given blend
 // (m = 1 for phi = 0 and 1, 2 for 0.5, 10 for 0.9, ...), with the signs of a blend in [0, 1] and
 // 32-bit accumulations' room (sum |c| < 2^20).
 static void integer_coefficients(double phi, DevParams& d) {
-    const double up7[7] = {-3, 25, -101, 319, 214, -38, 4}, cd6[7] = {0, 7, -56, 259, 259, -56, 7};
+    const double up7_420[7] = {-3, 25, -101, 319, 214, -38, 4}, cd6_420[7] = {0, 7, -56, 259, 259, -56, 7};
     d.lin_int = 0;
     if (!(phi >= 0.0 && phi <= 1.0)) return;
     for (int m = 1; m <= 500; m++) {
         int c[7];
         bool whole = true;
         for (int k = 0; k < 7; k++) {
-            const double v = m * (up7[k] * phi + cd6[k] * (1.0 - phi)), r = std::nearbyint(v);
+            const double v = m * (up7_420[k] * phi + cd6_420[k] * (1.0 - phi)), r = std::nearbyint(v);
             c[k] = (int)r;
             whole = whole && std::fabs(v - r) <= 1e-12 * m;
         }
