@@ -12,10 +12,10 @@ namespace f3d {
 // come from the arithmetic mean of u, v, w, T and of the metric row at the two adjacent cells
 // (cl, cr linear indices), read from global memory. Rows of L and of R are selected by a
 // runtime index, and the field loop is not unrolled: one copy of the WENO code serves the
-// five fields (the FP64 characteristic sweeps hold 96 registers with no spills this way).
-// Spreading a face over five lanes, one field each, with the fluxes exchanged by shuffles
-// ran 7.5% slower per RK3 step on the 256x64x64 shock tube than one thread per face: the
-// five copies of the basis cost more than the idle lanes of a short WENO queue.
+// five fields. Within a tile one thread takes a face: spreading it over five lanes, one field
+// each, with the fluxes exchanged by shuffles, ran 7.5% slower per RK3 step on the 256x64x64 shock
+// tube (five copies of the basis). k_weno.cu takes the listed faces one field a warp, where the basis
+// is formed once for the five.
 template <class R> struct CharBasis {
     R u, v, w, c, q2, H, qn, ql, qm, nx, ny, nz, lx, ly, lz, mx, my, mz, c2, K2, Kc;
 };

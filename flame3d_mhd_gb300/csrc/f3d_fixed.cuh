@@ -13,7 +13,8 @@
 // FP64 instruction a face and component instead of 14. On the 256x64x64 shock tube the three
 // sweeps' FP64 thread instructions go from 181-189 / 160-167 / 166-184 million a launch to
 // 112 / 90 / 107, the sweeps from 517 / 434 / 453 to 366 / 324 / 373 us and the RK3 step from 4.68
-// to 3.67 ms; the viscous ramp's step at 512x256x128 from 75.4 to 61.0 ms. Five faces a strip:
+// to 3.67 ms; the viscous ramp's step at 512x256x128 from 75.4 to 61.0 ms (all measured before the
+// WENO faces left the tiles). Five faces a strip:
 // their windows share four positions, which bounds the spread, and 22 conversions serve five
 // faces; 13 strips cover a tile's 65 faces exactly.
 //

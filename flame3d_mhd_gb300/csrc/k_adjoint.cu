@@ -4,9 +4,9 @@
 //   --split--> Fp, Fm --reconstruction--> face fluxes --difference x J--> L,
 //   plus Q --gradients--> Fv --CD4 x J--> L (viscous).
 // The kernels below run it backwards for a cotangent Lb of L (interior cells):
-//   k_sweep_vjp<d,char> face cotangents from J Lb, reverse of UP7/WENO7/WENO5/NND2 on the
-//                       forward branch (component- or characteristic-wise: char_face_vjp),
-//                       reverse of the split (SW, LF, VL, AUSM), into Qb;
+//   k_sweep_vjp<d,faces> face cotangents from J Lb, reverse of UP7/WENO7/WENO5/NND2 on the
+//                       forward branch (component- or characteristic-wise: char_face_vjp; listed
+//                       WENO faces by k_weno_vjp.cu), reverse of the split (SW, LF, VL, AUSM), into Qb;
 //   k_visc_fvb          Fv cotangents: transpose of the CD4 divergence (div.jl:14-48);
 //   k_visc_vjp          reverse of viscousFlux per cell into gradient/centre cotangents;
 //   k_visc_gather       transpose of the CD4 gradients (viscous.jl:29-42) into Qb;
@@ -35,7 +35,8 @@ namespace f3d {
 // state (its eigenvectors, a side's stencil of one field and its cotangents). Smaller blocks
 // (xi 4 x 64 on 64 threads, three per SM; eta / zeta 4 x 64 on 96 threads, two per SM):
 // adjoint / forward 3.70 on the 256x64x64 shock tube against 3.78 for the component-wise
-// shape and 3.90 for 192-thread blocks with 255 registers (same box, alternating builds)
+// shape and 3.90 for 192-thread blocks with 255 registers (same box, alternating builds). Used
+// where the WENO faces are not listed: metric cotangents, or no room for the lists
 #ifndef V_C_TL0
 #define V_C_TL0 4
 #define V_C_NT0 64
