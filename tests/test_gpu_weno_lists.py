@@ -100,3 +100,47 @@ def test_reverse_equals_the_tiles_reverse(gpu_lib, n, which, character, split):
         assert torch.isfinite(got).all()
         assert (got - want).abs().max() <= 1e-11 * scale, float((got - want).abs().max() / scale)
     s.close()
+
+
+@pytest.mark.parametrize("n", [(4, 4, 4), (33, 5, 9), (65, 9, 63)])
+@pytest.mark.parametrize("fixed,hybrid", [((5.0, 6.0, 7.0), (3.5, 6.0, 7.0)), ((0.0, 0.0, 0.0), (1e-30, 1e-30, 1e-30))])
+@pytest.mark.parametrize("split", ["SW", "LF", "VL", "AUSM"])
+def test_reverse_of_a_fixed_branch(gpu_lib, n, fixed, hybrid, split):
+    """Every face linear or every face NND2, reversed by the tiles without WENO code (which split cells
+    for NND2 faces alone), against the same faces under the hybrid switch with metric cotangents
+    requested, whose tiles hold all branches and split every cell."""
+    import torch
+
+    from flame3d_mhd_gb300.solver import Flame3D
+    nx, ny, nz = n
+    per = dict(kind=abi.BC_PERIODIC)
+    out = []
+    for p in (fixed, hybrid):
+        s = Flame3D(abi.make_params(nx, ny, nz, phi1=p[0], phi2=p[1], phi3=p[2], viscous=0, character=0, split=split,
+                                    bc=[per] * 6))
+        shape = (nz + 8, ny + 8, nx + 8)
+        g = torch.Generator(device="cuda").manual_seed(3)
+        uni = lambda *sh: torch.rand(sh, generator=g, dtype=torch.float64, device="cuda")  # noqa: E731
+        eye = [1.0, 0.0, 0.0, 0.0, 1.0, 0.0, 0.0, 0.0, 1.0]
+        # periodic inputs: the metrics are smooth functions of the cell indices
+        z, y, x = torch.meshgrid(*[torch.arange(m, dtype=torch.float64, device="cuda") - 4 for m in shape], indexing="ij")
+        w = [torch.sin(2 * np.pi * (x / nx + k * y / ny + z / nz)) for k in range(1, 10)]
+        s.set_metrics([e + 0.1 * v for e, v in zip(eye, w)], torch.ones(shape, dtype=torch.float64, device="cuda"))
+        Q = torch.empty((6, *shape), dtype=torch.float64, device="cuda")
+        Q[0] = 0.7 + 0.6 * uni(*shape)
+        Q[1:4] = 1.2 * uni(3, *shape) - 0.6
+        Q[4] = (0.3 + 1.2 * uni(*shape)) ** 2
+        Q[5] = Q[4] / (Q[0] * 287.0)
+        U = s.field(5)
+        s.prim2c(U, Q)
+        s.fillGhost(Q, U)
+        Lbar = s.field(5)
+        Lbar[:, 4:-4, 4:-4, 4:-4] = 2.0 * uni(5, nz, ny, nx) - 1.0
+        if p is hybrid:
+            bars = [s.field(1) for _ in range(10)]
+            s.set_metrics_cotangent(bars[:9], bars[9])
+        out.append(s.rhs_vjp(U, Lbar).clone())
+        s.close()
+    # sums of the same ~100 rounded products a cell in another order
+    assert torch.isfinite(out[0]).all()
+    assert (out[0] - out[1]).abs().max() <= 1e-13 * out[1].abs().max()
