@@ -315,16 +315,14 @@ __global__ void __launch_bounds__(VTile<DIR, FACES>::NT, VTile<DIR, FACES>::MINB
             if (l >= nl) continue;
             const int p0 = sp * LIN_STRIP;
             const double* G = sG + n * TL * NFV;
-            double gm[LIN_STRIP], gp[LIN_STRIP];
-            linear_strip_both(P, p0 - 7, [&](int t) { return t >= 0 && t < NFV ? G[gidx(l, t)] : 0.0; }, gm, gp);
-#pragma unroll
-            for (int f = 0; f < LIN_STRIP; f++)
-                if (p0 + f < np) {
-                    const int s = n * TL * NP + sidx(l, p0 + f);
-                    // linear faces alone leave the cotangents at zero so far
-                    if (__double_as_longlong(gp[f]) << 1) sFpb[s] = (f64(sFpb[s]) + f64(gp[f])).v;
-                    if (__double_as_longlong(gm[f]) << 1) sFmb[s] = (f64(sFmb[s]) + f64(gm[f])).v;
-                }
+            const unsigned want = (1u << min(LIN_STRIP, np - p0)) - 1u;
+            linear_strip_both(P, p0 - 7, want, [&](int t) { return t >= 0 && t < NFV ? G[gidx(l, t)] : 0.0; },
+                              [&](int f, double gm, double gp) {
+                                  const int s = n * TL * NP + sidx(l, p0 + f);
+                                  // linear faces alone leave the cotangents at zero so far
+                                  if (__double_as_longlong(gp) << 1) sFpb[s] = (f64(sFpb[s]) + f64(gp)).v;
+                                  if (__double_as_longlong(gm) << 1) sFmb[s] = (f64(sFmb[s]) + f64(gm)).v;
+                              });
         }
         __syncthreads();
     }

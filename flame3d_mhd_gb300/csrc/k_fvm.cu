@@ -278,14 +278,12 @@ __global__ void __launch_bounds__(FvmLaunch<EIGEN>::NT, FvmLaunch<EIGEN>::MINB) 
             if (l >= nl) continue;
             const int t0 = st * LIN_STRIP;
             const double* u = sU + n * TL * NP;
-            double up[LIN_STRIP], down[LIN_STRIP];
-            linear_strip_both(P, t0, [&](int p) { return p <= last ? u[sidx(l, p)] : 0.0; }, up, down);
-#pragma unroll
-            for (int f = 0; f < LIN_STRIP; f++)
-                if (t0 + f <= nc) {
-                    sL[n * TL * NF + fidx(l, t0 + f)] = up[f];
-                    sL[(n + 5) * TL * NF + fidx(l, t0 + f)] = down[f];
-                }
+            const unsigned want = (1u << min(LIN_STRIP, nc + 1 - t0)) - 1u;
+            linear_strip_both(P, t0, want, [&](int p) { return p <= last ? u[sidx(l, p)] : 0.0; },
+                              [&](int f, double up, double down) {
+                                  sL[n * TL * NF + fidx(l, t0 + f)] = up;
+                                  sL[(n + 5) * TL * NF + fidx(l, t0 + f)] = down;
+                              });
         }
         __syncthreads();
     }

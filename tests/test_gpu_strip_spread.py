@@ -1,0 +1,113 @@
+"""GPU: sums of the integer strips (f3d_fixed.cuh) whose own window holds none of the strip's large
+values keep the accuracy of FP64 sums of their own terms. Steps and impulses of many orders of
+magnitude at every offset from the strips' starts, in both directions along the line; each value
+is held to a tolerance relative to what it reads."""
+import numpy as np
+import pytest
+
+from flame3d_mhd_gb300 import abi
+
+pytestmark = pytest.mark.gpu
+
+EPS = 2.0 ** -53
+PER = [dict(kind=abi.BC_PERIODIC)] * 6
+LINEAR = dict(phi1=5.0, phi2=6.0, phi3=7.0)  # above any sensor value: every face is linear
+
+
+def _dev(a):
+    import torch
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def _box(d, n, m=6):
+    """Interior size (nx, ny, nz): n along direction d, m across."""
+    return tuple(n if e == d else m for e in range(3))
+
+
+@pytest.mark.parametrize("d", [0, 1, 2])
+@pytest.mark.parametrize("step", [1e-6, 1e-12, 1e-20])
+@pytest.mark.parametrize("offset", range(5))
+def test_finite_volume_states_beside_a_step(gpu_lib, d, step, offset):
+    """CD6 states (their outermost coefficients are zero) of a gas whose density and pressure fall by
+    `step` and rise again: faces that read the small state alone have its flux."""
+    import torch
+
+    from flame3d_mhd_gb300.solver import Flame3D
+    from oracle import oracle as orc
+    n = _box(d, 72)
+    P = abi.make_params(*n, viscous=0, linear_phi=0.0, scheme=abi.SCHEME_FVM_CONS, bc=PER, **LINEAR)
+    shape = (n[2] + 8, n[1] + 8, n[0] + 8)
+    z, y, x = np.meshgrid(*[(np.arange(k) - 3.5) for k in shape], indexing="ij")
+    i = np.broadcast_to(np.arange(shape[2 - d]).reshape([-1 if a == 2 - d else 1 for a in range(3)]), shape)
+    small = ((i >= 12 + offset) & (i < 31 + offset)) | ((i >= 44 + offset) & (i < 57 + offset))
+    r = np.random.default_rng(4)
+    rho = np.where(small, step, 1.0) * r.uniform(0.99, 1.01, shape)
+    Q = np.empty((6, *shape))
+    Q[0], Q[1:4] = rho, np.array([0.3, -0.2, 0.4]).reshape(3, 1, 1, 1)
+    Q[4] = 0.7 * rho
+    Q[5] = Q[4] / (rho * P.rg)
+    m, J = [np.full(shape, e) for e in (1., 0., 0., 0., 1., 0., 0., 0., 1.)], np.ones(shape)
+    s = Flame3D(P)
+    s.set_metrics([_dev(a) for a in m], _dev(J))
+    s.set_coordinates(_dev(x), _dev(y), _dev(z))
+    phi, U = np.zeros(shape), orc.prim2c(P, Q)
+    want = orc.fvm_face_flux(P, d, False, phi, np.ones(shape), Q, U, x, y, z)
+    F = torch.zeros((5, *orc.face_shape(P, d)), dtype=torch.float64, device="cuda")
+    s.advect(d, F, _dev(phi), _dev(Q))
+    s.close()
+    got = np.moveaxis(F.cpu().numpy(), 3 - d, -1)
+    want = np.moveaxis(want, 3 - d, -1)
+    line = np.moveaxis(small, 2 - d, -1)[0, 0]
+    faces = [t for t in range(want.shape[-1]) if line[t + 1:t + 7].all()]  # CD6 reads positions t+1 .. t+6
+    assert len(faces) >= 18
+    # an HLLC flux of states with relative error ~4 eps is within ~100 eps of its largest component
+    scale = np.abs(want).max(0)
+    for t in faces:
+        assert (np.abs(got[..., t] - want[..., t]).max(0) <= 1e-13 * scale[..., t]).all(), t
+
+
+@pytest.mark.parametrize("d", [0, 1, 2])
+@pytest.mark.parametrize("towards", [1, -1])
+@pytest.mark.parametrize("step", [1e-9, 1e-12, 1e-19])
+def test_reverse_of_localised_cotangents(gpu_lib, d, towards, step):
+    """Cotangents of a masked objective: they fall by `step` and rise again along one direction, at
+    every offset from a strip's start. The gas is supersonic, so a cell hears from one side. UP7
+    (integer strips) against a blend 2^-40 away from it, which has no small denominator and is summed in
+    FP64: the two linear operators differ by 2^-40 of their coefficients."""
+    from flame3d_mhd_gb300.solver import Flame3D
+    for offset in range(5):
+        n = _box(d, 72)
+        shape = (n[2] + 8, n[1] + 8, n[0] + 8)
+        r = np.random.default_rng(6)
+        q = np.empty((6, *shape))
+        q[0] = r.uniform(0.8, 1.2, shape)
+        q[1:4] = r.uniform(-0.2, 0.2, (3, *shape))
+        q[1 + d] += 3.0 * towards
+        q[4] = q[0] * r.uniform(0.6, 0.8, shape)
+        q[5] = q[4] / (q[0] * 287.0)
+        i = np.arange(n[d])
+        small = ((i >= 8 + offset) & (i < 27 + offset)) | ((i >= 40 + offset) & (i < 53 + offset))
+        mag = np.where(small, step, 1.0).reshape([-1 if a == 2 - d else 1 for a in range(3)])
+        Lbar = np.zeros((5, *shape))
+        inner = (5, n[2], n[1], n[0])
+        Lbar[:, 4:-4, 4:-4, 4:-4] = mag * r.uniform(0.5, 1.0, inner) * r.choice([-1.0, 1.0], inner)
+        out = []
+        for phi in (1.0, 1.0 - 2.0 ** -40):
+            s = Flame3D(abi.make_params(*n, viscous=0, linear_phi=phi, bc=PER, **LINEAR))
+            one, zero = np.ones(shape), np.zeros(shape)
+            s.set_metrics([_dev(a) for a in (one, zero, zero, zero, one, zero, zero, zero, one)], _dev(one))
+            U = s.field(5)
+            Q = _dev(q)
+            s.prim2c(U, Q)
+            s.fillGhost(Q, U)
+            out.append(s.rhs_vjp(U, _dev(Lbar)).cpu().numpy()[:, 4:-4, 4:-4, 4:-4])
+            s.close()
+        a, b = out
+        # Fp of cell c enters the right-hand sides of c - 3 .. c + 4, Fm those of c - 4 .. c + 3
+        hears = np.arange(-3, 5) if towards > 0 else np.arange(-4, 4)
+        reach = np.array([mag.ravel()[(c + hears) % n[d]].max() for c in range(n[d])]).reshape(mag.shape)
+        assert (reach == step).sum() >= 15
+        scale = np.abs(b).max()
+        # coefficients differ by 60/420 2^-40, the Jacobian's entries are below `scale` per unit of cotangent
+        off = np.abs(a - b) / (scale * reach)
+        assert off.max() <= 8 * 2.0 ** -40, (offset, float(off.max()))
