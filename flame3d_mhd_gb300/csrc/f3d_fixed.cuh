@@ -14,26 +14,28 @@
 // sweeps' FP64 thread instructions go from 181-189 / 160-167 / 166-184 million a launch to
 // 112 / 90 / 107, the sweeps from 517 / 434 / 453 to 366 / 324 / 373 us and the RK3 step from 4.68
 // to 3.67 ms; the viscous ramp's step at 512x256x128 from 75.4 to 61.0 ms (all measured before the
-// WENO faces left the tiles). Five faces a strip:
-// their windows share four positions, which bounds the spread, and 22 conversions serve five
-// faces; 13 strips cover a tile's 65 faces exactly.
+// WENO faces left the tiles). Five faces a strip: 22 conversions serve five faces, and 13 strips
+// cover a tile's 65 faces exactly.
 //
-// Accuracy: a value whose exponent lies within 9 of the largest is exact; smaller ones lose bits
-// below 2^-62 of the largest. A strip is taken only when a flux that all of its five faces read is
-// within 2^5 of the largest; other strips (and infinities, NaN and magnitudes near the ends of the FP64
-// range) are summed in FP64. linear_strip_both decides sum by sum: each is formed from integers only if the
-// larger of its own two central values is within 2^5 of the strip's largest, or if every value of the
-// strip enters exactly (beyond_spread): what is truncated then stays below 0.3 x 2^-53 of the sum of the
-// magnitudes of its own terms, a third of an FP64 evaluation's rounding. The strip's largest value need
-// not be one that a sum reads: with the values 4..7 of a strip tested together, a step of 1e-12 between
-// values 6 and 7 left the sum of values 0..6 with a relative error of 1e-8.
+// Accuracy: a value whose exponent lies within 9 of the strip's largest is exact; smaller ones are
+// truncated to a multiple of 2^-61 of it (in units of the largest's power of two). The largest need not
+// be a value that a sum reads, or reads under a coefficient that matters (they go down to 3/420), so each
+// sum is looked at by itself (beyond_spread): it is formed from integers if one of the values under
+// its central coefficients (214/420 and above) is within 2^5 of the largest, or if every value of the strip
+// enters exactly. What is truncated is then at most 2.9 units for a face (1.2 for a one-sided sum), the
+// central term alone at least 2^-6 of the largest, so the error is below 0.7 x 2^-53 (0.3) of the sum of
+// the magnitudes of the sum's own terms, less than an FP64 evaluation rounds. Then one rounding to FP64
+// and one in the product with 1/D. Other sums, infinities, NaN and strips whose magnitudes lie
+// near the ends of the FP64 range are formed in FP64. Against extended precision the right-hand side of
+// a coarse tube is off by 0.95 / 0.85 / 0.91 (Steger-Warming / Lax-Friedrichs / AUSM) and of a
+// finite-volume vortex by 0.97 of what FP64 sums leave.
 #pragma once
 #include "f3d_kernels.cuh"
 
 namespace f3d {
 
-constexpr int LIN_STRIP = 5;    // faces a strip: the five windows share positions 4..7
-constexpr int LIN_SPREAD = 5;   // largest exponent minus that of the shared positions, or of a sum's centre
+constexpr int LIN_STRIP = 5;    // faces a strip
+constexpr int LIN_SPREAD = 5;   // largest exponent minus that of a sum's centre
 
 // x 2^(1084 - E) as an integer (E: the strip's largest biased exponent), truncated towards zero
 __device__ __forceinline__ long long fixed_of(double x, int E) {
@@ -180,67 +182,80 @@ __device__ __forceinline__ void linear_strip_both(const DevParams& P, int t0, un
     }
 }
 
-// The five faces t0 .. t0+4 of one line and component: out[f] = sum_k lin[k] (Fp(t+k) + Fm(t+7-k)),
-// t = t0 + f. FP / FM(p) read the split fluxes at position p; positions past `last` were not
-// filled and count as zero (no face that is kept reads them).
-template <class FPA, class FMA>
-__device__ __forceinline__ void linear_strip(const DevParams& P, int t0, int last, FPA FP, FMA FM,
-                                             double out[LIN_STRIP]) {
+// Of the five faces t0 .. t0+4 of one line and component those in `want`: put(f, sum_k lin[k]
+// (Fp(t+k) + Fm(t+7-k))), t = t0 + f. FP / FM(p) read the split fluxes at position p; positions past
+// `last` were not filled and count as zero (no face in `want` reads them).
+template <class FPA, class FMA, class PUT>
+__device__ __forceinline__ void linear_strip(const DevParams& P, int t0, int last, unsigned want, FPA FP, FMA FM, PUT put) {
     constexpr int NV = LIN_STRIP + 6;
-    // FP64 bit patterns without their sign order like the magnitudes
-    unsigned top = 0u, mid = 0u;
+    // the strip's values V(q), q = 0..NV-1: Fp at t0 + q, Fm at t0 + 1 + q
+    auto P_ = [&](int q) { return t0 + q <= last ? FP(t0 + q) : 0.0; };
+    auto M_ = [&](int q) { return t0 + 1 + q <= last ? FM(t0 + 1 + q) : 0.0; };
+    // FP64 bit patterns without their sign order like the magnitudes; mid[i]: at position t0 + 3 + i
+    unsigned top = 0u, low = 0u, mid[LIN_STRIP + 1];
 #pragma unroll
-    for (int p = 0; p < NV; p++) {
-        const unsigned a = t0 + p <= last ? (unsigned)__double2hiint(FP(t0 + p)) & 0x7fffffffu : 0u;
-        const unsigned b = t0 + p + 1 <= last ? (unsigned)__double2hiint(FM(t0 + p + 1)) & 0x7fffffffu : 0u;
+    for (int i = 0; i <= LIN_STRIP; i++) mid[i] = 0u;
+#pragma unroll
+    for (int q = 0; q < NV; q++) {
+        const double v = P_(q), w = M_(q);
+        const unsigned a = (unsigned)__double2hiint(v) & 0x7fffffffu, b = (unsigned)__double2hiint(w) & 0x7fffffffu;
+        low |= (unsigned)__double2loint(v) | (unsigned)__double2loint(w);
         top = max(top, max(a, b));
-        if (p >= LIN_STRIP - 1 && p <= 6) mid = max(mid, max(a, b));
+        if (q >= 3 && q <= LIN_STRIP + 3) mid[q - 3] = max(mid[q - 3], a);
+        if (q >= 2 && q <= LIN_STRIP + 2) mid[q - 2] = max(mid[q - 2], b);
     }
-    const int E = (int)(top >> 20), Em = (int)(mid >> 20);
-    if (top == 0u) {  // all zero (or below 2^-1042)
+    if ((top | low) == 0u) {
 #pragma unroll
-        for (int f = 0; f < LIN_STRIP; f++) out[f] = 0.0;
+        for (int f = 0; f < LIN_STRIP; f++)
+            if (want >> f & 1u) put(f, 0.0);
         return;
     }
-    if (E < 200 || E > 1900 || E - Em > LIN_SPREAD) {
+    const int E = (int)(top >> 20);
+    unsigned far = want;  // the faces to sum in FP64
+    if (E >= 200 && E <= 1900) {
+        far = beyond_spread(E, want, [&](int f) { return max(mid[f], mid[f + 1]); });
+        if (far) {
+            bool exact = true;
 #pragma unroll
-        for (int f = 0; f < LIN_STRIP; f++) {
-            const int t = t0 + f;
-            out[f] = 0.0;
-            if (t + 7 <= last)
-                out[f] = P.cd.lin[0] * (FP(t) + FM(t + 7)) + P.cd.lin[1] * (FP(t + 1) + FM(t + 6)) +
-                         P.cd.lin[2] * (FP(t + 2) + FM(t + 5)) + P.cd.lin[3] * (FP(t + 3) + FM(t + 4)) +
-                         P.cd.lin[4] * (FP(t + 4) + FM(t + 3)) + P.cd.lin[5] * (FP(t + 5) + FM(t + 2)) +
-                         P.cd.lin[6] * (FP(t + 6) + FM(t + 1));
-        }
-        return;
-    }
-    // sums of the upper words (signed), and of the lower words under the positive and the
-    // negative coefficients (0, 2 and 5)
-    long long hs[LIN_STRIP];
-    unsigned long long lp[LIN_STRIP], ln[LIN_STRIP];
-#pragma unroll
-    for (int f = 0; f < LIN_STRIP; f++) { hs[f] = 0; lp[f] = ln[f] = 0ull; }
-    auto add = [&](int f, int k, int vh, unsigned vl) {
-        hs[f] += (long long)vh * P.lin_c[k];
-        if (k == 0 || k == 2 || k == 5) ln[f] += (unsigned long long)vl * (unsigned)(-P.lin_c[k]);
-        else lp[f] += (unsigned long long)vl * (unsigned)P.lin_c[k];
-    };
-#pragma unroll
-    for (int p = 0; p < NV; p++) {
-        const long long v = t0 + p <= last ? fixed_of(FP(t0 + p), E) : 0ll;
-        const long long w = t0 + p + 1 <= last ? fixed_of(FM(t0 + p + 1), E) : 0ll;
-#pragma unroll
-        for (int f = 0; f < LIN_STRIP; f++) {
-            const int kp = p - f, km = 6 + f - p;  // Fp(t + kp), Fm(t + 7 - km)
-            if (kp >= 0 && kp < 7) add(f, kp, (int)(v >> 32), (unsigned)v);
-            if (km >= 0 && km < 7) add(f, km, (int)(w >> 32), (unsigned)w);
+            for (int q = 0; q < NV; q++) exact = exact && enters_exactly(P_(q), E) && enters_exactly(M_(q), E);
+            if (exact) far = 0u;
         }
     }
+    if (far != want) {
+        // sums of the upper words (signed), and of the lower words under the positive and the
+        // negative coefficients (0, 2 and 5)
+        long long hs[LIN_STRIP];
+        unsigned long long lp[LIN_STRIP], ln[LIN_STRIP];
 #pragma unroll
-    for (int f = 0; f < LIN_STRIP; f++) {
-        const long long l = (long long)(lp[f] - ln[f]);
-        out[f] = F64(f64(fixed_to_f64(hs[f] + (l >> 32), (unsigned)l, E)) * F64(P.lin_s)).v;
+        for (int f = 0; f < LIN_STRIP; f++) { hs[f] = 0; lp[f] = ln[f] = 0ull; }
+        auto add = [&](int f, int k, int vh, unsigned vl) {
+            hs[f] += (long long)vh * P.lin_c[k];
+            if (k == 0 || k == 2 || k == 5) ln[f] += (unsigned long long)vl * (unsigned)(-P.lin_c[k]);
+            else lp[f] += (unsigned long long)vl * (unsigned)P.lin_c[k];
+        };
+#pragma unroll
+        for (int q = 0; q < NV; q++) {
+            const long long v = fixed_of(P_(q), E), w = fixed_of(M_(q), E);
+#pragma unroll
+            for (int f = 0; f < LIN_STRIP; f++) {
+                const int kp = q - f, km = 6 + f - q;  // Fp(t + kp), Fm(t + 7 - km)
+                if (kp >= 0 && kp < 7) add(f, kp, (int)(v >> 32), (unsigned)v);
+                if (km >= 0 && km < 7) add(f, km, (int)(w >> 32), (unsigned)w);
+            }
+        }
+#pragma unroll
+        for (int f = 0; f < LIN_STRIP; f++) {
+            const long long l = (long long)(lp[f] - ln[f]);
+            const double r = F64(f64(fixed_to_f64(hs[f] + (l >> 32), (unsigned)l, E)) * F64(P.lin_s)).v;
+            if ((want & ~far) >> f & 1u) put(f, r);
+        }
+    }
+    for (; far; far &= far - 1u) {
+        const int f = __ffs((int)far) - 1, t = t0 + f;
+        put(f, P.cd.lin[0] * (FP(t) + FM(t + 7)) + P.cd.lin[1] * (FP(t + 1) + FM(t + 6)) +
+                   P.cd.lin[2] * (FP(t + 2) + FM(t + 5)) + P.cd.lin[3] * (FP(t + 3) + FM(t + 4)) +
+                   P.cd.lin[4] * (FP(t + 4) + FM(t + 3)) + P.cd.lin[5] * (FP(t + 5) + FM(t + 2)) +
+                   P.cd.lin[6] * (FP(t + 6) + FM(t + 1)));
     }
 }
 

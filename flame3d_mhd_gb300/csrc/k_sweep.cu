@@ -248,12 +248,9 @@ __global__ void __launch_bounds__(Tile<DIR, R, FACES>::NT, Tile<DIR, R, FACES>::
                 if (!want) continue;
                 const R* fp = sFp + n * TL * NP;
                 const R* fm = sFm + n * TL * NP;
-                double out[LIN_STRIP];
-                linear_strip(P, t0, nc + 7, [&](int p) { return (double)fp[sidx(l, p)]; },
-                             [&](int p) { return (double)fm[sidx(l, p)]; }, out);
-#pragma unroll
-                for (int f = 0; f < LIN_STRIP; f++)
-                    if (want >> f & 1u) sF[n * TL * NF + fidx(l, t0 + f)] = out[f];
+                linear_strip(P, t0, nc + 7, want, [&](int p) { return (double)fp[sidx(l, p)]; },
+                             [&](int p) { return (double)fm[sidx(l, p)]; },
+                             [&](int f, double v) { sF[n * TL * NF + fidx(l, t0 + f)] = v; });
             }
         }
     }

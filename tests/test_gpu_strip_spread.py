@@ -111,3 +111,49 @@ def test_reverse_of_localised_cotangents(gpu_lib, d, towards, step):
         # coefficients differ by 60/420 2^-40, the Jacobian's entries are below `scale` per unit of cotangent
         off = np.abs(a - b) / (scale * reach)
         assert off.max() <= 8 * 2.0 ** -40, (offset, float(off.max()))
+
+
+@pytest.mark.parametrize("d", [0, 1, 2])
+@pytest.mark.parametrize("towards", [1, -1])
+@pytest.mark.parametrize("phi", [1.0, 0.5])
+def test_linear_faces_beside_large_values(gpu_lib, d, towards, phi):
+    """Face fluxes against sums in extended precision of the library's own split fluxes. A supersonic
+    gas (one of Fp, Fm is zero) with, at every offset from a strip's start, four cells of density ~1, one
+    2^-5 below and the rest ~2^-20: a face that reads the middle cell under its smallest coefficient
+    has nothing else of that size."""
+    from flame3d_mhd_gb300.solver import Flame3D
+    n = _box(d, 64, 12)
+    s = Flame3D(abi.make_params(*n, viscous=0, linear_phi=phi, bc=PER, **LINEAR))
+    shape = (n[2] + 8, n[1] + 8, n[0] + 8)
+    r = np.random.default_rng(9)
+    rho = 2.0 ** -20 * r.uniform(1.0, 2.0, shape)
+    line = np.moveaxis(rho, 2 - d, -1)  # a view: lines along the direction
+    big = r.uniform(1.0, 1.9, line.shape)
+    for a in range(line.shape[0]):
+        for b in range(line.shape[1]):
+            for c in range((3 * a + b) % 20, 72 - 8, 20):
+                at = range(c, c + 5) if towards > 0 else range(c + 4, c - 1, -1)
+                for k, p in enumerate(at):
+                    line[a, b, p] = big[a, b, p] * (1.0 if k < 4 else 2.0 ** -5)
+    q = np.zeros((6, *shape))
+    q[0] = rho
+    q[1 + d] = 3.0 * towards
+    q[4] = rho / 1.4
+    q[5] = q[4] / (rho * 287.0)
+    one, zero = np.ones(shape), np.zeros(shape)
+    s.set_metrics([_dev(a) for a in (one, zero, zero, zero, one, zero, zero, zero, one)], _dev(one))
+    Fp, Fm, F = s.field(5), s.field(5), s.face_field(d)
+    s.fluxSplit(d, _dev(q), Fp, Fm)
+    s.advect(d, F, None, _dev(q))
+    s.close()
+    ax, cut = 3 - d, [slice(None)] + [slice(4, -4)] * 3
+    cut[ax] = slice(None)
+    p, m = (np.moveaxis(a.cpu().numpy()[tuple(cut)], ax, -1).astype(np.longdouble) for a in (Fp, Fm))
+    nf = p.shape[-1] - 7
+    lin = [(u * phi + c * (1 - phi)) / np.longdouble(420) for u, c in zip((-3, 25, -101, 319, 214, -38, 4), (0, 7, -56, 259, 259, -56, 7))]
+    terms = [lin[k] * (p[..., k:k + nf] + m[..., 7 - k:7 - k + nf]) for k in range(7)]
+    got = np.moveaxis(F.cpu().numpy(), ax, -1)
+    # one of the pair is zero, so a sum has seven rounded products and coefficients: 7 + 7 + 2 roundings
+    # of at most the sum of the terms' magnitudes
+    off = np.abs(got - sum(terms)) / (EPS * sum(np.abs(t) for t in terms) + 1e-300)
+    assert off.max() <= 16.0, float(off.max())
