@@ -37,8 +37,9 @@ namespace f3d {
 constexpr int LIN_STRIP = 5;    // faces a strip
 constexpr int LIN_SPREAD = 5;   // largest exponent minus that of a sum's centre
 
-// x 2^(1084 - E) as an integer (E: the strip's largest biased exponent), truncated towards zero
-__device__ __forceinline__ long long fixed_of(double x, int E) {
+// x 2^(1084 - E) as an integer (E: the strip's largest biased exponent), truncated towards zero;
+// below: how many exponents x lies below the largest (a zero: E)
+__device__ __forceinline__ long long fixed_of(double x, int E, int& below) {
     const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
     const int e = (int)((hi >> 20) & 0x7ffu);
     // mantissa with its leading one at bit 63, then right to bit 61 and by the exponent's distance
@@ -46,9 +47,14 @@ __device__ __forceinline__ long long fixed_of(double x, int E) {
     const unsigned long long m =
         ((unsigned long long)(__funnelshift_l(lo, hi, 11) | 0x80000000u) << 32) | (unsigned long long)(lo << 11);
     unsigned long long v;
-    asm("shr.u64 %0, %1, %2;" : "=l"(v) : "l"(m), "r"(E - e + 2));  // shifts past 63 give 0
+    below = E - e;
+    asm("shr.u64 %0, %1, %2;" : "=l"(v) : "l"(m), "r"(below + 2));  // shifts past 63 give 0
     const long long s = (long long)((int)hi >> 31);
     return ((long long)v ^ s) - s;
+}
+__device__ __forceinline__ long long fixed_of(double x, int E) {
+    int below;
+    return fixed_of(x, E, below);
 }
 
 // The FP64 number nearest to (T 2^32 + r) 2^(E - 1084)
@@ -76,19 +82,26 @@ __device__ __forceinline__ double fixed_to_f64(long long T, unsigned r, int E) {
 
 // 12 times the fourth-order central difference, (a - d) - 8 (b - c) for a, b, c, d = f[-2], f[-1], f[1],
 // f[2] (viscous.jl:29-42), rounded once: no FP64 instruction instead of four (the 1/12 goes into a
-// metric factor). Values within 2^9 of the largest enter exactly. `plain` is cleared for values
-// outside 2^-823 .. 2^877 (infinities and NaN among them): the caller then takes difference12_fp64 for
-// all of its differences, in a block of its own (a fallback beside each call is turned into predicated
-// FP64 instructions, which hold the pipe although no lane runs them).
+// metric factor). Values within 2^9 of the largest enter exactly. Smaller ones are truncated: at most 17
+// units of 2^-61 of the largest's power of two, about half a unit in the last place of a result of 2^-4 of
+// it. `plain` is cleared where something was truncated (a zero beside other values is counted in) and
+// the result is smaller than that, the large values having cancelled, and for values outside 2^-823 ..
+// 2^877 (infinities and NaN among them): the caller then takes difference12_fp64 for all of its
+// differences, in a block of its own (a fallback beside each call is turned into predicated FP64
+// instructions, which hold the pipe although no lane runs them). 0.4% of the warps take it on the ramp
+// and the plate.
 __device__ __forceinline__ F64 difference12(double a, double b, double c, double d, bool& plain) {
-    unsigned top = 0u;
-    top = max(max((unsigned)__double2hiint(a) & 0x7fffffffu, (unsigned)__double2hiint(b) & 0x7fffffffu),
-              max((unsigned)__double2hiint(c) & 0x7fffffffu, (unsigned)__double2hiint(d) & 0x7fffffffu));
+    const unsigned top = max(max((unsigned)__double2hiint(a) & 0x7fffffffu, (unsigned)__double2hiint(b) & 0x7fffffffu),
+                             max((unsigned)__double2hiint(c) & 0x7fffffffu, (unsigned)__double2hiint(d) & 0x7fffffffu));
     const int E = (int)(top >> 20);
-    plain = plain && (top == 0u || (E >= 200 && E <= 1900));
-    const long long x = fixed_of(a, E) - fixed_of(d, E), y = fixed_of(b, E) - fixed_of(c, E);  // below 2^63
+    int da, db, dc, dd;
+    const long long x = fixed_of(a, E, da) - fixed_of(d, E, dd), y = fixed_of(b, E, db) - fixed_of(c, E, dc);  // below 2^63
     const long long l = (long long)(unsigned)x - 8ll * (long long)(unsigned)y;
     const double r = fixed_to_f64((x >> 32) - 8ll * (y >> 32) + (l >> 32), (unsigned)l, E);
+    const bool cut = max(max(da, db), max(dc, dd)) > 9;
+    const bool small = ((unsigned)__double2hiint(r) & 0x7fffffffu) < (top & 0x7ff00000u) - (4u << 20);
+    // no branches: twelve of these run side by side
+    plain &= (top == 0u) | (((unsigned)(E - 200) <= 1700u) & !(cut & small));
     return f64(top == 0u ? 0.0 : r);
 }
 __device__ __forceinline__ F64 difference12_fp64(double a, double b, double c, double d) {
@@ -106,6 +119,7 @@ template <class NEAR> __device__ __forceinline__ unsigned beyond_spread(int E, u
         if (near(f) < least) far |= 1u << f;
     return far & want;
 }
+
 // Whether a value enters a strip of exponent E without loss: 2^-9 of the largest or more, or zero
 __device__ __forceinline__ bool enters_exactly(double x, int E) {
     const unsigned a = (unsigned)__double2hiint(x) & 0x7fffffffu;

@@ -8,8 +8,9 @@
 //
 // What bounds it: in FP64 the FP64 pipe (98% busy; 224 bytes a cell would take 0.6 ms on the
 // 512x256x128 ramp). Differences as integers, the metrics times J/12 once and the viscosity through
-// one reciprocal root: 5.8 -> 3.7 ms a stage there, 118 -> 81 us on the plate 125x61x37. 128 threads with the
-// compiler's 126 registers; 102 or 85 registers (5 or 6 blocks per SM) are within 0.3%.
+// one reciprocal root: 5.8 -> 3.7 ms a stage there, 118 -> 81 us on the plate 125x61x37. 128 threads, five
+// blocks per SM (96 registers): the ramp's step 45.1 ms, 45.3 at four blocks (128 registers), 46.6 with the
+// compiler's 138, which the look at cancelled differences asks for (difference12).
 #include "f3d_fixed.cuh"
 
 namespace f3d {
@@ -18,7 +19,7 @@ __device__ __forceinline__ F64 cube_root(F64 x) { return f64(cbrt(x.v)); }
 __device__ __forceinline__ float cube_root(float x) { return cbrtf(x); }
 
 template <class R>
-__global__ void __launch_bounds__(128) k_viscous(const DevParams P, const R* __restrict__ Q, const R* m0,
+__global__ void __launch_bounds__(128, 5) k_viscous(const DevParams P, const R* __restrict__ Q, const R* m0,
                                                  const R* m1, const R* m2, const R* m3, const R* m4, const R* m5,
                                                  const R* m6, const R* m7, const R* m8, const R* __restrict__ J,
                                                  R* Fvx, R* Fvy, R* Fvz) {

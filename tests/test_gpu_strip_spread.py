@@ -157,3 +157,38 @@ def test_linear_faces_beside_large_values(gpu_lib, d, towards, phi):
     # of at most the sum of the terms' magnitudes
     off = np.abs(got - sum(terms)) / (EPS * sum(np.abs(t) for t in terms) + 1e-300)
     assert off.max() <= 16.0, float(off.max())
+
+
+@pytest.mark.parametrize("d", [0, 1, 2])
+@pytest.mark.parametrize("small", [1e-4, 1e-6, 1e-9, 1e-15, 1e-300])
+@pytest.mark.parametrize("inner", [True, False])
+def test_viscous_differences_of_values_that_cancel(gpu_lib, d, small, inner):
+    """f[-2] = f[2] of size one (or f[-1] = f[1]) beside values of size `small`: the large ones cancel in the
+    fourth-order difference, which keeps the accuracy of the small ones."""
+    from flame3d_mhd_gb300.solver import Flame3D
+    n = _box(d, 40, 5)
+    c_s, t_s, T = 1e-2, 1.0, 0.7
+    s = Flame3D(abi.make_params(*n, viscous=1, rg=1.0, c_s=c_s, t_s=t_s, bc=PER))
+    shape = (n[2] + 8, n[1] + 8, n[0] + 8)
+    r = np.random.default_rng(12)
+    f = small * r.uniform(0.5, 1.0, 48) * r.choice([-1.0, 1.0], 48)
+    centres = np.arange(6, 44, 5)
+    for c in centres:
+        k = 1 if inner else 2
+        f[c - k] = f[c + k] = r.uniform(0.5, 1.0)
+    q = np.zeros((6, *shape))
+    q[0], q[5], q[4] = 1.0, T, T
+    q[1 + d] = f.reshape([-1 if a == 2 - d else 1 for a in range(3)])
+    one, zero = np.ones(shape), np.zeros(shape)
+    s.set_metrics([_dev(a) for a in (one, zero, zero, zero, one, zero, zero, zero, one)], _dev(one))
+    F = [s.viscous_field() for _ in range(3)]
+    s.viscousFlux(*F, _dev(q))
+    s.close()
+    # only the normal gradient is there: the normal stress is 4/3 mu times it
+    got = np.moveaxis(F[d].cpu().numpy()[d], 2 - d, -1)[..., centres - 2]
+    v = f.astype(np.longdouble)
+    diff = (v[centres - 2] - v[centres + 2]) - 8 * (v[centres - 1] - v[centres + 1])
+    mu = np.longdouble(c_s) * np.longdouble(T) ** np.longdouble(1.5) / (np.longdouble(T) + t_s)
+    want = mu * diff / 12 * np.longdouble(4) / 3
+    # roundings: the difference 3, viscosity 5, stress and its factors 6
+    assert (np.abs(got - want) <= 16 * EPS * np.abs(want)).all(), float((np.abs(got - want) / np.abs(want)).max() / EPS)
