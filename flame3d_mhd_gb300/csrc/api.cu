@@ -549,7 +549,9 @@ int adjoint_supported(f3d_ctx* ctx) {
 // launch a stage), or, on grids above 2^23 cells, of one after the other to save memory
 size_t sb_planes(const f3d_ctx* ctx) { return ctx->dp.plane <= (1ll << 23) ? 30 : 10; }
 
-int adjoint_alloc(f3d_ctx* ctx) {
+// Allocated by the first reverse call and cleared on its stream: the legacy stream's work is not ordered
+// with a stream that does not wait for it.
+int adjoint_alloc(f3d_ctx* ctx, cudaStream_t st) {
     if (ctx->adj_slab) return F3D_OK;
     const size_t nc = (size_t)ctx->dp.plane;
     const size_t nv = (size_t)(ctx->params.nx + 4) * (ctx->params.ny + 4) * (ctx->params.nz + 4);
@@ -581,7 +583,7 @@ int adjoint_alloc(f3d_ctx* ctx) {
         for (int d = 0; d < 3; d++) { ctx->Fvb[d] = (double*)q; q += 4 * bv; }
         ctx->gb = (double*)q;
     }
-    e = cudaMemset(ctx->adj_slab, 0, total);
+    e = cudaMemsetAsync(ctx->adj_slab, 0, total, st);
     if (e == cudaSuccess) e = adjoint_configure();
     if (e != cudaSuccess) return cuda_fail(ctx, e, "adjoint set-up");
     return F3D_OK;
@@ -892,7 +894,8 @@ int f3d_create(const f3d_params* p, f3d_ctx** out) {
                           !(no_tma && no_tma[0] == '1');
     // phi outside cells 1..Nt-2 is never written; keep it defined (CUDA.zeros in solver.jl:296)
     if ((e = cudaMemset(mx ? (void*)ctx->phi32 : (void*)ctx->phi, 0, phi_bytes)) != cudaSuccess ||
-        (e = cudaMemset(q, 0, 32)) != cudaSuccess || (e = sweep_configure()) != cudaSuccess ||
+        (e = cudaMemset(q, 0, 32)) != cudaSuccess || (e = cudaStreamSynchronize(nullptr)) != cudaSuccess ||  // any stream may be next
+        (e = sweep_configure()) != cudaSuccess ||
         (fvm && (e = fvm_configure()) != cudaSuccess) || (want_tma && (e = sweep_tma_configure()) != cudaSuccess)) {
         cudaFree(ctx->slab);
         if (ctx->extra) cudaFree(ctx->extra);
@@ -1264,8 +1267,8 @@ int f3d_set_inflow_profile(f3d_ctx* ctx, int face, const double* prof, f3d_strea
 int f3d_rhs_vjp(f3d_ctx* ctx, const double* U, const double* Lbar, double* Ubar, f3d_stream stream) {
     int rc = check_ctx(ctx, true);
     if (rc || (rc = check_ptrs(ctx, {U, Lbar, Ubar}))) return rc;
-    if ((rc = adjoint_supported(ctx)) || (rc = adjoint_alloc(ctx))) return rc;
     cudaStream_t st = (cudaStream_t)stream;
+    if ((rc = adjoint_supported(ctx)) || (rc = adjoint_alloc(ctx, st))) return rc;
     F3D_CUDA(ctx, cudaMemsetAsync(Ubar, 0, (size_t)ctx->dp.plane * 5 * sizeof(double), st));
     if ((rc = prep_state(ctx, U, ctx->Qst[0], ctx->cst_[0], ctx->phst[0], st))) return rc;
     const bool mbar = ctx->mbar[0] != nullptr;
@@ -1291,8 +1294,8 @@ int f3d_rk3_step_vjp_stages(f3d_ctx* ctx, double dt, const double* U0, const dou
     if (Ubar == Ubar_next || Ubar == U0) return fail(ctx, F3D_ERR_ARG, "Ubar must not alias U0 or Ubar_next");
     for (double* o : {Ustage, Lbar_stage})
         if (o && (rc = check_ptrs(ctx, {o}))) return rc;
-    if ((rc = adjoint_supported(ctx)) || (rc = adjoint_alloc(ctx))) return rc;
     cudaStream_t st = (cudaStream_t)stream;
+    if ((rc = adjoint_supported(ctx)) || (rc = adjoint_alloc(ctx, st))) return rc;
     const DevParams& P = ctx->dp;
     // forward recompute of the two intermediate stage states U1, U2
     const double* Us[3] = {U0, ctx->U1, ctx->U2};

@@ -1,0 +1,109 @@
+"""What the host side of the library does when the runtime refuses something, and in which order it
+prepares memory: the library's objects linked with a stand-in for the CUDA runtime
+(fake_cudart.cpp), so no GPU is needed and no kernel runs."""
+import ctypes as C
+import subprocess
+from pathlib import Path
+
+import pytest
+
+from flame3d_mhd_gb300 import abi
+from flame3d_mhd_gb300 import build as b
+
+HERE = Path(__file__).resolve().parent
+PER = [dict(kind=abi.BC_PERIODIC)] * 6
+OUT_OF_MEMORY, INVALID = 2, 1  # cudaErrorMemoryAllocation, cudaErrorInvalidValue
+
+
+class Host:
+    """One context on the stand-in runtime; arrays are addresses that nothing reads."""
+
+    def __init__(self, lib, **kw):
+        self.lib, self.P = lib, abi.make_params(20, 12, 8, viscous=0, bc=PER, **kw)
+        lib.fake_reset()
+        self.ctx = C.c_void_p()
+        self.array = (C.c_void_p(0x500000000000 + (k << 24)) for k in range(1 << 20))
+        self.plane = 28 * 20 * 16
+
+    def create(self, ok=True):
+        rc = self.lib.f3d_create(C.byref(self.P), C.byref(self.ctx))
+        assert (rc == 0) == ok
+        return self
+
+    def metrics(self):
+        m = (C.c_void_p * 9)(*[next(self.array) for _ in range(9)])
+        assert self.lib.f3d_set_metrics(self.ctx, m, next(self.array), None) == 0
+        return self
+
+    def rhs(self, stream=0x77):
+        return self.lib.f3d_rhs(self.ctx, next(self.array), next(self.array), C.c_void_p(stream))
+
+    def vjp(self, stream=0x77):
+        a = [next(self.array) for _ in range(3)]
+        return self.lib.f3d_rhs_vjp(self.ctx, *a, C.c_void_p(stream))
+
+    def log(self):
+        """[(what, address, bytes, stream), ...] since the last call"""
+        text = self.lib.fake_log().decode()
+        new, self.seen = text[getattr(self, "seen", 0):], len(text)
+        rows = [r.split() for r in new.splitlines()]
+        return [(r[0], int(r[1], 16), int(r[2]), int(r[3], 16)) for r in rows]
+
+    def close(self):
+        if self.ctx:
+            assert self.lib.f3d_destroy(self.ctx) == 0
+            self.ctx = C.c_void_p()
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    b.build()
+    d = tmp_path_factory.mktemp("fake")
+    inc = Path(b.nvcc()).resolve().parent.parent / "include"
+    so = d / "libhost.so"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-Wl,-Bsymbolic", f"-I{inc}", "-o", str(so),
+                    str(HERE / "fake_cudart.cpp"), *map(str, sorted(b.BUILD.glob("*.o")))], check=True)
+    lib = C.CDLL(str(so))
+    real = abi.load()
+    for name in abi.EXPORTED:
+        getattr(lib, name).restype, getattr(lib, name).argtypes = getattr(real, name).restype, getattr(real, name).argtypes
+    lib.fake_log.restype = C.c_char_p
+    lib.fake_limit.argtypes, lib.fake_held.restype = [C.c_size_t], C.c_size_t
+    lib.fake_refuse.argtypes = [C.c_char_p, C.c_int]
+    yield lib
+    lib.fake_reset()
+
+
+@pytest.fixture
+def host(lib):
+    made = []
+
+    def make(**kw):
+        made.append(Host(lib, **kw))
+        return made[-1]
+    yield make
+    lib.fake_reset()
+    for h in made:
+        h.close()
+
+
+def _launches(rows, name):
+    return [r for r in rows if r[0].startswith("launch:") and name in r[0]]
+
+
+def test_memory_is_cleared_before_any_stream_uses_it(host):
+    """Streams that do not wait for the legacy stream (PyTorch's pool streams) may be the first to use a
+    context: the memory that f3d_create clears is waited for, and the adjoint's, which the first
+    reverse call takes, is cleared on that call's stream."""
+    h = host().create()
+    rows = h.log()
+    cleared = [i for i, r in enumerate(rows) if r[0] == "memset"]
+    waits = [i for i, r in enumerate(rows) if r[0] in ("sync", "sync-device") and r[3] == 0]
+    assert cleared and waits and waits[-1] > cleared[-1]
+    h.metrics().log()
+    assert h.vjp(0x99) == 0
+    rows = h.log()
+    taken = [r for r in rows if r[0] == "malloc"]
+    assert len(taken) == 1
+    sets = [r for r in rows if r[0] == "memset" and taken[0][1] <= r[1] < taken[0][1] + taken[0][2]]
+    assert any(r[2] == taken[0][2] for r in sets) and all(r[3] == 0x99 for r in sets)
