@@ -164,7 +164,9 @@ cudaError_t launch_weno_list(const DevParams& P, const WenoList& w, const double
 cudaError_t launch_weno(const WenoArgs& a, const double* phi, int sms, cudaStream_t st) {
     const long long most = (long long)a.P.nx * a.P.ny * a.P.nz / WF_FACES + 1;
     const int blocks = most < 4 * sms ? (int)most : 4 * sms;
-    launch_weno_list(a.P, a.w, phi, st);
+    // without its lists the faces would be those of the state before
+    const cudaError_t e = launch_weno_list(a.P, a.w, phi, st);
+    if (e != cudaSuccess) return e;
     if (a.P.character) k_weno_faces<true><<<blocks, WF_WARPS * 32, 0, st>>>(a);
     else k_weno_faces<false><<<blocks, WF_WARPS * 32, 0, st>>>(a);
     return cudaGetLastError();

@@ -107,3 +107,17 @@ def test_memory_is_cleared_before_any_stream_uses_it(host):
     assert len(taken) == 1
     sets = [r for r in rows if r[0] == "memset" and taken[0][1] <= r[1] < taken[0][1] + taken[0][2]]
     assert any(r[2] == taken[0][2] for r in sets) and all(r[3] == 0x99 for r in sets)
+
+
+def test_a_refused_list_stops_the_right_hand_side(host):
+    """Without its lists the WENO fluxes would be the previous state's."""
+    h = host().create().metrics()
+    h.log()
+    h.lib.fake_refuse(b"k_weno_list", INVALID)
+    assert h.rhs() == abi.F3D_ERR_CUDA
+    rows = h.log()
+    assert any(r[0].startswith("refused:") for r in rows)
+    assert not _launches(rows, "k_weno_faces") and not _launches(rows, "k_sweep")
+    h.lib.fake_reset()
+    h.seen = 0
+    assert h.rhs() == abi.F3D_OK
