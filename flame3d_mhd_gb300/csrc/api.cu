@@ -356,7 +356,8 @@ SweepArgs sweep_args(f3d_ctx* ctx, int dir, const double* Q, bool hybrid, const 
     return a;
 }
 
-// List the WENO faces of a state and compute their fluxes (k_weno.cu); the sweeps then read them.
+// List the WENO faces of a state and compute their fluxes (k_weno.cu); the sweeps then read them. The
+// state's sensor comes directly before it, and has cleared the counts.
 int list_weno(f3d_ctx* ctx, const double* Q, const double* csnd, const double* phi, cudaStream_t st) {
     if (!ctx->weno.list) return F3D_OK;
     WenoArgs a;
@@ -441,7 +442,7 @@ int run_rhs(f3d_ctx* ctx, const double* Q, double* acc, SweepArgs last, cudaStre
             mark(ctx, K_SOUND, st);
         }
         if (hybrid) {
-            F3D_CUDA(ctx, launch_sensor(P, Q, ctx->phi, st, false, fill_current ? nullptr : ctx->csnd));
+            F3D_CUDA(ctx, launch_sensor(P, Q, ctx->phi, st, false, fill_current ? nullptr : ctx->csnd, ctx->weno.count));
             mark(ctx, K_SENSOR, st);
         }
         if (ctx->params.viscous) {
@@ -559,12 +560,12 @@ int adjoint_alloc(f3d_ctx* ctx, cudaStream_t st) {
     const size_t b1 = up(nc * 8);
     const size_t bv = up(nv * 8);
     const int ncache = ctx->params.adjoint_lean ? 1 : 3;
-    size_t total = b1 * (6 + 5 * 5 + 8 * ncache) + (ctx->weno.list ? up(sb_planes(ctx) * nc * 8) : 0) + (ctx->params.viscous ? bv * (12 + 12) : 0);
+    size_t total = b1 * (6 + 5 * 5 + 8 * ncache) + 256 + (ctx->weno.list ? up(sb_planes(ctx) * nc * 8) : 0) + (ctx->params.viscous ? bv * (12 + 12) : 0);
     cudaError_t e = cudaMalloc(&ctx->adj_slab, total);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc (adjoint scratch)");
     char* q = (char*)ctx->adj_slab;
     if (ctx->weno.list) { ctx->Sb = (double*)q; q += up(sb_planes(ctx) * nc * 8); }
-    ctx->Qb = (double*)q; q += 6 * b1;
+    ctx->Qb = (double*)q; q += 6 * b1 + 256;  // and the counts of the reverse's lists, cleared with it
     ctx->Lt = (double*)q; q += 5 * b1;
     ctx->U1 = (double*)q; q += 5 * b1;
     ctx->U2 = (double*)q; q += 5 * b1;
@@ -593,7 +594,7 @@ int adjoint_alloc(f3d_ctx* ctx, cudaStream_t st) {
 // buffers: everything the RHS and its VJP need from the forward state.
 int prep_state(f3d_ctx* ctx, const double* U, double* Q, double* csnd, double* phi, cudaStream_t st) {
     F3D_CUDA(ctx, launch_prim_fill(ctx->dp, U, Q, nullptr, csnd, 0, st));
-    if (ctx->dp.fixed_branch < 0) F3D_CUDA(ctx, launch_sensor(ctx->dp, Q, phi, st));
+    if (ctx->dp.fixed_branch < 0) F3D_CUDA(ctx, launch_sensor(ctx->dp, Q, phi, st, false, nullptr, ctx->weno.count));
     return F3D_OK;
 }
 
@@ -624,7 +625,7 @@ int rhs_vjp_prepared(f3d_ctx* ctx, const double* U, const double* Q, const doubl
     const bool mbar = ctx->mbar[0] != nullptr;
     const DevParams& P = ctx->dp;
     const bool hybrid = P.fixed_branch < 0;
-    F3D_CUDA(ctx, cudaMemsetAsync(ctx->Qb, 0, (size_t)P.plane * 6 * sizeof(double), st));
+    F3D_CUDA(ctx, cudaMemsetAsync(ctx->Qb, 0, (size_t)P.plane * 6 * sizeof(double) + WENO_COUNTS * sizeof(unsigned), st));
     // the WENO faces from their lists, unless metric cotangents are wanted (formed in the tiles)
     const bool listed = ctx->Sb && !mbar;
     WenoVjpArgs w;
@@ -632,6 +633,7 @@ int rhs_vjp_prepared(f3d_ctx* ctx, const double* U, const double* Q, const doubl
     if (listed) {
         w.P = P;
         w.w = ctx->weno;
+        w.w.count = (unsigned*)(ctx->Qb + 6 * P.plane);
         w.Q = Q;
         w.csnd = csnd;
         w.J = ctx->J;
@@ -643,10 +645,10 @@ int rhs_vjp_prepared(f3d_ctx* ctx, const double* U, const double* Q, const doubl
         for (int d = 0; d < 3; d++) w.S[d] = ctx->S[d];
         w.Qb = ctx->Qb;
         w.Sb = ctx->Sb;
-        w.any = ctx->weno.count + 8;
+        w.any = w.w.count + 8;
         w.d0 = 0;
         w.d1 = 3;
-        F3D_CUDA(ctx, launch_weno_list(P, ctx->weno, phi, st));
+        F3D_CUDA(ctx, launch_weno_list(P, w.w, phi, st));
         if (at_once) F3D_CUDA(ctx, launch_weno_vjp(w, ctx->sms, st));
     }
     for (int d = 0; d < 3; d++) {
@@ -833,8 +835,7 @@ int f3d_create(const f3d_params* p, f3d_ctx** out) {
         ctx->weno.count = (unsigned*)w;
         ctx->weno.list = (int*)(w + 256);
         ctx->weno.flux = (double*)(w + 256 + bl);
-        if ((e = cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->device)) == cudaSuccess)
-            e = cudaMemset(w, 0, 256);
+        e = cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->device);
         total = up(total) + lists;
     }
     if (e != cudaSuccess) {

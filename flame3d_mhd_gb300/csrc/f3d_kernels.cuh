@@ -39,8 +39,10 @@ inline cudaError_t launch_after(const DevParams& P, void (*kernel)(Params...), u
 enum OutMode { OUT_SET = 0, OUT_ADD = 1, OUT_RHS = 2, OUT_STAGE = 3, OUT_FACES = 4 };
 
 // The listed WENO faces of a state (k_weno.cu): one list of `plane` left-cell indices a direction,
-// WENO7 faces from its front and WENO5 faces from its back, their six counts (and the finished
-// blocks of k_weno_faces), and the fluxes, five planes a direction.
+// WENO7 faces from its front and WENO5 faces from its back, their six counts (WENO_COUNTS words, zero
+// before a listing: a listing that finds those of one whose later kernels were refused would
+// append behind it and run out of the arrays), and the fluxes, five planes a direction.
+constexpr int WENO_COUNTS = 16;  // six counts, and from word 8 three flags of the reverse
 struct WenoList {
     int* list;
     unsigned* count;
@@ -217,9 +219,10 @@ cudaError_t launch_prim2c(const DevParams& P, const double* Q, double* U, cudaSt
 cudaError_t launch_lincomb(const DevParams& P, double* U, const double* Un, double a, double b, cudaStream_t st);
 cudaError_t launch_sound(const DevParams& P, const double* Q, double* csnd, cudaStream_t st);
 // exact: phi bit for bit as the oracle's; otherwise values that give the same branch map
-// (FP32 away from the thresholds, FP64 near them); csnd: also the split's sound speed (not exact)
+// (FP32 away from the thresholds, FP64 near them); csnd: also the split's sound speed (not exact);
+// counts: also clear the counts of the lists that are made from phi (not exact)
 cudaError_t launch_sensor(const DevParams& P, const double* Q, double* phi, cudaStream_t st, bool exact = false,
-                          double* csnd = nullptr);
+                          double* csnd = nullptr, unsigned* counts = nullptr);
 cudaError_t launch_metric_prep(const DevParams& P, const double* const m[9], double* S[3], double* Ah[9],
                                cudaStream_t st);
 cudaError_t launch_split_debug(const DevParams& P, const double* Q, const double* csnd, const double* const A[3],

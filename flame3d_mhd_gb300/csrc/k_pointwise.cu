@@ -276,9 +276,10 @@ __device__ __forceinline__ double sensor_term(double a, double b, double c) {
 // the branch map is the FP64 sensor's, with three FP64 divisions saved at almost every cell.
 // csnd (optional): the split's sound speed of every cell is formed here too, for a right-hand side
 // whose state no primitive fill has prepared (one launch and one pass over p and T less).
-template <bool EXACT> __global__ void k_sensor(const DevParams P, const double* Q, double* phi, double* csnd) {
+template <bool EXACT> __global__ void k_sensor(const DevParams P, const double* Q, double* phi, double* csnd, unsigned* counts) {
     after_previous();
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (!EXACT && counts && c < WENO_COUNTS) counts[c] = 0u;
     if (c >= P.plane) return;
     if (!EXACT && csnd) {
         double q[6];
@@ -311,9 +312,10 @@ template <bool EXACT> __global__ void k_sensor(const DevParams P, const double* 
     double fz = sensor_term(pzm, pc, pzp);
     phi[c] = __dadd_rn(__dadd_rn(fx, fy), fz);
 }
-cudaError_t launch_sensor(const DevParams& P, const double* Q, double* phi, cudaStream_t st, bool exact, double* csnd) {
-    if (exact) k_sensor<true><<<pw_blocks(P.plane), PW_THREADS, 0, st>>>(P, Q, phi, nullptr);
-    else launch_after(P, k_sensor<false>, pw_blocks(P.plane), PW_THREADS, st, P, Q, phi, csnd);
+cudaError_t launch_sensor(const DevParams& P, const double* Q, double* phi, cudaStream_t st, bool exact, double* csnd,
+                          unsigned* counts) {
+    if (exact) k_sensor<true><<<pw_blocks(P.plane), PW_THREADS, 0, st>>>(P, Q, phi, nullptr, nullptr);
+    else launch_after(P, k_sensor<false>, pw_blocks(P.plane), PW_THREADS, st, P, Q, phi, csnd, counts);
     return cudaGetLastError();
 }
 

@@ -8,7 +8,8 @@
 // sub-core then bounds the tile). Here they are listed first and then spread evenly:
 //   k_weno_list   one thread per cell: the branch of the faces on its upper side in the three
 //                 directions (from the shock sensor, as the sweeps decide it); WENO faces are
-//                 appended to one list a direction, WENO7 from its front and WENO5 from its back;
+//                 appended to one list a direction, WENO7 from its front and WENO5 from its back. The
+//                 counts must be zero: the sensor's kernel, which every listing follows, clears them;
 //   k_weno_faces  blocks of five warps take 32 faces of one list at a time: the warps split the
 //                 eight stencil cells (one cell of 32 faces a warp) and form the face bases, then
 //                 take one characteristic field (or component) each, then one flux component each.
@@ -142,14 +143,6 @@ __global__ void __launch_bounds__(WF_WARPS * 32, 4) k_weno_faces(const WenoArgs 
                 *out = char_right_row<F64>(sm.basis[lane], wp, flux).v;
             }
             __syncthreads();
-        }
-    }
-    // the last block to finish clears the counts for the next lists (every block has read them)
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(&w.count[6], 1u) == gridDim.x - 1) {
-#pragma unroll
-            for (int li = 0; li < 7; li++) w.count[li] = 0u;
         }
     }
 }

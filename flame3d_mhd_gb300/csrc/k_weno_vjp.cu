@@ -349,14 +349,6 @@ __global__ void __launch_bounds__(WV_WARPS * 32, 3) k_weno_vjp(const WenoVjpArgs
         }
         __syncthreads();
     }
-    // with the last direction the last block clears the counts (every block has read its own by then)
-    if (a.d1 == 3 && threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(&a.w.count[6], 1u) == gridDim.x - 1) {
-#pragma unroll
-            for (int li = 0; li < 7; li++) a.w.count[li] = 0u;
-        }
-    }
 }
 
 cudaError_t weno_vjp_configure() {

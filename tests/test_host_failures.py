@@ -121,3 +121,26 @@ def test_a_refused_list_stops_the_right_hand_side(host):
     h.lib.fake_reset()
     h.seen = 0
     assert h.rhs() == abi.F3D_OK
+
+
+def test_lists_start_from_zero_after_a_refused_launch(host):
+    """The counts of a listing whose later kernels were refused are cleared before the next one: lists
+    appended behind them would run out of their arrays."""
+    h = host().create().metrics()
+    for call, refused in ((h.rhs, b"k_weno_faces"), (h.vjp, b"k_weno_vjp"), (h.vjp, b"k_sweep_vjp")):
+        h.lib.fake_refuse(refused, INVALID)
+        assert call() == abi.F3D_ERR_CUDA
+        h.lib.fake_refuse(b"", 0)
+        h.log()
+        assert h.rhs() == abi.F3D_OK and h.vjp() == abi.F3D_OK
+        clean, lists = set(), 0
+        for what, at, size, _ in h.log():
+            if what == "clears":
+                clean.add(at)
+            elif what == "memset":
+                clean |= {at + k for k in range(0, size, 8)}
+            elif what == "counts":
+                assert at in clean, hex(at)
+                clean.discard(at)  # the listing that follows uses them
+                lists += 1
+        assert lists == 2
