@@ -242,7 +242,8 @@ struct f3d_ctx {
     void* adj_slab = nullptr;
     double *Qb = nullptr, *Lt = nullptr, *U1 = nullptr, *U2 = nullptr, *Xb = nullptr, *Yb = nullptr;
     double *Qst[3] = {}, *cst_[3] = {}, *phst[3] = {};  // Q, sound speed and sensor of the stage states
-    double* Sb = nullptr;  // split-flux cotangents of the listed WENO faces (10 planes, zero between calls)
+    double* Sb = nullptr;  // split-flux cotangents of the listed WENO faces (sb_planes, zero between calls)
+    bool Sb_clean = true;  // false from the first launch that writes Sb until the last one that clears it
     double *Fvb[3] = {}, *gb = nullptr;
     // metric and Jacobian cotangents (borrowed; f3d_set_metrics_cotangent) and the forward
     // RHS of the first two stage states kept for the Jacobian's term (10 arrays, owned)
@@ -646,6 +647,8 @@ int rhs_vjp_prepared(f3d_ctx* ctx, const double* U, const double* Q, const doubl
         w.Qb = ctx->Qb;
         w.Sb = ctx->Sb;
         w.any = w.w.count + 8;
+        if (!ctx->Sb_clean) F3D_CUDA(ctx, cudaMemsetAsync(ctx->Sb, 0, sb_planes(ctx) * P.plane * sizeof(double), st));
+        ctx->Sb_clean = false;
         w.d0 = 0;
         w.d1 = 3;
         F3D_CUDA(ctx, launch_weno_list(P, w.w, phi, st));
@@ -681,6 +684,7 @@ int rhs_vjp_prepared(f3d_ctx* ctx, const double* U, const double* Q, const doubl
         }
         F3D_CUDA(ctx, launch_sweep_vjp(d, a, st));
     }
+    ctx->Sb_clean = true;
     if (ctx->params.viscous)
         F3D_CUDA(ctx, launch_viscous_vjp(P, Q, ctx->m, ctx->J, Lb, ctx->Fvb, ctx->gb, ctx->Qb, st,
                                          mbar ? ctx->mbar : nullptr, ctx->Jbar, alpha));

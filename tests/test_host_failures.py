@@ -144,3 +144,20 @@ def test_lists_start_from_zero_after_a_refused_launch(host):
                 clean.discard(at)  # the listing that follows uses them
                 lists += 1
         assert lists == 2
+
+
+def test_split_cotangents_start_from_zero_after_a_refused_launch(host):
+    """The reverse sweeps clear the split-flux cotangents they read; where one of them was refused, the next
+    reverse call clears them all first (and only then)."""
+    h = host().create().metrics()
+    planes = 30 * h.plane * 8
+    cleared = lambda: sum(r[0] == "memset" and r[2] == planes for r in h.log())  # noqa: E731
+    assert h.vjp() == abi.F3D_OK and cleared() == 0
+    assert h.vjp() == abi.F3D_OK and cleared() == 0
+    for refused in (b"k_weno_vjp", b"k_sweep_vjp"):
+        h.lib.fake_refuse(refused, INVALID)
+        assert h.vjp() == abi.F3D_ERR_CUDA
+        h.lib.fake_refuse(b"", 0)
+        h.log()
+        assert h.vjp() == abi.F3D_OK and cleared() == 1
+        assert h.vjp() == abi.F3D_OK and cleared() == 0
