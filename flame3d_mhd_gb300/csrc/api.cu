@@ -278,6 +278,7 @@ int fail(f3d_ctx* ctx, int code, const std::string& msg) {
 }
 
 int cuda_fail(f3d_ctx* ctx, cudaError_t e, const char* where) {
+    cudaGetLastError();  // reported here: not again by the next call's launches
     return fail(ctx, F3D_ERR_CUDA, std::string(where) + ": " + cudaGetErrorString(e));
 }
 
@@ -561,11 +562,28 @@ int adjoint_alloc(f3d_ctx* ctx, cudaStream_t st) {
     const size_t b1 = up(nc * 8);
     const size_t bv = up(nv * 8);
     const int ncache = ctx->params.adjoint_lean ? 1 : 3;
-    size_t total = b1 * (6 + 5 * 5 + 8 * ncache) + 256 + (ctx->weno.list ? up(sb_planes(ctx) * nc * 8) : 0) + (ctx->params.viscous ? bv * (12 + 12) : 0);
-    cudaError_t e = cudaMalloc(&ctx->adj_slab, total);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc (adjoint scratch)");
+    const size_t total = b1 * (6 + 5 * 5 + 8 * ncache) + 256 + (ctx->params.viscous ? bv * (12 + 12) : 0);
+    const size_t sb = ctx->weno.list ? up(sb_planes(ctx) * nc * 8) : 0;
+    size_t taken = total + sb;
+    cudaError_t e = cudaMalloc(&ctx->adj_slab, taken);
+    if (e != cudaSuccess && sb) {  // no room for Sb: the tiles reverse their WENO faces
+        cudaGetLastError();
+        taken = total;
+        e = cudaMalloc(&ctx->adj_slab, taken);
+    }
+    if (e != cudaSuccess) {
+        ctx->adj_slab = nullptr;
+        return cuda_fail(ctx, e, "cudaMalloc (adjoint scratch)");
+    }
+    e = cudaMemsetAsync(ctx->adj_slab, 0, taken, st);
+    if (e == cudaSuccess) e = adjoint_configure();
+    if (e != cudaSuccess) {
+        cudaFree(ctx->adj_slab);
+        ctx->adj_slab = nullptr;
+        return cuda_fail(ctx, e, "adjoint set-up");
+    }
     char* q = (char*)ctx->adj_slab;
-    if (ctx->weno.list) { ctx->Sb = (double*)q; q += up(sb_planes(ctx) * nc * 8); }
+    if (taken > total) { ctx->Sb = (double*)q; q += sb; }
     ctx->Qb = (double*)q; q += 6 * b1 + 256;  // and the counts of the reverse's lists, cleared with it
     ctx->Lt = (double*)q; q += 5 * b1;
     ctx->U1 = (double*)q; q += 5 * b1;
@@ -585,9 +603,6 @@ int adjoint_alloc(f3d_ctx* ctx, cudaStream_t st) {
         for (int d = 0; d < 3; d++) { ctx->Fvb[d] = (double*)q; q += 4 * bv; }
         ctx->gb = (double*)q;
     }
-    e = cudaMemsetAsync(ctx->adj_slab, 0, total, st);
-    if (e == cudaSuccess) e = adjoint_configure();
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "adjoint set-up");
     return F3D_OK;
 }
 
@@ -843,6 +858,7 @@ int f3d_create(const f3d_params* p, f3d_ctx** out) {
         total = up(total) + lists;
     }
     if (e != cudaSuccess) {
+        cudaGetLastError();
         if (ctx->slab) cudaFree(ctx->slab);
         if (ctx->extra) cudaFree(ctx->extra);
         delete ctx;

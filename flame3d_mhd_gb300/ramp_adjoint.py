@@ -266,8 +266,9 @@ def main(argv=None):
         used = total - free
         # stage states and cotangents (6), the reversal's Un, Q (6/5) and step scratch, the
         # cotangent, the final state, the two RHS buffers of the angle term, the objective's
-        # source term, the angle term's Q and the forward pass's Un, Q: 19 states of headroom
-        reserve = 19 * state_b
+        # source term, the angle term's Q and the forward pass's Un, Q: 19 states of headroom; and
+        # the split-flux cotangents of listed WENO faces (30 planes, 10 above 2^23 cells)
+        reserve = (19 + (6 if R.U0[0].numel() <= 1 << 23 else 2)) * state_b
         slots = int((a.hbm_gb * 1e9 - used - reserve) // state_b)
         if slots < 2:
             raise SystemExit(f"--hbm-gb {a.hbm_gb} leaves no room for trajectory states ({used / 1e9:.1f} GB used)")

@@ -19,7 +19,7 @@ class Host:
     """One context on the stand-in runtime; arrays are addresses that nothing reads."""
 
     def __init__(self, lib, **kw):
-        self.lib, self.P = lib, abi.make_params(20, 12, 8, viscous=0, bc=PER, **kw)
+        self.lib, self.P = lib, abi.make_params(20, 12, 8, bc=PER, **{"viscous": 0, **kw})
         lib.fake_reset()
         self.ctx = C.c_void_p()
         self.array = (C.c_void_p(0x500000000000 + (k << 24)) for k in range(1 << 20))
@@ -161,3 +161,39 @@ def test_split_cotangents_start_from_zero_after_a_refused_launch(host):
         h.log()
         assert h.vjp() == abi.F3D_OK and cleared() == 1
         assert h.vjp() == abi.F3D_OK and cleared() == 0
+
+
+@pytest.mark.parametrize("viscous", [0, 1])
+def test_reverse_without_room_for_the_listed_faces(host, viscous):
+    """Where the device has room for the adjoint's scratch, but not for the split-flux cotangents of listed WENO
+    faces beside it, the reverse runs with its WENO faces in the tiles; with less it is refused, and runs
+    once there is room."""
+    h = host(viscous=viscous)
+    h.create().metrics()
+    need = 8 * (h.plane * (6 + 25 + 24) + (24 * 16 * 12 * 24 if viscous else 0))
+    spare = 64 * 1024  # rounding of the arrays
+    h.lib.fake_limit(h.lib.fake_held() + need // 2)
+    assert h.vjp() == abi.F3D_ERR_CUDA
+    assert h.rhs() == abi.F3D_OK  # the refusal is not reported again
+    h.lib.fake_limit(h.lib.fake_held() + need + spare)
+    h.log()
+    assert h.vjp() == abi.F3D_OK
+    rows = h.log()
+    assert not _launches(rows, "k_weno_vjp")
+    assert len([r for r in _launches(rows, "k_sweep_vjp") if "ELi1EE" in r[0]]) == 3  # characteristic faces in the tiles
+    assert h.vjp() == abi.F3D_OK
+
+
+def test_right_hand_side_without_room_for_the_lists(host):
+    """A context whose lists do not fit keeps its WENO faces in the tiles."""
+    h = host().create()
+    full = h.lib.fake_held()
+    h.close()
+    h.lib.fake_limit(full - 1)
+    h.create().metrics().log()
+    assert h.lib.fake_held() < full - 100 * h.plane
+    h.lib.fake_limit(1 << 40)
+    assert h.rhs() == abi.F3D_OK and h.vjp() == abi.F3D_OK
+    rows = h.log()
+    assert not _launches(rows, "k_weno")
+    assert len([r for r in _launches(rows, "k_sweepIL") if "ELi1EdE" in r[0]]) == 3
