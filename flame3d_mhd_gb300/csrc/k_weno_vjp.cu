@@ -20,7 +20,9 @@ namespace f3d {
 // Reverse of one side of WENO7 in the forms of weno7_sums (f3d_flux.cuh): V(k) the stencil, g the
 // cotangent of 12 times its value; returns 12 times the value, Vb the stencil's cotangents.
 // With w_k = alpha_k / D the value's cotangents are q_k: g w_k, and through the bases b_k = t_k^2,
-// t_k = e_k + sigma_k I_k: I_k-bar = -2 sigma_k g w_k (q_k - N/D) / t_k.
+// t_k = e_k + sigma_k I_k: I_k-bar = -2 sigma_k g w_k (q_k - N/D) / t_k. The weights and 1 / t_k come from
+// products of the b_k and one reciprocal of them all; where that product leaves the range (t above ~1e38,
+// fluxes above ~1e18) from four quotients instead, which hold to t ~ 1e154.
 __device__ __forceinline__ F64 weno7_reverse(const F64 v[7], F64 s0, F64 g, F64 Vb[7]) {
     using C = W7Ldl<double>;
     const double rw[4] = {1.0, 0.28867513459481287, 0.23570226039551584, 0.5};  // 1 / sqrt(1, 12, 18, 4)
@@ -40,9 +42,20 @@ __device__ __forceinline__ F64 weno7_reverse(const F64 v[7], F64 s0, F64 g, F64 
     }
     const F64 q[4] = {F64(13.0) * d[2] + F64(-10.0) * d[1] + F64(3.0) * d[0], (F64(4.0) * d[2] - d[1]) + F64(3.0) * d[3],
                       (F64(6.0) * d[3] + d[2]) - d[4], (F64(-4.0) * d[4] + d[5]) + F64(9.0) * d[3]};
-    const F64 p01 = b[0] * b[1], p23 = b[2] * b[3];
-    const F64 al[4] = {p23 * b[1], p23 * b[0], p01 * b[3], p01 * b[2]};
-    const F64 rD = recip(al[0] + al[1] + al[2] + al[3]), rP = recip(p01 * p23);
+    const F64 p01 = b[0] * b[1], p23 = b[2] * b[3], all = p01 * p23;
+    F64 al[4] = {p23 * b[1], p23 * b[0], p01 * b[3], p01 * b[2]}, it[4];  // alpha_k and 1 / t_k
+    if (recip_range(all.v)) {
+        const F64 rP = recip_step(all.v);
+#pragma unroll
+        for (int k = 0; k < 4; k++) it[k] = t[k] * (al[k] * rP);  // t_k / b_k
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            it[k] = f64(1.0 / t[k].v);
+            al[k] = it[k] * it[k];
+        }
+    }
+    const F64 rD = recip(al[0] + al[1] + al[2] + al[3]);
     const F64 Q = (al[0] * q[0] + al[1] * q[1] + al[2] * q[2] + al[3] * q[3]) * rD;
     const F64 gm = F64(-2.0) * g;
     F64 qb[4], db[6];
@@ -52,8 +65,7 @@ __device__ __forceinline__ F64 weno7_reverse(const F64 v[7], F64 s0, F64 g, F64 
     for (int k = 0; k < 4; k++) {
         const F64 w = al[k] * rD;
         qb[k] = g * w;
-        // 1 / t_k = t_k / b_k = t_k alpha_k / (b_0 b_1 b_2 b_3)
-        const F64 Ib = ((gm * sg[k]) * (w * (q[k] - Q))) * (t[k] * (al[k] * rP));
+        const F64 Ib = ((gm * sg[k]) * (w * (q[k] - Q))) * it[k];
         const F64 h = Ib + Ib, y1b = y1[k] * h, y2b = z2[k] * h;
         db[k] += y1b;
         db[k + 1] = (db[k + 1] + y2b) + F64(C::a(k)) * y1b;
@@ -89,8 +101,20 @@ __device__ __forceinline__ F64 weno5_reverse(const F64 v[5], F64 s0, F64 g, F64 
         b[k] = t[k] * t[k];
     }
     const F64 q[3] = {F64(5.0) * d[1] + F64(-2.0) * d[0], d[1] + F64(2.0) * d[2], F64(4.0) * d[2] - d[3]};
-    const F64 al[3] = {b[1] * b[2], b[0] * b[2], b[0] * b[1]};
-    const F64 rD = recip(al[0] + al[1] + al[2]), rP = recip(al[0] * b[0]);
+    const F64 all = b[0] * b[1] * b[2];
+    F64 al[3] = {b[1] * b[2], b[0] * b[2], b[0] * b[1]}, it[3];
+    if (recip_range(all.v)) {
+        const F64 rP = recip_step(all.v);
+#pragma unroll
+        for (int k = 0; k < 3; k++) it[k] = t[k] * (al[k] * rP);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            it[k] = f64(1.0 / t[k].v);
+            al[k] = it[k] * it[k];
+        }
+    }
+    const F64 rD = recip(al[0] + al[1] + al[2]);
     const F64 Q = (al[0] * q[0] + al[1] * q[1] + al[2] * q[2]) * rD;
     const F64 gm = F64(-2.0) * g;
     F64 qb[3], sb[3], fb[3];
@@ -98,7 +122,7 @@ __device__ __forceinline__ F64 weno5_reverse(const F64 v[5], F64 s0, F64 g, F64 
     for (int k = 0; k < 3; k++) {
         const F64 w = al[k] * rD;
         qb[k] = g * w;
-        const F64 Ib = ((gm * sg[k]) * (w * (q[k] - Q))) * (t[k] * (al[k] * rP));
+        const F64 Ib = ((gm * sg[k]) * (w * (q[k] - Q))) * it[k];
         const F64 h = Ib + Ib;
         sb[k] = (k13 * s[k]) * h;
         fb[k] = f[k] * h;
