@@ -284,11 +284,16 @@ __global__ void __launch_bounds__(WV_WARPS * 32, 3) k_weno_vjp(const WenoVjpArgs
                 fb = sm.Fb[wp * WV_FACES + lane];
             }
             const F64 g = fb * unit;
+            // a component without a cotangent has none to pass on, whatever its stencil holds
+            const bool none = !CHAR && (__double_as_longlong(fb.v) << 1) == 0;
+            if (none)
+#pragma unroll
+                for (int k = 0; k < 14; k++) sm.Vb[(wp * 14 + k) * WV_FACES + lane] = f64(0.0);
             F64 lb[5], both = f64(0.0);
 #pragma unroll
             for (int e = 0; e < 5; e++) lb[e] = f64(0.0);
 #pragma unroll 1
-            for (int side = 0; side < 2; side++) {
+            for (int side = none ? 2 : 0; side < 2; side++) {
                 const double* f = sm.f + (side == 0 ? 0 : 40 * WV_FACES) + lane;
                 // upwind order: position k of the plus side, 7 - k of the minus side
                 auto at = [&](int k) { return (side == 0 ? k : 7 - k) * WV_FACES; };
@@ -350,7 +355,7 @@ __global__ void __launch_bounds__(WV_WARPS * 32, 3) k_weno_vjp(const WenoVjpArgs
                     } else {
                         v = sm.Vb[(wp * 14 + side * 7 + k) * WV_FACES + lane];
                     }
-                    atomicAdd(Sb + ((side == 0 ? k : 7 - k) - 3) * stride, v.v);
+                    if (__double_as_longlong(v.v) << 1) atomicAdd(Sb + ((side == 0 ? k : 7 - k) - 3) * stride, v.v);
                 }
             }
             if (CHAR && wp == ch % WV_WARPS) {

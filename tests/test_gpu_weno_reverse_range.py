@@ -63,3 +63,27 @@ def test_reverse_of_large_and_small_fluxes(gpu_lib, which, character, size):
     # as for sizes of order one: both are sums of the same rounded products in another order
     for a, b in zip(listed, tiles):
         assert (a - b).abs().max() <= 1e-11 * b.abs().max()
+
+
+@pytest.mark.parametrize("which", sorted(THRESHOLDS))
+@pytest.mark.parametrize("component", [None, 1])
+def test_no_cotangent_beside_non_finite_values(gpu_lib, which, component):
+    """Component-wise faces whose cotangent is zero pass nothing on, also where the state is not finite."""
+    import torch
+    n = (40, 9, 6)
+    s = _solver(n, which, 0)
+    U, Lbar = _case(s, n, 1.0)
+    U[1, 8, 8, 12] = U[2, 8, 9, 30] = 1e200  # pressures at their floor, so the faces stay WENO; fluxes overflow
+    if component is None:
+        Lbar[..., 4:28] = 0.0  # a masked objective: only the right part of the grid counts
+    else:
+        keep = Lbar[component].clone()
+        Lbar.zero_()
+        Lbar[component, ..., 28:44] = keep[..., 28:44]
+    listed, tiles = _both(s, U, Lbar)
+    s.close()
+    fin = torch.isfinite(tiles)
+    assert not fin.all() and fin[:, 4:-4, 4:-4, 4:-4].any()
+    # (the lists' quotients hold where the tiles' products overflow: more of their values may be finite)
+    assert torch.isfinite(listed[fin]).all()
+    assert (listed[fin] - tiles[fin]).abs().max() <= 1e-11 * tiles[fin].abs().max()
