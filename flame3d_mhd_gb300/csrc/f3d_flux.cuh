@@ -255,14 +255,23 @@ __device__ __forceinline__ double weno7_ref32(float V1, float V2, float V3, floa
     weno7_parts<float>(V1, V2, V3, V4, V5, V6, V7, q, Is);
     // alpha_k over their common denominator (one FP64 division a side instead of five): the
     // reference's values to within FP64 rounding, far below the Float32 the result is rounded to.
-    // Bases from 1e-20 to 3e38: the triple products stay within 1e-120 .. 1e231. Plain double
-    // expressions: branches here change how the compiler contracts the mixed form's FP32 faces in
-    // the same kernels
+    // Bases from 1e-20 to 3e38: the triple products stay within 1e-120 .. 1e231. An indicator beyond
+    // Float32's range has an alpha of zero, as the quotient gives it: it is left out of the others'
+    // products. Plain double expressions and selections: branches here change how the compiler
+    // contracts the mixed form's FP32 faces in the same kernels
     const double e1 = 1e-20;
-    const double b1 = sq(e1 + (double)(Is[0] * s0)), b2 = sq(e1 + (double)(Is[1] * s0));
-    const double b3 = sq(e1 + (double)(Is[2] * s0)), b4 = sq(e1 + (double)(Is[3] * s0));
-    const double p12 = b1 * b2, p34 = b3 * b4;
-    const double a1 = b2 * p34, a2 = 12.0 * b1 * p34, a3 = 18.0 * p12 * b4, a4 = 4.0 * p12 * b3;
+    const float x[4] = {Is[0] * s0, Is[1] * s0, Is[2] * s0, Is[3] * s0};
+    double b[4], w[4] = {0.0, 12.0, 18.0, 4.0};
+    bool first = false;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const bool over = (__float_as_uint(x[k]) & 0x7fffffffu) == 0x7f800000u;
+        b[k] = over ? 1.0 : sq(e1 + (double)x[k]);
+        w[k] = over ? 0.0 : w[k];
+        if (k == 0) first = over;
+    }
+    const double p12 = b[0] * b[1], p34 = b[2] * b[3];
+    const double a1 = first ? 0.0 : b[1] * p34, a2 = w[1] * b[0] * p34, a3 = w[2] * p12 * b[3], a4 = w[3] * p12 * b[2];
     return (a1 * (double)q[0] + a2 * (double)q[1] + a3 * (double)q[2] + a4 * (double)q[3]) / (a1 + a2 + a3 + a4);
 }
 // WENO5 in Float32 with one division per alpha and one for their sum (schemes.jl:233-252).
