@@ -29,24 +29,20 @@ static int fixed_branch_of(const f3d_params& p) {
     return -1;
 }
 
-// The linear coefficients as integers over a common denominator D (f3d_fixed.cuh): 420 m with
-// the smallest m <= 500 that makes 420 m (up7_420 phi + cd6_420 (1 - phi)) whole for the given blend
-// (m = 1 for phi = 0 and 1, 2 for 0.5, 10 for 0.9, ...), with the signs of a blend in [0, 1] and
-// 32-bit accumulations' room (sum |c| < 2^20).
+// The linear coefficients as integers over a common denominator D = 420 m (f3d_fixed.cuh): with a blend
+// phi = k / (3 m) they are (cd6 m + (up7 - cd6) k / 3) / (420 m), up7 - cd6 being whole multiples of three.
+// The smallest m <= 500 (1 for phi = 0 and 1, 2 for 0.5, 10 for 0.9, ...) whose quotient is phi to the last
+// bit of numbers near one, which is less than the coefficients' own rounding; a blend that is only near such a
+// quotient keeps the FP64 sums. In [0, 1] the signs are those of up7, and 32-bit accumulations have room
+// (sum |c| < 2^20).
 static void integer_coefficients(double phi, DevParams& d) {
-    const double up7_420[7] = {-3, 25, -101, 319, 214, -38, 4}, cd6_420[7] = {0, 7, -56, 259, 259, -56, 7};
+    const int cd6_420[7] = {0, 7, -56, 259, 259, -56, 7}, third[7] = {-1, 6, -15, 20, -15, 6, -1};
     d.lin_int = 0;
     if (!(phi >= 0.0 && phi <= 1.0)) return;
     for (int m = 1; m <= 500; m++) {
-        int c[7];
-        bool whole = true;
-        for (int k = 0; k < 7; k++) {
-            const double v = m * (up7_420[k] * phi + cd6_420[k] * (1.0 - phi)), r = std::nearbyint(v);
-            c[k] = (int)r;
-            whole = whole && std::fabs(v - r) <= 1e-12 * m;
-        }
-        if (!whole) continue;
-        for (int k = 0; k < 7; k++) d.lin_c[k] = c[k];
+        const int k = (int)std::nearbyint(3.0 * m * phi);
+        if (std::fabs(phi - k / (3.0 * m)) > 0x1p-53) continue;
+        for (int n = 0; n < 7; n++) d.lin_c[n] = cd6_420[n] * m + third[n] * k;
         d.lin_s = 1.0 / (420.0 * m);
         d.lin_int = 1;
         return;

@@ -192,3 +192,39 @@ def test_viscous_differences_of_values_that_cancel(gpu_lib, d, small, inner):
     want = mu * diff / 12 * np.longdouble(4) / 3
     # roundings: the difference 3, viscosity 5, stress and its factors 6
     assert (np.abs(got - want) <= 16 * EPS * np.abs(want)).all(), float((np.abs(got - want) / np.abs(want)).max() / EPS)
+
+
+@pytest.mark.parametrize("d", [0, 1, 2])
+@pytest.mark.parametrize("parity", [0, 1])
+@pytest.mark.parametrize("phi", [0.5 + 1.6e-14, 0.9 - 1.6e-14, 1.0 - 1.6e-14, 1.6e-14, 0.3, 0.1 + 0.2])
+def test_linear_faces_of_a_blend_near_a_small_denominator(gpu_lib, d, parity, phi):
+    """A blend 1.6e-14 away from a quotient of small numbers is not that quotient: a supersonic gas whose
+    density alternates from cell to cell, in which the two schemes' difference is largest."""
+    from flame3d_mhd_gb300.solver import Flame3D
+    n = _box(d, 64)
+    s = Flame3D(abi.make_params(*n, viscous=0, linear_phi=phi, bc=PER, **LINEAR))
+    shape = (n[2] + 8, n[1] + 8, n[0] + 8)
+    r = np.random.default_rng(10)
+    odd = (np.arange(shape[2 - d]) % 2 == parity).reshape([-1 if a == 2 - d else 1 for a in range(3)])
+    q = np.zeros((6, *shape))
+    q[0] = np.where(odd, 1.0, 2.0 ** -20) * r.uniform(1.0, 1.01, shape)
+    q[1 + d] = 3.0
+    q[4] = q[0] / 1.4
+    q[5] = q[4] / (q[0] * 287.0)
+    one, zero = np.ones(shape), np.zeros(shape)
+    s.set_metrics([_dev(a) for a in (one, zero, zero, zero, one, zero, zero, zero, one)], _dev(one))
+    Fp, Fm, F = s.field(5), s.field(5), s.face_field(d)
+    s.fluxSplit(d, _dev(q), Fp, Fm)
+    s.advect(d, F, None, _dev(q))
+    s.close()
+    ax, cut = 3 - d, [slice(None)] + [slice(4, -4)] * 3
+    cut[ax] = slice(None)
+    p, m = (np.moveaxis(a.cpu().numpy()[tuple(cut)], ax, -1).astype(np.longdouble) for a in (Fp, Fm))
+    nf = p.shape[-1] - 7
+    e = np.longdouble(phi)
+    lin = [(u * e + c * (1 - e)) / np.longdouble(420) for u, c in zip((-3, 25, -101, 319, 214, -38, 4), (0, 7, -56, 259, 259, -56, 7))]
+    terms = [lin[k] * (p[..., k:k + nf] + m[..., 7 - k:7 - k + nf]) for k in range(7)]
+    got = np.moveaxis(F.cpu().numpy(), ax, -1)
+    # as beside large values: 16 roundings of the terms
+    off = np.abs(got - sum(terms)) / (EPS * sum(np.abs(t) for t in terms) + 1e-300)
+    assert off.max() <= 16.0, float(off.max())
