@@ -42,10 +42,12 @@ __global__ void __launch_bounds__(128, 5) k_viscous(const DevParams P, const R* 
     if constexpr (sizeof(R) == 8) {
         // C_s T^(3/2) / (T + T_s) = C_s T^2 (T (T + T_s)^2)^(-1/2): one reciprocal root instead of a
         // root and a quotient (five multiplications and 368 cycles of
-        // the FP64 pipe against three and 1120)
+        // the FP64 pipe against three and 1120). Where T (T + T_s)^2 is not a positive normal number
+        // (T zero, negative or not finite, or beyond 1e102) the quotient itself
         const A a = T + A(K.t_s), b = (T * a) * a;
-        mu = (A(K.c_s) * T) * (T * rsq(b));
-        if (((__double_as_longlong(T.v)) << 1) == 0) mu = f64(0.0);  // T = 0, where the root has a pole
+        const unsigned e = (unsigned)__double2hiint(b.v) >> 20;  // sign and exponent
+        if (e - 1u <= 2045u) mu = (A(K.c_s) * T) * (T * rsq(b));
+        else mu = f64(K.c_s * T.v * ::sqrt(T.v) / (T.v + K.t_s));
     } else {
         mu = K.c_s * T * sqrt(T) / (T + K.t_s);
     }
