@@ -85,7 +85,7 @@ __device__ __forceinline__ void char_left_row(const CharBasis<R>& b, int n, R l[
 
 // The characteristic flux of field n at the face: the field's projection L_n F of the stencil's
 // split fluxes, reconstructed by WENO7 (br 1) or WENO5 (br 2) on each side.
-template <class R, class FPA, class FMA>
+template <class R, bool REF32 = false, class FPA, class FMA>
 __device__ __forceinline__ R char_field_flux(const DevParams& P, const CharBasis<R>& b, int n, int br, int p0, R s0,
                                              FPA FP, FMA FM) {
     R l[5];
@@ -100,14 +100,9 @@ __device__ __forceinline__ R char_field_flux(const DevParams& P, const CharBasis
         return weno_pair(br, s0, [&](int k) { return projP(p0 + k); }, [&](int k) { return projM(p0 + 7 - k); });
     } else {
         const R tmp1 = R(1) / R(12), tmp2 = R(1) / R(6);
-        if (P.ref32) {  // the reference's Float32 reconstruction of the characteristic fields
-            if (br == 1) {
-                const double fp = weno7_ref32(projP(p0), projP(p0 + 1), projP(p0 + 2), projP(p0 + 3), projP(p0 + 4),
-                                              projP(p0 + 5), projP(p0 + 6), s0);
-                const double fm = weno7_ref32(projM(p0 + 7), projM(p0 + 6), projM(p0 + 5), projM(p0 + 4),
-                                              projM(p0 + 3), projM(p0 + 2), projM(p0 + 1), s0);
-                return (float)((fp + fm) * (double)tmp1);
-            }
+        if constexpr (REF32) {  // the reference's Float32 reconstruction of the characteristic fields
+            if (br == 1)
+                return weno7_ref32_pair(s0, [&](int k) { return projP(p0 + k); }, [&](int k) { return projM(p0 + 7 - k); });
             return (weno5_ref32(projP(p0 + 1), projP(p0 + 2), projP(p0 + 3), projP(p0 + 4), projP(p0 + 5), s0) +
                     weno5_ref32(projM(p0 + 6), projM(p0 + 5), projM(p0 + 4), projM(p0 + 3), projM(p0 + 2), s0)) *
                    tmp2;
@@ -140,20 +135,15 @@ __device__ __forceinline__ R char_right_row(const CharBasis<R>& b, int k, const 
 }
 
 // Component n of a component-wise WENO7 (schemes.jl:143-230) / WENO5 (:231-276) face
-template <class R, class FPA, class FMA>
+template <class R, bool REF32 = false, class FPA, class FMA>
 __device__ __forceinline__ R comp_field_flux(const DevParams& P, int n, int br, int p0, R s0, FPA FP, FMA FM) {
     if constexpr (sizeof(R) == 8) {
         return weno_pair(br, s0, [&](int k) { return FP(n, p0 + k); }, [&](int k) { return FM(n, p0 + 7 - k); });
     } else {
         const R tmp1 = R(1) / R(12), tmp2 = R(1) / R(6);
-        if (P.ref32) {  // the reference's Float32 reconstruction
-            if (br == 1) {
-                const double fp = weno7_ref32(FP(n, p0), FP(n, p0 + 1), FP(n, p0 + 2), FP(n, p0 + 3), FP(n, p0 + 4),
-                                              FP(n, p0 + 5), FP(n, p0 + 6), s0);
-                const double fm = weno7_ref32(FM(n, p0 + 7), FM(n, p0 + 6), FM(n, p0 + 5), FM(n, p0 + 4),
-                                              FM(n, p0 + 3), FM(n, p0 + 2), FM(n, p0 + 1), s0);
-                return (float)((fp + fm) * (double)tmp1);
-            }
+        if constexpr (REF32) {  // the reference's Float32 reconstruction
+            if (br == 1)
+                return weno7_ref32_pair(s0, [&](int k) { return FP(n, p0 + k); }, [&](int k) { return FM(n, p0 + 7 - k); });
             return (weno5_ref32(FP(n, p0 + 1), FP(n, p0 + 2), FP(n, p0 + 3), FP(n, p0 + 4), FP(n, p0 + 5), s0) +
                     weno5_ref32(FM(n, p0 + 6), FM(n, p0 + 5), FM(n, p0 + 4), FM(n, p0 + 3), FM(n, p0 + 2), s0)) *
                    tmp2;
@@ -175,7 +165,7 @@ __device__ __forceinline__ R comp_field_flux(const DevParams& P, int n, int br, 
 // p0..p0+7 of the line (face between positions p0+3 and p0+4). FP/FM(n, pos) read shared
 // memory. For characteristic mode the face state comes from global memory at the two
 // adjacent cells (cl, cr linear indices).
-template <bool CHAR, class R, class FPA, class FMA>
+template <bool CHAR, class R, bool REF32 = false, class FPA, class FMA>
 __device__ __forceinline__ void face_flux(const DevParams& P, const SweepArgs& a, int br, int p0, R s0,
                                           long long cl, long long cr, FPA FP, FMA FM, R out[5]) {
     const auto& K = cst<R>(P);
@@ -211,7 +201,7 @@ __device__ __forceinline__ void face_flux(const DevParams& P, const SweepArgs& a
     }
     if (!CHAR) {
 #pragma unroll 1
-        for (int n = 0; n < 5; n++) out[n] = comp_field_flux<R>(P, n, br, p0, s0, FP, FM);
+        for (int n = 0; n < 5; n++) out[n] = comp_field_flux<R, REF32>(P, n, br, p0, s0, FP, FM);
         return;
     }
     // characteristic-wise, schemes.jl:756-999
@@ -220,7 +210,7 @@ __device__ __forceinline__ void face_flux(const DevParams& P, const SweepArgs& a
                   static_cast<const R*>(a.A[2]), s0, cl, cr, cb);
     R flux[5];
 #pragma unroll 1
-    for (int n = 0; n < 5; n++) flux[n] = char_field_flux<R>(P, cb, n, br, p0, s0, FP, FM);
+    for (int n = 0; n < 5; n++) flux[n] = char_field_flux<R, REF32>(P, cb, n, br, p0, s0, FP, FM);
 #pragma unroll
     for (int k = 0; k < 5; k++) out[k] = char_right_row<R>(cb, k, flux);
 }

@@ -256,23 +256,41 @@ __device__ __forceinline__ double weno7_ref32(float V1, float V2, float V3, floa
     // alpha_k over their common denominator (one FP64 division a side instead of five): the
     // reference's values to within FP64 rounding, far below the Float32 the result is rounded to.
     // Bases from 1e-20 to 3e38: the triple products stay within 1e-120 .. 1e231. An indicator beyond
-    // Float32's range has an alpha of zero, as the quotient gives it: it is left out of the others'
-    // products. Plain double expressions and selections: branches here change how the compiler
-    // contracts the mixed form's FP32 faces in the same kernels
+    // Float32's range gives NaN here (weno7_ref32_quotients)
     const double e1 = 1e-20;
-    const float x[4] = {Is[0] * s0, Is[1] * s0, Is[2] * s0, Is[3] * s0};
-    double b[4], w[4] = {0.0, 12.0, 18.0, 4.0};
-    bool first = false;
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const bool over = (__float_as_uint(x[k]) & 0x7fffffffu) == 0x7f800000u;
-        b[k] = over ? 1.0 : sq(e1 + (double)x[k]);
-        w[k] = over ? 0.0 : w[k];
-        if (k == 0) first = over;
-    }
-    const double p12 = b[0] * b[1], p34 = b[2] * b[3];
-    const double a1 = first ? 0.0 : b[1] * p34, a2 = w[1] * b[0] * p34, a3 = w[2] * p12 * b[3], a4 = w[3] * p12 * b[2];
+    const double b1 = sq(e1 + (double)(Is[0] * s0)), b2 = sq(e1 + (double)(Is[1] * s0));
+    const double b3 = sq(e1 + (double)(Is[2] * s0)), b4 = sq(e1 + (double)(Is[3] * s0));
+    const double p12 = b1 * b2, p34 = b3 * b4;
+    const double a1 = b2 * p34, a2 = 12.0 * b1 * p34, a3 = 18.0 * p12 * b4, a4 = 4.0 * p12 * b3;
     return (a1 * (double)q[0] + a2 * (double)q[1] + a3 * (double)q[2] + a4 * (double)q[3]) / (a1 + a2 + a3 + a4);
+}
+// Both sides of a face with one quotient per alpha, for faces whose value is NaN otherwise: an indicator
+// that overflowed Float32 has a weight of zero. P, M: the sides' upwind-ordered stencils. Not inlined, and
+// fed from the stencils again, so that the faces that do not need it hold no register for it.
+static __device__ __noinline__ float weno7_ref32_quotients(const float* P, const float* M, float s0) {
+    double f = 0.0;
+    const double e1 = 1e-20;
+    for (int side = 0; side < 2; side++) {
+        const float* V = side == 0 ? P : M;
+        float q[4], Is[4];
+        weno7_parts<float>(V[0], V[1], V[2], V[3], V[4], V[5], V[6], q, Is);
+        const double a1 = 1.0 / sq(e1 + (double)(Is[0] * s0)), a2 = 12.0 / sq(e1 + (double)(Is[1] * s0));
+        const double a3 = 18.0 / sq(e1 + (double)(Is[2] * s0)), a4 = 4.0 / sq(e1 + (double)(Is[3] * s0));
+        f += (a1 * (double)q[0] + a2 * (double)q[1] + a3 * (double)q[2] + a4 * (double)q[3]) / (a1 + a2 + a3 + a4);
+    }
+    return (float)(f * (double)(1.f / 12.f));
+}
+template <class PF, class MF> __device__ __forceinline__ float weno7_ref32_pair(float s0, PF P, MF M) {
+    const double fp = weno7_ref32(P(0), P(1), P(2), P(3), P(4), P(5), P(6), s0);
+    const double fm = weno7_ref32(M(0), M(1), M(2), M(3), M(4), M(5), M(6), s0);
+    const float f = (float)((fp + fm) * (double)(1.f / 12.f));
+    if (f == f) return f;
+    float p[7], m[7];
+    for (int k = 0; k < 7; k++) {
+        p[k] = P(k);
+        m[k] = M(k);
+    }
+    return weno7_ref32_quotients(p, m, s0);
 }
 // WENO5 in Float32 with one division per alpha and one for their sum (schemes.jl:233-252).
 __device__ __forceinline__ float weno5_ref32(float V1, float V2, float V3, float V4, float V5, float s0) {

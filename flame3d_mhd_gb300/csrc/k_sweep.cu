@@ -33,7 +33,7 @@ namespace f3d {
 // 160 x 4 4.74 -> 288 x 3 4.64 ms, 320 x 3 4.67, 192 x 5 4.82. Tiles of eight lines or of
 // 32 cells lose more on the smaller grids than the ramp gains.
 // FP32: the same tile sizes (~20 KB). The Float32 form (FP64 WENO7 weights) on 320 threads, five
-// blocks per SM (32 registers, the characteristic form spills ~270 bytes): one pass per phase and 50
+// blocks per SM (32 registers, the characteristic form spills ~310 bytes, component-wise ~95): one pass per phase and 50
 // warps an SM for the latencies of the weights. RK3 step of its shock tube 256x64x64, 128 threads x
 // 6 -> 320 x 5: 4.80 -> 4.07 ms (288 x 6 4.12, 288 x 5 4.19, 160 x 7 4.40, 224 x 6 4.47, 288 x 3 5.06).
 // The mixed form (grids without TMA rows) keeps 128 x 6, 80 registers: on small grids the spills
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(Tile<DIR, R, FACES>::NT, Tile<DIR, R, FACES>::
         if (FACES != WENO_LISTED && (br == 1 || br == 2)) s0 = A(2) / (arith(Sr[cl]) + arith(Sr[cr]));
         auto FP = [&](int n, int p) { return arith(sFp[n * TL * NP + sidx(l, p)]); };
         auto FM = [&](int n, int p) { return arith(sFm[n * TL * NP + sidx(l, p)]); };
-        face_flux<FACES == WENO_CHAR || FACES == WENO_CHAR_REF32, A>(P, a, br, t, s0, cl, cr, FP, FM, out);
+        face_flux<FACES == WENO_CHAR || FACES == WENO_CHAR_REF32, A, FloatTile<FACES>::REF32>(P, a, br, t, s0, cl, cr, FP, FM, out);
         const int f = fidx(l, t);
 #pragma unroll
         for (int n = 0; n < 5; n++) sF[n * TL * NF + f] = plain(out[n]);
