@@ -103,18 +103,19 @@ __device__ __forceinline__ F64 recip_ieee(F64 b) {
     const F64 r = recip_step(b.v);
     return r + (f64(in_register(1.0)) - b * r) * r;
 }
-// a/b: a times the reciprocal and one residual correction (six FMAs; as near to the IEEE quotient
-// as recip_ieee) where the quotient and the residual are normal; the IEEE division elsewhere
+// a/b: a times the reciprocal and one residual correction (Markstein's; six FMAs; as near to the IEEE
+// quotient as recip_ieee) where the quotient and the residual are normal; the IEEE division elsewhere
 __device__ __forceinline__ F64 operator/(F64 a, F64 b) {
     const unsigned ha = (unsigned)__double2hiint(a.v) & 0x7fffffffu, ea = ha >> 20;
     const unsigned eb = ((unsigned)__double2hiint(b.v) >> 20) & 0x7ffu;
     // both factors, the quotient and the residual well inside the normal range, or a zero dividend
-    const bool plain = eb - 2u <= 2040u && ((ea - 110u <= 1900u && ea - eb + 900u <= 1800u) ||
-                                            (ha | (unsigned)__double2loint(a.v)) == 0u);
+    const bool zero = (ha | (unsigned)__double2loint(a.v)) == 0u;
+    const bool plain = eb - 2u <= 2040u && ((ea - 110u <= 1900u && ea - eb + 900u <= 1800u) || zero);
     if (!plain) return f64(a.v / b.v);
     const F64 r = recip_step(b.v);
     const F64 q = a * r;
-    return q + (a - b * q) * r;
+    const F64 c = q + (a - b * q) * r;  // (a zero's sign would be lost here)
+    return f64(zero ? q.v : c.v);
 }
 using ::fabs;  // the overloads below stand beside the library's
 using ::sqrt;
