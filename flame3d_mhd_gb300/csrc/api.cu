@@ -212,6 +212,10 @@ struct f3d_ctx {
     double* dtl = nullptr;
     double* sc = nullptr;
     long long tt = 0;
+    // scratch that must be zero before its first use: cleared by the first call that has a stream
+    // (clear_once), since the legacy stream's work is not ordered with streams that do not wait for it
+    struct { void* p; size_t bytes; } unset[3] = {};
+    int n_unset = 0;
     void* extra = nullptr;
     // mixed precision: FP32 copies and FP32 intermediates
     float* Q32 = nullptr;
@@ -310,6 +314,16 @@ int check_ctx(f3d_ctx* ctx, bool need_state, bool f32_entry = false) {
         if (ctx->params.bc[f].kind == F3D_BC_INFLOW_PROFILE && !ctx->dp.prof[f])
             return fail(ctx, F3D_ERR_STATE, "inflow profile not set (call f3d_set_inflow_profile)");
     if (cudaSetDevice(ctx->device) != cudaSuccess) return fail(ctx, F3D_ERR_CUDA, "cudaSetDevice failed");
+    return F3D_OK;
+}
+
+// Clear the scratch that f3d_create left unset: in the entries that set the metrics, which every other
+// entry that reads it needs, and in those that read it without metrics.
+int clear_once(f3d_ctx* ctx, cudaStream_t st) {
+    for (; ctx->n_unset > 0; ctx->n_unset--) {
+        const auto& u = ctx->unset[ctx->n_unset - 1];
+        F3D_CUDA(ctx, cudaMemsetAsync(u.p, 0, u.bytes, st));
+    }
     return F3D_OK;
 }
 
@@ -812,12 +826,13 @@ int f3d_create(const f3d_params* p, f3d_ctx** out) {
     const size_t nplane = (size_t)ctx->dp.plane;
     if (p->lts || p->filter == F3D_FILTER_NONLINEAR) {  // local dt, filter sensor (zero outside the interior)
         const size_t eb = nplane * sizeof(double) * 2;
-        if (cudaMalloc(&ctx->extra, eb) != cudaSuccess || cudaMemset(ctx->extra, 0, eb) != cudaSuccess) {
-            if (ctx->extra) cudaFree(ctx->extra);
+        if (cudaMalloc(&ctx->extra, eb) != cudaSuccess) {
+            cudaGetLastError();
             delete ctx;
             std::fprintf(stderr, "f3d_create: cudaMalloc of the step-component scratch failed\n");
             return F3D_ERR_CUDA;
         }
+        ctx->unset[ctx->n_unset++] = {ctx->extra, eb};
         ctx->dtl = (double*)ctx->extra;
         ctx->sc = ctx->dtl + nplane;
     }
@@ -910,9 +925,9 @@ int f3d_create(const f3d_params* p, f3d_ctx** out) {
     const bool want_tma = p->precision == F3D_PREC_MIXED && !fvm && sweep_tma_usable(ctx->dp) &&
                           !(no_tma && no_tma[0] == '1');
     // phi outside cells 1..Nt-2 is never written; keep it defined (CUDA.zeros in solver.jl:296)
-    if ((e = cudaMemset(mx ? (void*)ctx->phi32 : (void*)ctx->phi, 0, phi_bytes)) != cudaSuccess ||
-        (e = cudaMemset(q, 0, 32)) != cudaSuccess || (e = cudaStreamSynchronize(nullptr)) != cudaSuccess ||  // any stream may be next
-        (e = sweep_configure()) != cudaSuccess ||
+    ctx->unset[ctx->n_unset++] = {mx ? (void*)ctx->phi32 : (void*)ctx->phi, phi_bytes};
+    ctx->unset[ctx->n_unset++] = {q, 32};
+    if ((e = sweep_configure()) != cudaSuccess ||
         (fvm && (e = fvm_configure()) != cudaSuccess) || (want_tma && (e = sweep_tma_configure()) != cudaSuccess)) {
         cudaFree(ctx->slab);
         if (ctx->extra) cudaFree(ctx->extra);
@@ -966,6 +981,7 @@ int f3d_set_metrics(f3d_ctx* ctx, const double* const metrics[9], const double* 
     if ((rc = check_ptrs(ctx, {metrics[0], metrics[1], metrics[2], metrics[3], metrics[4], metrics[5], metrics[6],
                               metrics[7], metrics[8], jac})))
         return rc;
+    if ((rc = clear_once(ctx, (cudaStream_t)stream))) return rc;
     for (int n = 0; n < 9; n++) ctx->m[n] = metrics[n];
     ctx->J = jac;
     drop_step_graph(ctx);  // a captured step holds the previous metric pointers
@@ -1107,6 +1123,7 @@ int f3d_set_metrics_f32(f3d_ctx* ctx, const float* const metrics[9], const float
     if ((rc = check_ptrs(ctx, {metrics[0], metrics[1], metrics[2], metrics[3], metrics[4], metrics[5], metrics[6],
                               metrics[7], metrics[8], jac})))
         return rc;
+    if ((rc = clear_once(ctx, (cudaStream_t)stream))) return rc;
     for (int n = 0; n < 9; n++) ctx->m32.A[n] = const_cast<float*>(metrics[n]);  // read only
     ctx->m32.J = const_cast<float*>(jac);
     drop_step_graph(ctx);
@@ -1211,6 +1228,7 @@ int f3d_filter(f3d_ctx* ctx, double* U, double* Un, const double* Q, f3d_stream 
     int rc = check_ctx(ctx, false);
     if (rc || (rc = check_ptrs(ctx, {U, Un, Q}))) return rc;
     if (!ctx->params.filter) return fail(ctx, F3D_ERR_ARG, "params.filter is F3D_FILTER_NONE");
+    if ((rc = clear_once(ctx, (cudaStream_t)stream))) return rc;
     return apply_filter(ctx, U, Un, Q, (cudaStream_t)stream);
 }
 
@@ -1413,6 +1431,7 @@ int f3d_check_finite(f3d_ctx* ctx, const double* U, f3d_stream stream) {
     int rc = check_ctx(ctx, false);
     if (rc || (rc = check_ptrs(ctx, {U}))) return rc;
     cudaStream_t st = (cudaStream_t)stream;
+    if ((rc = clear_once(ctx, st))) return rc;
     int flag[2] = {0, 0};  // the non-finite flag, then the kernel status word
     F3D_CUDA(ctx, cudaMemsetAsync(ctx->dscalar, 0, 8, st));
     F3D_CUDA(ctx, launch_check_finite(ctx->dp, U, (int*)ctx->dscalar, st));

@@ -30,9 +30,9 @@ class Host:
         assert (rc == 0) == ok
         return self
 
-    def metrics(self):
+    def metrics(self, stream=0x77):
         m = (C.c_void_p * 9)(*[next(self.array) for _ in range(9)])
-        assert self.lib.f3d_set_metrics(self.ctx, m, next(self.array), None) == 0
+        assert self.lib.f3d_set_metrics(self.ctx, m, next(self.array), C.c_void_p(stream)) == 0
         return self
 
     def rhs(self, stream=0x77):
@@ -91,15 +91,29 @@ def _launches(rows, name):
     return [r for r in rows if r[0].startswith("launch:") and name in r[0]]
 
 
-def test_memory_is_cleared_before_any_stream_uses_it(host):
+@pytest.mark.parametrize("first", ["metrics", "check", "filter"])
+def test_memory_is_cleared_before_any_stream_uses_it(host, first):
     """Streams that do not wait for the legacy stream (PyTorch's pool streams) may be the first to use a
-    context: the memory that f3d_create clears is waited for, and the adjoint's, which the first
-    reverse call takes, is cleared on that call's stream."""
-    h = host().create()
+    context: what must be zero is cleared on the stream of the first call that needs it, once, and the
+    adjoint's scratch, which the first reverse call takes, on that call's."""
+    h = host(filter=abi.FILTER_NONLINEAR if first == "filter" else abi.FILTER_NONE).create()
     rows = h.log()
-    cleared = [i for i, r in enumerate(rows) if r[0] == "memset"]
-    waits = [i for i, r in enumerate(rows) if r[0] in ("sync", "sync-device") and r[3] == 0]
-    assert cleared and waits and waits[-1] > cleared[-1]
+    held = [r for r in rows if r[0] == "malloc"]
+    assert not any(r[0] == "memset" for r in rows)
+    if first == "check":
+        h.lib.f3d_check_finite(h.ctx, next(h.array), C.c_void_p(0x55))
+    elif first == "filter":
+        h.lib.f3d_filter(h.ctx, *[next(h.array) for _ in range(3)], C.c_void_p(0x55))
+    else:
+        h.metrics(0x55)
+    rows = [r for r in h.log() if r[0] == "memset" and any(m[1] <= r[1] < m[1] + m[2] for m in held)]
+    sizes = {r[2] for r in rows}
+    assert 32 in sizes and any(s >= 8 * h.plane for s in sizes) and all(r[3] == 0x55 for r in rows)
+    assert first != "filter" or 16 * h.plane in sizes
+    h.metrics(0x66)
+    assert not any(r[0] == "memset" for r in h.log())
+    if first == "filter":
+        return  # the adjoint has no filters
     h.metrics().log()
     assert h.vjp(0x99) == 0
     rows = h.log()
