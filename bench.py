@@ -62,6 +62,13 @@ STEP_BYTES_PER_CELL = 3 * 160 + 2 * 40
 KERNEL_TRAFFIC_PER_CELL = {"sweep_xi": 139.8, "sweep_eta": 197.5, "sweep_zeta": 290.7}
 
 
+def largest_kernels(prof: dict) -> tuple[str, str]:
+    """Of {kernel: [ms, launches]} the one that takes most time, and the one of those whose bytes a
+    cell are fixed: the WENO faces' depend on how many faces are listed."""
+    ms = lambda k: prof[k][0]  # noqa: E731
+    return max(prof, key=ms), max((k for k in prof if k in KERNEL_BYTES_PER_CELL), key=ms)
+
+
 def load_peaks() -> dict:
     p = ROOT / "MEASURED_PEAKS.json"
     if p.exists():
@@ -461,8 +468,7 @@ def run_ours(args):
                 a[1] += n
     launches_per_step = sum(n for _, n in prof.values()) // 3
     total_ms = sum(t for t, _ in prof.values())
-    # the largest kernel whose bytes a cell are fixed (weno_faces' depend on the number of WENO faces)
-    top = max((k for k in prof if k in KERNEL_BYTES_PER_CELL), key=lambda k: prof[k][0])
+    largest, top = largest_kernels(prof)
     top_avg_ms = prof[top][0] / prof[top][1]
     peaks = load_peaks()
     alg = KERNEL_BYTES_PER_CELL[top] * cells
@@ -473,6 +479,8 @@ def run_ours(args):
                 "traffic_source": "ncu DRAM bytes per cell of the stage-mode sweep on this workload", "kernel": top,
                 "peak_source": peaks["source"],
                 "alg_bytes_per_launch": alg, "avg_launch_ms": top_avg_ms,
+                "largest_kernel": {"kernel": largest, "ms_per_stage": prof[largest][0] / 9,
+                                   "bytes": KERNEL_BYTES_PER_CELL[largest] * cells if largest in KERNEL_BYTES_PER_CELL else None},
                 "shares": {k: round(v[0] / total_ms, 4) for k, v in sorted(prof.items())}}
     step_gbs = STEP_BYTES_PER_CELL * cells / (ms_step / 1e3) / 1e9
 
@@ -561,16 +569,17 @@ def run_ours(args):
     # against the FMA-chain peak measured on this GPU now
     from flame3d_mhd_gb300.solver import measure_pipes
     fp64_peak, fp32_peak = measure_pipes()
-    line["roofline_fp64_pipe"] = {"bound": "fp64", "peak": fp64_peak, "unit": "TFLOP/s", "fp32_peak": fp32_peak,
-                                  "achieved": None, "frac": None, "flops_per_cell_rhs": None,
-                                  "note": "flops from the oracle's exact op count (CPU leg), of which the linear faces' run as integers (the fraction may exceed 1); GPU divides "
-                                          "and square roots cost ~10 FMA slots each but count as 1"}
+    line["formula_flops"] = {"achieved": None, "unit": "TFLOP/s", "per_cell_rhs": None, "fp64_fma_peak": fp64_peak,
+                             "fp32_fma_peak": fp32_peak, "per_fma_peak": None,
+                             "note": "operations of the formulas (the oracle's exact count, CPU leg) per second, and over the "
+                                     "FP64 FMA-chain peak of this run; not a use of the FP64 pipe: the linear faces' products "
+                                     "run as integers, divides and roots count as one"}
     if rank == 0 and ws == 1 and not args.no_cpu:
         line["parity"] = rhs_parity(r64.cpu().numpy())
         line["cpu_baseline"] = cpu_sample()
         f = workload_flops_per_cell()
         ach = f * value * 1e6 / ws / 1e12
-        line["roofline_fp64_pipe"].update(achieved=ach, frac=ach / fp64_peak, flops_per_cell_rhs=f)
+        line["formula_flops"].update(achieved=ach, per_cell_rhs=f, per_fma_peak=ach / fp64_peak)
     if rank == 0:
         print(json.dumps(line), flush=True)
     s.close()
