@@ -377,7 +377,8 @@ template <class R> __device__ __forceinline__ R weno7(R V1, R V2, R V3, R V4, R 
 //    (as alpha_k = prod_{j != k} b_j), and the two sides share one reciprocal:
 //    N_p / D_p + N_m / D_m = (N_p D_m + N_m D_p) / (D_p D_m).
 // 149 FP64 instructions for a pair of WENO7 sides against 182, 88 for WENO5 against 140. Bases far
-// beyond any flux's (products outside 2^-1000 .. 2^800) take two IEEE quotients.
+// beyond any flux's (products outside 2^-1000 .. 2^800) and numerators near the subnormal numbers take
+// two IEEE quotients.
 struct WenoSums {
     F64 base, N, D;
 };
@@ -438,9 +439,13 @@ template <class VF> __device__ __forceinline__ WenoSums weno5_sums(VF V, F64 s0,
 // The sum of both sides' values; unit: 1/12 (WENO7) or 1/6 (WENO5)
 __device__ __forceinline__ F64 weno_join(const WenoSums& p, const WenoSums& m, double unit) {
     const F64 D = p.D * m.D, base = p.base + m.base;
-    const unsigned e = ((unsigned)__double2hiint(D.v) >> 20) & 0x7ffu;
-    if (e - 23u > 1800u) return base + F64(unit) * (p.N / p.D + m.N / m.D);
-    return base + F64(unit) * ((p.N * m.D + m.N * p.D) * recip_step(D.v));
+    const F64 N = p.N * m.D + m.N * p.D;
+    const unsigned e = ((unsigned)__double2hiint(D.v) >> 20) & 0x7ffu, n = ((unsigned)__double2hiint(N.v) >> 20) & 0x7ffu;
+    // N near or below the smallest normal number, with terms that are not zero (a component whose
+    // differences are below ~1e-60: D is 1e-240 there)
+    const bool tiny = n < 64u && (((unsigned)__double2hiint(p.N.v) | (unsigned)__double2hiint(m.N.v)) & 0x7fffffffu) != 0u;
+    if (e - 23u > 1800u || tiny) return base + F64(unit) * (p.N / p.D + m.N / m.D);
+    return base + F64(unit) * (N * recip_step(D.v));
 }
 // br 1: WENO7, 2: WENO5. P(k), M(k): the two sides' upwind-ordered stencils
 template <class PF, class MF> __device__ __forceinline__ F64 weno_pair(int br, F64 s0, PF P, MF M) {
