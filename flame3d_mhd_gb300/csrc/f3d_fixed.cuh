@@ -21,17 +21,18 @@
 // truncated to a multiple of 2^-61 of it (in units of the largest's power of two). The largest need not
 // be a value that a sum reads, or reads under a coefficient that matters (they go down to 3/420), so each
 // sum is looked at by itself (beyond_spread): it is formed from integers if one of the values under
-// its central coefficients (214/420 and above) is within 2^5 of the largest, or if every value that it
-// reads enters exactly. What is truncated is then at most 2.9 units for a face (1.2 for a one-sided sum), the
-// central term alone at least 2^-6 of the largest, so the error is below 0.7 x 2^-53 (0.3) of the sum of
-// the magnitudes of the sum's own terms, less than an FP64 evaluation rounds. A one-sided sum is also formed
-// from integers if a value beside its centre is within 2^3 of the largest, or the largest itself beyond that:
-// under coefficients of 38/420 and 4/420 and above such a term is at least 2^-6.7 of the largest, and the
-// error again below 0.7 x 2^-53 of the terms (the cotangents of a line's first faces, whose outermost is a
-// hundred times the others'). Then one rounding to FP64 and one in the product with 1/D. Other sums,
-// infinities, NaN and strips whose magnitudes lie near the ends of the FP64 range are formed in FP64. Against extended precision the right-hand side of
-// a coarse tube is off by 0.95 / 0.85 / 0.91 (Steger-Warming / Lax-Friedrichs / AUSM) and of a
-// finite-volume vortex by 0.97 of what FP64 sums leave.
+// its central coefficients (214/420 and above) is within 2^5 of the largest, or if every value (of the
+// strip; one-sided sums: that it reads) enters exactly. What is truncated is then at most 2.9 units for a
+// face (1.2 for a one-sided sum), the central term alone at least 2^-6 of the largest, so the error is
+// below 0.7 x 2^-53 (0.3) of the sum of the magnitudes of the sum's own terms, less than an FP64
+// evaluation rounds. A one-sided sum is also formed from integers if a value beside its centre is within
+// 2^3 of the largest, or the largest itself beyond that: under coefficients of 38/420 and 4/420 and above
+// such a term is at least 2^-6.7 of the largest, and the error again below 0.7 x 2^-53 of the terms (the
+// cotangents of a line's first faces, whose outermost is a hundred times the others'). Then one rounding
+// to FP64 and one in the product with 1/D. Other sums, infinities, NaN and strips whose magnitudes lie near
+// the ends of the FP64 range are formed in FP64. Against extended precision the right-hand side of a coarse
+// tube is off by 0.95 / 0.85 / 0.91 (Steger-Warming / Lax-Friedrichs / AUSM) and of a finite-volume
+// vortex by 0.97 of what FP64 sums leave.
 #pragma once
 #include "f3d_kernels.cuh"
 
@@ -123,11 +124,11 @@ template <class NEAR> __device__ __forceinline__ unsigned beyond_spread(int E, u
     return far & want;
 }
 
-// The sums f whose values f .. f + n - 1 all have their bit in `exact`
-__device__ __forceinline__ unsigned whole_windows(unsigned exact, int n) {
+// The sums f whose values f .. f + 7 all have their bit in `exact`
+__device__ __forceinline__ unsigned whole_windows(unsigned exact) {
     unsigned whole = exact;
 #pragma unroll
-    for (int k = 1; k < n; k++) whole &= exact >> k;
+    for (int k = 1; k < 8; k++) whole &= exact >> k;
     return whole;
 }
 // Whether a value enters a strip of exponent E without loss: 2^-9 of the largest or more, or zero
@@ -172,7 +173,7 @@ __device__ __forceinline__ void linear_strip_both(const DevParams& P, int t0, un
                 m[p] = __double2hiint(v) & 0x7fffffff;
                 exact |= (unsigned)enters_exactly(v, E) << p;
             }
-            far &= ~whole_windows(exact, 8);
+            far &= ~whole_windows(exact);
             // values away from the centre count as much less as their coefficients: 38/420 and above
             // beside it, 4/420 and above beyond (both sums; for any blend)
 #pragma unroll
@@ -250,10 +251,10 @@ __device__ __forceinline__ void linear_strip(const DevParams& P, int t0, int las
     if (E >= 200 && E <= 1900) {
         far = beyond_spread(E, want, [&](int f) { return max(mid[f], mid[f + 1]); });
         if (far) {
-            unsigned exact = 0u;
+            bool exact = true;
 #pragma unroll
-            for (int q = 0; q < NV; q++) exact |= (unsigned)(enters_exactly(P_(q), E) && enters_exactly(M_(q), E)) << q;
-            far &= ~whole_windows(exact, 7);
+            for (int q = 0; q < NV; q++) exact = exact && enters_exactly(P_(q), E) && enters_exactly(M_(q), E);
+            if (exact) far = 0u;
         }
     }
     if (far != want) {
