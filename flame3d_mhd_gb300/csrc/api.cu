@@ -850,8 +850,7 @@ int f3d_create(const f3d_params* p, f3d_ctx** out) {
     }
     // the listed WENO faces (k_weno.cu) of the hybrid finite-difference scheme in FP64: 132 bytes
     // a cell, taken up to 25 GiB (a tenth of the device's memory) and where there is
-    // room; without them the tiles keep their WENO faces. So do the FP32 forms, whose faces are
-    // cheap and whose results would change in the last FP32 bits with the place they are computed in
+    // room; without them the tiles keep their WENO faces. So do the FP32 forms, for which no lists are built
     const size_t bl = up(3 * nc * 4), lists = 256 + bl + 15 * nc * 8;
     bool listed = !fvm && !mx && ctx->dp.fixed_branch < 0 && lists <= ((size_t)25 << 30);
     cudaError_t e = cudaMalloc(&ctx->slab, up(total) + (listed ? lists : 0));

